@@ -9,7 +9,7 @@ same for every seed of a case, as it is in a running engine.
 
 kinds
   chunk   one generateChunkMesh call (no cache), host arrays
-  edit    one player edit: applyCSGOperations on a cached chunk, then its mesh
+  edit    one player edit: applyCSGOperations on a cached chunk, freeChunkOctree, then its new mesh
   tiles   a block of LOD0 chunks around the surface, one batch
   clipmap the nodes nearest a travelling camera, LOD 0 and up, one batch
   frame   all the clipmap nodes of one camera, one batch
@@ -359,6 +359,7 @@ def run(s):
         if kind == "edit":  # dig, then fill, then dig again: each edit changes the field
             s["mg"].apply_csg_operations(s["ops"][s["turn"] & 1], s["min"], s["size"])
             s["turn"] += 1
+            lvn.lib().lvn_meshgen_free_chunk_octree(s["mg"].handle, s["min"], s["size"])  # the mesh follows the field
         mo = s["out"]
         _ok(lvn.lib().lvn_meshgen_generate_chunk_mesh(s["mg"].handle, s["min"], s["size"], C.byref(mo)),
             "generate_chunk_mesh")
