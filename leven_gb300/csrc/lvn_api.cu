@@ -354,7 +354,7 @@ struct lvn_meshgen {
     std::vector<int32_t> last_suse;
 
     // pools
-    DevBuf desc, cs, bs, brushes, mats, planes, edge_tiles, vox_tiles, hmap;
+    DevBuf desc, cs, bs, brushes, mats, planes, edge_tiles, vox_tiles, hmap, search;
     DevBuf edge_keys, edge_chunk, edge_info, edge_work, node_codes, node_info, node_chunk;
     DevBuf edge_slots, node_slots, quad_scratch, node_tile_counts, chunk_tile_off;
     DevBuf vertices, triangles, seams;
@@ -438,6 +438,7 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
     LVN_CK(m->mats.ensure((size_t)F * n));
     LVN_CK(m->planes.ensure(sizeof(uint4) * 3 * (size_t)field_rows(m->vpc) * n));
     LVN_CK(m->hmap.ensure(sizeof(float) * (size_t)field_rows(m->vpc) * n));
+    LVN_CK(m->search.ensure(sizeof(float4) * 2 * kSearchLengths * (size_t)n));
     LVN_CK(m->edge_tiles.ensure(sizeof(int4) * (size_t)edge_tiles_per_chunk(m->vpc) * n));
     LVN_CK(m->vox_tiles.ensure(sizeof(int) * (size_t)vox_tiles_per_chunk(m->vpc) * n));
     LVN_CK(m->chunk_tile_off.ensure(sizeof(int) * (size_t)(n + 1)));
@@ -585,6 +586,7 @@ BatchPtrs make_ptrs(lvn_meshgen* m, int n) {
     b.mats = m->mats.as<uint8_t>();
     b.planes = m->planes.as<uint4>();
     b.hmap = m->hmap.as<float>();
+    b.search = m->search.as<float4>();
     b.edge_tiles = m->edge_tiles.as<int4>();
     b.vox_tiles = m->vox_tiles.as<int>();
     b.edge_keys = m->edge_keys.as<int32_t>();
@@ -1507,7 +1509,7 @@ void lvn_meshgen_destroy(lvn_meshgen* m) {
         }
     }
     if (m->ev_order) cudaEventDestroy(m->ev_order);
-    DevBuf* bufs[] = {&m->desc,       &m->cs,         &m->bs,         &m->brushes,      &m->mats,  &m->planes, &m->hmap,
+    DevBuf* bufs[] = {&m->desc,       &m->cs,         &m->bs,         &m->brushes,      &m->mats,  &m->planes, &m->hmap, &m->search,
                       &m->edge_tiles, &m->vox_tiles,  &m->edge_keys,  &m->edge_chunk,   &m->edge_info, &m->edge_work,
                       &m->node_codes, &m->node_info,  &m->node_chunk, &m->edge_slots,   &m->node_slots,
                       &m->quad_scratch, &m->node_tile_counts, &m->chunk_tile_off, &m->vertices, &m->triangles,

@@ -38,13 +38,22 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int kThreads = 256;
-constexpr int kHermiteSmemThreads = 1024;   // k_hermite_smem: one CTA per SM
+constexpr int kHermiteSmemThreads = 768;    // k_hermite_smem: one CTA per SM; 80 registers a thread, no spills
 // batches at least this large take k_hermite_smem: with the caves density,
 // whose 3D fBm reads the tables most, from 256 chunks (the sweep's first 256,
 // 512 and 1024 chunks ran 5%, 4% and 4% faster a step than with k_hermite);
 // with a heightfield alone from 2048 (a 128-chunk batch ran 8% slower)
 constexpr int kHermiteSmemMinChunks = 2048;
 constexpr int kHermiteSmemMinChunksCaves = 256;
+constexpr int kHermiteCtas = 3;             // k_hermite: CTAs of kThreads per SM
+// Batches of at most this many 64 x 64 voxel faces (chunks x vpc^2) take
+// k_hermite_wide, which trades work for depth: one 64^3 chunk of the terrain
+// takes 12.9 us instead of 47, of the 2D fBm 13.6 instead of 21.8, of the
+// caves 29.5 instead of 42.  Two chunks still gain (17.3 against 22.9 us, 37
+// against 47); four lose with the fBm densities (25.4 against 23.1, 70 against
+// 54), whose searches skip samples, while the terrain takes all of them.
+constexpr int kHermiteWideFaces = 2 * 64 * 64;
+constexpr int kHermiteWideFacesTerrain = 4 * 64 * 64;
 
 // ---------------------------------------------------------------------------
 // geometry
@@ -460,12 +469,104 @@ __device__ __forceinline__ float simp_solve(const SimpQef& q, float s, float& ox
 // stage 0: reset per-chunk state
 // ---------------------------------------------------------------------------
 
+// Interpolation bounds of the crossing search (search_edges).  Along an edge
+// the density is a sum of octaves; between two samples `len` density units
+// apart an octave of 2D or 3D simplex noise of frequency f and amplitude a
+// stays within min(a H (f len)^2 u (1 - u) / 2, 2 a A) of the line through its
+// values there, u in [0, 1] the position between them: H bounds the second
+// derivative along an axis of the noise summed over all lattice points, A its
+// magnitude (tests/test_search_bounds.py derives both).  So the density lies
+// within 4 Q u (1 - u) + C of the line, Q summing the octaves taken by their
+// curvature and C those taken by their magnitude.  C also holds
+//   * twice the error of a float density evaluation against the exact sum:
+//     per octave the coordinates' products (exact when frequency and
+//     lacunarity are powers of two), the unskew and, beyond 2^20, the sample
+//     position itself round by 2^-24 of the coordinate each, times the noise's
+//     gradient bound |dx| + |dy| (+ |dz|); 1e-5 of the amplitude covers the
+//     corner terms' own arithmetic;
+//   * for the octaves from kJumpOctaves up, the jumps of 3D simplex noise:
+//     a corner outside the evaluated simplex would add up to 32 (0.6 - r^2)^4
+//     |g| r with r^2 >= 0.5, at most B in all, so the evaluated noise may
+//     leave the smooth lattice sum by B at either end and between (the 2D
+//     kernel's radius ends at the simplex boundary: no jump).  The lower
+//     octaves' share is added per edge, where they do change simplex
+//     (edge_jump); without that test an LOD0 edge takes 10.2 samples, with it
+//     for two octaves 7.6, for three 7.2, for four 7.1.
+// Entry 4 * class + log2(length) - 1 holds (Q, C, 1 / (8 Q), 0); class 0 is an
+// edge along y (3D term only), class 1 along x or z.  Non-finite parameters
+// give an infinite C, with which no sample is ever skipped.
+constexpr float kNoise3Curve = 41.f, kNoise2Curve = 46.f;   // H
+constexpr float kNoise3Max = 1.0f, kNoise2Max = 1.02f;      // A
+constexpr float kNoise3Slope = 14.f, kNoise2Slope = 11.5f;  // the gradient's 1-norm
+constexpr float kNoise3Jump = 0.0054f;                      // B
+constexpr int kJumpOctaves = 3;
+
+__device__ __forceinline__ void search_bounds(const DensityParams& dp, const ChunkDesc& d, int vpc, float4* out) {
+    float reach = 0.f;  // largest coordinate of the chunk's field
+    for (int a = 0; a < 3; a++)
+        reach = fmaxf(reach, fmaxf(fabsf((float)d.off[a]), fabsf((float)d.off[a] + (float)d.scale * (float)(vpc + 2))));
+    const float eps = 6.2e-8f;  // 2^-24 and a little
+    auto pow2 = [](float f) { return (__float_as_int(f) & 0x7fffff) == 0; };
+    const float far = reach < 1048576.f ? 0.f : 1.f;  // samples at multiples of 1/16 are exact below 2^20
+    float err3 = 0.f, jump = 0.f, err2 = 0.f;
+    if (dp.mode == LVN_DENSITY_CAVES) {
+        const float prod = pow2(dp.freq3) && pow2(dp.lacunarity3) ? 0.f : 1.f;
+        float f = fabsf(dp.freq3), a = fabsf(dp.amp3);
+        for (int k = 0; k < dp.octaves3; k++) {
+            err3 += a * (kNoise3Slope * (2.2f + far + prod * (float)(k + 1)) * eps * f * reach + 1e-5f);
+            if (k >= kJumpOctaves) jump += 2.f * kNoise3Jump * a;
+            f *= fabsf(dp.lacunarity3);
+            a *= fabsf(dp.gain3);
+        }
+    }
+    {
+        const float prod = pow2(dp.freq2) && pow2(dp.lacunarity2) ? 0.f : 1.f;
+        float f = fabsf(dp.freq2), a = fabsf(dp.amp2);
+        for (int k = 0; k < dp.octaves2; k++) {
+            err2 += a * (kNoise2Slope * (2.2f + far + prod * (float)(k + 1)) * eps * f * reach + 1e-5f);
+            f *= fabsf(dp.lacunarity2);
+            a *= fabsf(dp.gain2);
+        }
+    }
+    // y's rounding beyond 2^20; the rounding of the sums y - amp2 h + amp3 n is
+    // relative to their values (the 1e-6 of search_edges, and 1e-4 here)
+    const float round = far * 2.f * eps * reach + 1e-4f;
+    for (int e = 0; e < 2 * kSearchLengths; e++) {
+        const bool xz = e >= kSearchLengths;
+        const float len = (float)d.scale * (float)(2 << (e & (kSearchLengths - 1))) * 0.0625f;
+        // along y the height is one float for every sample
+        float Q = 0.f, C = 2.f * (err3 + round + (xz ? err2 : 0.f)) + jump;
+        auto octaves = [&](int n, float f, float lac, float a, float gain, float H, float A) {
+            for (int k = 0; k < n; k++) {
+                const float w = len * f;
+                const float p = H * w * w * 0.125f;
+                if (p < 3.f * A) Q += a * p;
+                else C += 2.f * A * a;
+                f *= lac;
+                a *= gain;
+            }
+        };
+        if (dp.mode == LVN_DENSITY_CAVES)
+            octaves(dp.octaves3, fabsf(dp.freq3), fabsf(dp.lacunarity3), fabsf(dp.amp3), fabsf(dp.gain3), kNoise3Curve,
+                    kNoise3Max);
+        if (xz)
+            octaves(dp.octaves2, fabsf(dp.freq2), fabsf(dp.lacunarity2), fabsf(dp.amp2), fabsf(dp.gain2), kNoise2Curve,
+                    kNoise2Max);
+        Q *= 1.001f;
+        C *= 1.001f;
+        if (!(Q + C < 1e30f)) Q = 0.f, C = __int_as_float(0x7f800000);
+        out[e] = make_float4(Q, C, Q > 1e-30f ? 1.f / (8.f * Q) : 1e30f, 0.f);
+    }
+}
+
 __global__ void k_reset(BatchPtrs b) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < b.n) {
         ChunkState z;
         memset(&z, 0, sizeof(z));
         b.cs[i] = z;
+        if (b.search && b.density.mode != LVN_DENSITY_REFERENCE)
+            search_bounds(b.density, b.desc[i], b.vpc, b.search + (size_t)2 * kSearchLengths * i);
     }
     if (i == 0) {
         BatchState z;
@@ -1245,99 +1346,52 @@ __global__ void __launch_bounds__(kThreads) k_edge_scatter(BatchPtrs b) {
 // stage 6: hermite data per edge
 // ---------------------------------------------------------------------------
 
-// FindEdgeIntersectionInfo (density_field.cl:96-151).  A y edge keeps x and z
-// fixed, so its height term is evaluated once; the other edges evaluate it
-// per sample.  Each density evaluation has one call site in a loop, which
-// keeps the kernel small enough for the instruction cache.
-// `hm` is the chunk's height map (the field kernel's height term per column),
-// or null: the height at an edge's end points is then read, not recomputed,
-// with the same arguments and so the same value.
-template <int VPC, int MODE, class N>
-__device__ __forceinline__ float4 hermite_density(const BatchPtrs& b, const N& nz, const ChunkDesc& d, int key,
-                                                  const float* hm) {
-    using G = Geo<VPC>;
-    const int axis = key & 3;
-    const int hidx = key >> 2;
-    const int lx = hidx & G::MASK, ly = (hidx >> G::SHIFT) & G::MASK, lz = (hidx >> (2 * G::SHIFT)) & G::MASK;
+// An edge of the hermite work list: its end points (an edge leaves point 0
+// along one axis), its field columns in the chunk's height map.
+struct HermiteEdge {
+    float px, py, pz;   // point 0
+    float step;         // point 1's coordinate along the axis minus point 0's
+    int axis;
+    int c0, c1;         // the end points' columns
+};
+
+// Voxel-index bits and mask of an edge key (Geo::SHIFT, Geo::MASK), and the
+// field dimension, for the hermite kernels: they use them once an edge, so one
+// instance serves every chunk size
+__device__ __forceinline__ int key_shift(int vpc) { return 32 - __clz(vpc); }
+__device__ __forceinline__ void key_voxel(int key, int vpc, int& x, int& y, int& z) {
+    const int hidx = key >> 2, shift = key_shift(vpc), mask = (1 << shift) - 1;
+    x = hidx & mask, y = (hidx >> shift) & mask, z = (hidx >> (2 * shift)) & mask;
+}
+
+__device__ __forceinline__ HermiteEdge hermite_edge(int vpc, const ChunkDesc& d, int key) {
+    HermiteEdge e;
+    e.axis = key & 3;
+    int lx, ly, lz;
+    key_voxel(key, vpc, lx, ly, lz);
     const int s = d.scale;
     const int wx = s * lx + d.off[0], wy = s * ly + d.off[1], wz = s * lz + d.off[2];
-    const float p0x = (float)wx, p0y = (float)wy, p0z = (float)wz;
-    const float p1x = (float)(wx + (axis == 0 ? s : 0));
-    const float p1y = (float)(wy + (axis == 1 ? s : 0));
-    const float p1z = (float)(wz + (axis == 2 ? s : 0));
-    const DensityParams& dp = b.density;
-    const bool yedge = axis == 1;
-    float t = 0.f;
-    float hbest = 0.f;
-    if (b.crossing_mode == 0) {
-        // 17-sample search for min |d| (density_field.cl:122-136); first minimum wins
-        float minv = FLT_MAX;
-        float cur = 0.f;
-        // the end points are field columns: (lx, lz) and (lx, lz) + the x or z step
-        const int c0 = lx + G::FD * lz, c1 = c0 + (axis == 0 ? 1 : axis == 2 ? G::FD : 0);
-        float hy = 0.f;
-        if (yedge) hy = hm ? hm[c0] : height_m<MODE>(nz, dp, p0x, p0z);
-        for (int i = 0; i <= 16; i++) {
-            const float px = fmaf(p1x - p0x, cur, p0x);
-            const float py = fmaf(p1y - p0y, cur, p0y);
-            const float pz = fmaf(p1z - p0z, cur, p0z);
-            // t = 0 and t = 1 (cur sums 16 exact 1/16 steps) land on the end points
-            const float h = yedge ? hy
-                            : (hm && (i == 0 || i == 16)) ? hm[i == 0 ? c0 : c1]
-                                                          : height_m<MODE>(nz, dp, px, pz);
-            const float dv = fabsf(dens_h<MODE>(nz, dp, h, px, py, pz));
-            if (dv < minv) { t = cur; minv = dv; hbest = h; }
-            cur += 0.0625f;
-        }
-    } else {
-        float e0 = 0.f, e1 = 0.f;
-        for (int j = 0; j < 2; j++) {
-            const float qx = j ? p1x : p0x, qy = j ? p1y : p0y, qz = j ? p1z : p0z;
-            const float v = dens_h<MODE>(nz, dp, height_m<MODE>(nz, dp, qx, qz), qx, qy, qz);
-            e0 = j == 0 ? v : e0;
-            e1 = j == 1 ? v : e1;
-        }
-        const float den = e0 - e1;
-        t = den != 0.f ? e0 / den : 0.5f;
-        t = fminf(fmaxf(t, 0.f), 1.f);
-        hbest = height_m<MODE>(nz, dp, fmaf(p1x - p0x, t, p0x), fmaf(p1z - p0z, t, p0z));
-    }
-    const float px = fmaf(p1x - p0x, t, p0x);
-    const float py = fmaf(p1y - p0y, t, p0y);
-    const float pz = fmaf(p1z - p0z, t, p0z);
-    const float h = 0.001f;
-    // central differences: x+h, x-h, z+h, z-h need their own height term;
-    // y+h and y-h share the one at (px, pz)
-    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;  // registers, not an indexed array
-    for (int j = 0; j < 4; j++) {
-        const float qx = j == 0 ? px + h : j == 1 ? px - h : px;
-        const float qz = j == 2 ? pz + h : j == 3 ? pz - h : pz;
-        const float v = dens_h<MODE>(nz, dp, height_m<MODE>(nz, dp, qx, qz), qx, py, qz);
-        d0 = j == 0 ? v : d0;
-        d1 = j == 1 ? v : d1;
-        d2 = j == 2 ? v : d2;
-        d3 = j == 3 ? v : d3;
-    }
-    float ny0 = 0.f, ny1 = 0.f;
-    for (int j = 0; j < 2; j++) {
-        const float v = dens_h<MODE>(nz, dp, hbest, px, j ? py - h : py + h, pz);
-        ny0 = j == 0 ? v : ny0;
-        ny1 = j == 1 ? v : ny1;
-    }
-    float nx = d0 - d1;
-    float ny = ny0 - ny1;
-    float nzv = d2 - d3;
-    normalize3(nx, ny, nzv);
-    return make_float4(nx, ny, nzv, t);
+    e.px = (float)wx, e.py = (float)wy, e.pz = (float)wz;
+    const int wa = e.axis == 0 ? wx : e.axis == 1 ? wy : wz;
+    e.step = (float)(wa + s) - (float)wa;
+    e.c0 = lx + (vpc + 2) * lz;
+    e.c1 = e.c0 + (e.axis == 0 ? 1 : e.axis == 2 ? vpc + 2 : 0);
+    return e;
+}
+
+// mix(point 0, point 1, t): the other coordinates of the end points are equal
+__device__ __forceinline__ void edge_point(const HermiteEdge& e, float t, float& x, float& y, float& z) {
+    const float w = fmaf(e.step, t, e.axis == 0 ? e.px : e.axis == 1 ? e.py : e.pz);
+    x = e.axis == 0 ? w : e.px;
+    y = e.axis == 1 ? w : e.py;
+    z = e.axis == 2 ? w : e.pz;
 }
 
 // CSG FindEdgeIntersectionInfo (apply_csg_operation.cl:443-477)
-template <int VPC>
 __device__ __forceinline__ float4 hermite_brush(const BatchPtrs& b, const ChunkDesc& d, int key) {
-    using G = Geo<VPC>;
     const int axis = key & 3;
-    const int hidx = key >> 2;
-    const int lx = hidx & G::MASK, ly = (hidx >> G::SHIFT) & G::MASK, lz = (hidx >> (2 * G::SHIFT)) & G::MASK;
+    int lx, ly, lz;
+    key_voxel(key, b.vpc, lx, ly, lz);
     const int s = d.scale;
     const int wx = s * lx + d.off[0], wy = s * ly + d.off[1], wz = s * lz + d.off[2];
     const float p0x = (float)wx, p0y = (float)wy, p0z = (float)wz;
@@ -1382,18 +1436,16 @@ __device__ __forceinline__ float4 hermite_brush(const BatchPtrs& b, const ChunkD
 // interpolation of the end points' densities, normal from central
 // differences of the density field (one-sided at the field's faces)
 // interpolated to the crossing.
-template <int VPC>
 __device__ __forceinline__ float4 hermite_sdens(const BatchPtrs& b, int slot, int key) {
-    using G = Geo<VPC>;
-    const int axis = key & 3;
-    const int hidx = key >> 2;
-    const int lx = hidx & G::MASK, ly = (hidx >> G::SHIFT) & G::MASK, lz = (hidx >> (2 * G::SHIFT)) & G::MASK;
-    const float* D = b.sdens + (size_t)slot * G::F;
+    const int axis = key & 3, FD = b.vpc + 2;
+    int lx, ly, lz;
+    key_voxel(key, b.vpc, lx, ly, lz);
+    const float* D = b.sdens + (size_t)slot * FD * FD * FD;
     auto at = [&](int x, int y, int z) {
-        x = min(max(x, 0), G::FD - 1);
-        y = min(max(y, 0), G::FD - 1);
-        z = min(max(z, 0), G::FD - 1);
-        return D[x + G::FD * (y + G::FD * z)];
+        x = min(max(x, 0), FD - 1);
+        y = min(max(y, 0), FD - 1);
+        z = min(max(z, 0), FD - 1);
+        return D[x + FD * (y + FD * z)];
     };
     const int ox = axis == 0, oy = axis == 1, oz = axis == 2;
     const float d0 = at(lx, ly, lz), d1 = at(lx + ox, ly + oy, lz + oz);
@@ -1415,51 +1467,450 @@ __device__ __forceinline__ float4 hermite_sdens(const BatchPtrs& b, int slot, in
     return make_float4(nx, ny, nzv, t);
 }
 
-// The hermite work list, grid-stride: plain x/z edges, plain y edges,
-// CSG-created edges, in segments, so that a warp's 32 edges take the same path.
-template <int VPC, int MODE, class N>
-__device__ __forceinline__ void hermite_list(const BatchPtrs& b, const N& nz) {
-    const int nplain = b.bs->total_xz + b.bs->total_y;
-    const int total = nplain + b.bs->total_created;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < total; w += gridDim.x * blockDim.x) {
+// The jumps SearchBound leaves out: those of the first kJumpOctaves octaves of
+// the 3D term that change simplex along the edge.
+__device__ __forceinline__ float edge_jump(const DensityParams& dp, const HermiteEdge& e) {
+    float w0 = e.axis == 0 ? e.px : e.axis == 1 ? e.py : e.pz;
+    float wa = fmaf(e.step, 0.0625f, w0), wb = fmaf(e.step, 0.9375f, w0), w1 = fmaf(e.step, 1.f, w0);
+    float o1 = e.axis == 0 ? e.py : e.px, o2 = e.axis == 2 ? e.py : e.pz;
+    float jump = 0.f, amp = fabsf(dp.amp3), f = dp.freq3;
+#pragma unroll
+    for (int k = 0; k < kJumpOctaves; k++) {
+        w0 = w0 * f, wa = wa * f, wb = wb * f, w1 = w1 * f, o1 = o1 * f, o2 = o2 * f;
+        if (k < dp.octaves3 && !Noise::same_simplex3(e.axis, w0, wa, wb, w1, o1, o2, k)) jump += 2.01f * kNoise3Jump * amp;
+        f = dp.lacunarity3;
+        amp = amp * fabsf(dp.gain3);
+    }
+    return jump;
+}
+
+// The crossing search of one edge: which samples are evaluated, and the first
+// minimum of |density| over all 17 (density_field.cl:122-136).  The sign change
+// is bisected first, which finds a small |d| in four evaluations; then each
+// interval between evaluated samples is passed over when its SearchBound keeps
+// every sample inside it above the smallest |d| so far, and halved otherwise.
+// A skipped sample is strictly above the final minimum, so the result (the
+// first of equal minima) is that of all 17.  `sval` keeps the inner samples'
+// densities, sample m at [(m - 1) * NT].
+struct EdgeSearch {
+    float d0, d1, jump;  // end densities, the edge's jumps
+    float minv, hbest;   // smallest |d| so far, the height there (unless at an end)
+    int best;            // its sample, -1 = none below FLT_MAX
+    int lo, hi;          // the sign change's bracket
+
+    __device__ __forceinline__ void start(float e0, float e1) {
+        d0 = e0, d1 = e1;
+        minv = FLT_MAX, best = -1, hbest = 0.f;
+        if (fabsf(d0) < minv) minv = fabsf(d0), best = 0;
+        if (fabsf(d1) < minv) minv = fabsf(d1), best = 16;
+        lo = 0, hi = 16;
+    }
+    // sample m has density dv and height h
+    template <int NT>
+    __device__ __forceinline__ void take(int m, float dv, float h, float* sval) {
+        sval[(m - 1) * NT] = dv;
+        const float a = fabsf(dv);
+        if (a < minv || (a == minv && m < best)) minv = a, best = m, hbest = h;
+    }
+    template <int NT>
+    __device__ __forceinline__ float at(int m, const float* sval) const {
+        return m == 0 ? d0 : m == 16 ? d1 : sval[(m - 1) * NT];
+    }
+    // whether a sample strictly inside the interval of 2^(log2len) samples
+    // between densities da and db may reach minv; NaN rules nothing out
+    __device__ __forceinline__ bool may_hold(int log2len, float da, float db, const float4* bound) const {
+        if (!bound || (da < 0.f) != (db < 0.f)) return true;
+        const float4 q = bound[log2len - 1];
+        const float A = fabsf(da), B = fabsf(db), u0 = __int_as_float((127 - log2len) << 23);  // 1 / len
+        // the least of A + (B - A) u - 4 Q u (1 - u), which is convex in u, over
+        // the interval's samples
+        const float u = fminf(fmaxf(fmaf(A - B, q.z, 0.5f), u0), 1.f - u0);
+        const float low = fmaf(B - A, u, A) - 4.f * q.x * u * (1.f - u) - (q.y + jump);
+        return !(low - 1e-6f * (A + B + q.x) > minv);
+    }
+    // After the bisection: the middles of the intervals it left beside its path
+    // (8, 4 and 2 samples long) that may hold a smaller |d|
+    template <int NT>
+    __device__ __forceinline__ uint32_t open(const float* sval, const float4* bound) const {
+        uint32_t out = 0;
+#pragma unroll
+        for (int l = 3; l >= 1; l--) {
+            const int len = 1 << l;
+            const int from = (lo & ~(2 * len - 1)) + (lo & len ? 0 : len);
+            if (may_hold(l, at<NT>(from, sval), at<NT>(from + len, sval), bound)) out |= 1u << (from + len / 2);
+        }
+        return out;
+    }
+    // The same of the halves of the intervals whose middles were just evaluated
+    // (a middle's lowest set bit is the halves' length)
+    template <int NT>
+    __device__ __forceinline__ uint32_t reopen(uint32_t middles, const float* sval, const float4* bound) const {
+        uint32_t out = 0;
+        for (middles &= 0x5554u; middles; middles &= middles - 1) {  // halves of one sample hold nothing
+            const int m = __ffs(middles) - 1, len = m & -m, l = 31 - __clz(len);
+            const float dm = sval[(m - 1) * NT];
+            if (may_hold(l, at<NT>(m - len, sval), dm, bound)) out |= 1u << (m - len / 2);
+            if (may_hold(l, dm, at<NT>(m + len, sval), bound)) out |= 1u << (m + len / 2);
+        }
+        return out;
+    }
+};
+
+// Samples that a warp's 32 edges still want, dealt over its lanes
+constexpr int kWarpTasks = 128;  // at most four an edge at a time (EdgeSearch::open, reopen)
+struct WarpTasks {
+    float val[kWarpTasks], height[kWarpTasks];
+    uint16_t task[kWarpTasks];  // owner lane << 5 | sample
+};
+
+// 32 plain edges of the work list, one a lane of the warp:
+//   steps 0-1   the end densities
+//   steps 2-5   the bisection of the sign change
+//   step 6      rounds of further samples: the lanes' counts differ (on the caves
+//               sweep 7.2 / 7.8 / 9.1 of the 17 samples are evaluated at LOD0 /
+//               LOD1 / LOD2, 12 at LOD4 and 5, where an edge spans whole noise
+//               cells), so the wanted samples of all 32 edges are listed and
+//               every lane evaluates one of the list, whoever owns it
+//   steps 7-12  the normal (density_field.cl:137-150): six densities 0.001 apart
+//               at the crossing; the two along y share the crossing's height
+// All steps share one call site of the height term and one of the density,
+// because several copies of the noise code outgrow the instruction cache: with
+// a copy for the ends, the search and the normals the warps waited 2.4 cycles an
+// instruction for instructions, with one 0.3.
+// A heightfield's density at a height is one fma, so it has no steps 0-1, and
+// its y edges (one height) none before 7.
+template <int MODE, int NT, class N>
+__device__ __forceinline__ void hermite_edges(const BatchPtrs& b, const N& nz, int w, bool valid, bool yseg, float* sval,
+                                              WarpTasks* wt) {
+    const DensityParams& dp = b.density;
+    const int lane = threadIdx.x & 31;
+    const bool linear = b.crossing_mode != 0;
+    constexpr bool kCaves = MODE == LVN_DENSITY_CAVES;
+    int idx = -1;  // the lane's edge
+    HermiteEdge e{0.f, 0.f, 0.f, 0.f, 1, 0, 0};
+    const float* hm = nullptr;
+    const float4* bound = nullptr;  // the chunk's SearchBound entries of the edge's class
+    if (valid) {
         const int i = b.edge_work[w];
         const int c = b.edge_chunk[i];
-        const ChunkDesc& d = b.desc[c];
         const int key = b.edge_keys[i];
-        const int slot = b.s_on ? b.sslot[c] : -1;
-        const float* hm = b.hmap ? b.hmap + (size_t)c * Geo<VPC>::FD * Geo<VPC>::FD : nullptr;
-        b.edge_info[i] = w >= nplain ? hermite_brush<VPC>(b, d, key)
-                         : slot >= 0 ? hermite_sdens<VPC>(b, slot, key)
-                                     : hermite_density<VPC, MODE>(b, nz, d, key, hm);
+        if (b.s_on && b.sslot[c] >= 0) {
+            b.edge_info[i] = hermite_sdens(b, b.sslot[c], key);
+        } else {
+            idx = i;
+            e = hermite_edge(b.vpc, b.desc[c], key);
+            hm = b.hmap ? b.hmap + (size_t)c * (b.vpc + 2) * (b.vpc + 2) : nullptr;
+            bound = b.search ? b.search + (size_t)2 * kSearchLengths * c + (yseg ? 0 : kSearchLengths) : nullptr;
+        }
+    }
+    if (!__any_sync(FULL, idx >= 0)) return;
+    EdgeSearch s;
+    s.jump = 0.f;
+    float t = 0.f, nx = 0.f, ny = 0.f, nzv = 0.f;
+    float h0 = 0.f, h1 = 0.f;  // the end points' heights
+    if (hm) h0 = hm[e.c0], h1 = yseg ? h0 : hm[e.c1];
+    int step = 0, base = 0, total = 0, off = 0;
+    uint32_t want = 0;
+    for (;;) {
+        float x, y, z, h = h0;
+        bool needh = !yseg;
+        if (step < 2) {  // also where the height map is missing, for the heights alone
+            edge_point(e, (float)step, x, y, z);
+            needh = b.hmap == nullptr;
+            h = step ? h1 : h0;
+        } else if (step < 6) {
+            edge_point(e, (float)((s.lo + s.hi) >> 1) * 0.0625f, x, y, z);
+        } else if (step == 6) {
+            const int k = wt->task[min(base + lane, total - 1)];
+            HermiteEdge o;  // the owner's edge
+            const int src = k >> 5;
+            o.px = __shfl_sync(FULL, e.px, src), o.py = __shfl_sync(FULL, e.py, src), o.pz = __shfl_sync(FULL, e.pz, src);
+            o.step = __shfl_sync(FULL, e.step, src), o.axis = __shfl_sync(FULL, e.axis, src);
+            h = __shfl_sync(FULL, h0, src);
+            edge_point(o, (float)(k & 31) * 0.0625f, x, y, z);
+        } else {
+            edge_point(e, t, x, y, z);
+            const float d = 0.001f;
+            x = step == 7 ? x + d : step == 8 ? x - d : x;
+            z = step == 9 ? z + d : step == 10 ? z - d : z;
+            y = step == 11 ? y + d : step == 12 ? y - d : y;
+            needh = step < 11;
+            h = s.hbest;
+        }
+        if (needh) h = height_m<MODE>(nz, dp, x, z);
+        float v = dens_h<MODE>(nz, dp, h, x, y, z);
+        if (step < 2) {
+            if (step == 0) h0 = h, nx = v;
+            else h1 = h;
+            if (++step < 2) continue;
+            if (linear) {
+                const float den = nx - v;
+                t = fminf(fmaxf(den != 0.f ? nx / den : 0.5f, 0.f), 1.f);
+                edge_point(e, t, x, y, z);
+                s.hbest = height_m<MODE>(nz, dp, x, z);  // the linear mode has a call site of its own
+                step = 7;
+                continue;
+            }
+            s.start(nx, v);
+            if (kCaves) {
+                s.jump = edge_jump(dp, e);
+            } else if (yseg) {  // the heightfield's y edge: every sample of y - amp h
+                for (int m = 1; m < 16; m++) {
+                    edge_point(e, (float)m * 0.0625f, x, y, z);
+                    const float a = fabsf(dens_h<MODE>(nz, dp, h0, x, y, z));
+                    if (a < s.minv || (a == s.minv && m < s.best)) s.minv = a, s.best = m, s.hbest = h0;
+                }
+                t = s.best < 0 ? 0.f : (float)s.best * 0.0625f;
+                s.hbest = s.best < 0 ? 0.f : h0;
+                step = 7;
+            }
+            continue;
+        }
+        if (step < 6) {
+            const int m = (s.lo + s.hi) >> 1;
+            s.take<NT>(m, v, h, sval);
+            if ((v < 0.f) == (s.d0 < 0.f)) s.lo = m;
+            else s.hi = m;
+            if (++step < 6) continue;
+            want = idx >= 0 ? s.open<NT>(sval, bound) : 0u;
+        } else if (step == 6) {
+            if (base + lane < total) wt->val[base + lane] = v, wt->height[base + lane] = h;
+            base += 32;
+            if (base < total) continue;
+            __syncwarp();
+            int k = off;
+            for (uint32_t u = want; u; u &= u - 1, k++) s.take<NT>(__ffs(u) - 1, wt->val[k], wt->height[k], sval);
+            want = s.reopen<NT>(want, sval, bound);
+            __syncwarp();  // the list is rewritten below
+        } else {
+            nx = step == 7 ? v : step == 8 ? nx - v : nx;
+            nzv = step == 9 ? v : step == 10 ? nzv - v : nzv;
+            ny = step == 11 ? v : step == 12 ? ny - v : ny;
+            if (++step <= 12) continue;
+            if (idx >= 0) {
+                normalize3(nx, ny, nzv);
+                b.edge_info[idx] = make_float4(nx, ny, nzv, t);
+            }
+            return;
+        }
+        // list the samples wanted next, each lane's in a run of its own
+        __syncwarp();
+        const int n = __popc(want);
+        const int incl = warp_inclusive(n);
+        total = __shfl_sync(FULL, incl, 31);
+        off = incl - n;
+        base = 0;
+        step = 6;
+        if (total > 0) {
+            int k = off;
+            for (uint32_t u = want; u; u &= u - 1) wt->task[k++] = (uint16_t)(lane << 5 | (__ffs(u) - 1));
+            __syncwarp();
+        } else {
+            t = s.best < 0 ? 0.f : (float)s.best * 0.0625f;
+            if (s.best < 0) s.hbest = 0.f;
+            else if (s.best == 0 || yseg) s.hbest = h0;
+            else if (s.best == 16) s.hbest = h1;
+            step = 7;
+        }
     }
 }
 
-template <int VPC, int MODE>
-__global__ void __launch_bounds__(kThreads) k_hermite(BatchPtrs b) {
+// A plain edge of the reference terrain: its ridged octaves have no curvature
+// bound, so all 17 samples of an x / z edge are evaluated; the heights around
+// the crossing share their simplices (terrain_near).
+template <class N>
+__device__ __forceinline__ float4 hermite_terrain(const BatchPtrs& b, const N& nz, const HermiteEdge& e, const float* hm) {
+    const float amp = 900.f;  // MAX_TERRAIN_HEIGHT
+    const bool yedge = e.axis == 1;
+    float t = 0.f, hbest = 0.f, x, y, z;
+    if (b.crossing_mode == 0) {
+        float minv = FLT_MAX, hy = 0.f;
+        if (yedge) hy = hm ? hm[e.c0] : nz.terrain(e.px, e.pz);
+        for (int i = 0; i <= 16; i++) {
+            edge_point(e, (float)i * 0.0625f, x, y, z);
+            const float h = yedge ? hy : (hm && (i == 0 || i == 16)) ? hm[i == 0 ? e.c0 : e.c1] : nz.terrain(x, z);
+            const float dv = fabsf(fmaf(-amp, h, y));
+            if (dv < minv) t = (float)i * 0.0625f, minv = dv, hbest = h;
+        }
+    } else {
+        float e0 = 0.f;
+        for (int j = 0; j < 3; j++) {  // both ends, then the crossing's height: one call site
+            edge_point(e, j == 2 ? t : (float)j, x, y, z);
+            hbest = nz.terrain(x, z);
+            const float v = fmaf(-amp, hbest, y);
+            if (j == 1) {
+                const float den = e0 - v;
+                t = fminf(fmaxf(den != 0.f ? e0 / den : 0.5f, 0.f), 1.f);
+            }
+            e0 = v;
+        }
+    }
+    edge_point(e, t, x, y, z);
+    const float o = 0.001f;
+    float2 hx, hz;
+    nz.terrain_near(x, z, make_float2(x + o, x - o), make_float2(z + o, z - o), o, hx, hz);
+    float nx = fmaf(-amp, hx.x, y) - fmaf(-amp, hx.y, y);
+    float ny = fmaf(-amp, hbest, y + o) - fmaf(-amp, hbest, y - o);
+    float nzv = fmaf(-amp, hz.x, y) - fmaf(-amp, hz.y, y);
+    normalize3(nx, ny, nzv);
+    return make_float4(nx, ny, nzv, t);
+}
+
+// The hermite work list: plain x / z edges, plain y edges, CSG-created edges,
+// in segments, 32 edges of one kind at a time (the x / z edges, which cost the
+// most, first).  Each warp starts with a group of its own, dealt CTA by CTA so
+// that every SM has as many, and takes further ones in turn.
+template <int MODE, int NT, class N>
+__device__ __forceinline__ void hermite_list(const BatchPtrs& b, const N& nz, float* sval, WarpTasks* wt) {
+    const int FD2 = (b.vpc + 2) * (b.vpc + 2);
+    const int lane = threadIdx.x & 31;
+    const int nxz = b.bs->total_xz, ny = b.bs->total_y, nc = b.bs->total_created;
+    const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const int bx = (nxz + 31) / 32, by = (ny + 31) / 32, bc = (nc + 31) / 32;
+    for (int j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < bx + by + bc;) {
+        const int seg = j < bx ? 0 : j < bx + by ? 1 : 2;
+        const int k = (seg == 0 ? j : seg == 1 ? j - bx : j - bx - by) * 32 + lane;
+        const bool valid = k < (seg == 0 ? nxz : seg == 1 ? ny : nc);
+        const int w = (seg == 0 ? 0 : seg == 1 ? nxz : nxz + ny) + k;
+        if (seg == 2 || MODE == LVN_DENSITY_REFERENCE) {
+            if (valid) {
+                const int i = b.edge_work[w];
+                const int c = b.edge_chunk[i], key = b.edge_keys[i];
+                const int slot = b.s_on ? b.sslot[c] : -1;
+                float4 r;
+                if (seg == 2) r = hermite_brush(b, b.desc[c], key);
+                else if (slot >= 0) r = hermite_sdens(b, slot, key);
+                else r = hermite_terrain(b, nz, hermite_edge(b.vpc, b.desc[c], key), b.hmap ? b.hmap + (size_t)c * FD2 : nullptr);
+                b.edge_info[i] = r;
+            }
+        } else {
+            hermite_edges<MODE == LVN_DENSITY_REFERENCE ? LVN_DENSITY_FBM2D : MODE, NT>(b, nz, w, valid, seg == 1, sval, wt);
+        }
+        int nj = 0;
+        if (lane == 0) nj = warps + atomicAdd(&b.bs->hermite_next, 1);
+        j = __shfl_sync(FULL, nj, 0);
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, kHermiteCtas) k_hermite(BatchPtrs b) {
+    constexpr bool kSearch = MODE != LVN_DENSITY_REFERENCE;
     __shared__ __align__(16) float sg[64];
+    __shared__ float sval[kSearch ? 15 * kThreads : 1];
+    __shared__ WarpTasks wt[kSearch ? kThreads / 32 : 1];
     stage_gradients(sg, b.grad);
     __syncthreads();
     if (b.bs->overflow) return;
-    hermite_list<VPC, MODE>(b, Noise{b.perm_t3, sg});
+    hermite_list<MODE, kThreads>(b, Noise{b.perm_t3, sg}, sval + threadIdx.x, wt + (threadIdx.x >> 5));
 }
 
-// The same for large batches: one 1024-thread CTA per SM holds the two
-// simplex lookup tables (kT3Bytes) in shared memory, so a table read is a
-// shared load with a 32-bit address instead of a read-only global load with
-// a 64-bit one (9% fewer instructions a 3D fBm).  Such a CTA takes an SM's
-// registers and most of its shared memory, leaving the stages beside hermite
-// in the batch DAG no room; on a large batch hermite's share of the step
-// outweighs that, on a small one it does not.
-template <int VPC, int MODE>
+// The same for large batches: one CTA per SM holds the two simplex lookup
+// tables (kT3Bytes) in shared memory, so a table read is a shared load with a
+// 32-bit address instead of a read-only global load with a 64-bit one (9%
+// fewer instructions a 3D fBm).  Such a CTA takes an SM's registers and most
+// of its shared memory, leaving the stages beside hermite in the batch DAG no
+// room; on a large batch hermite's share of the step outweighs that, on a
+// small one it does not.
+constexpr int kHermiteSmemBytes =
+    kT3Bytes + 15 * 4 * kHermiteSmemThreads + kHermiteSmemThreads / 32 * (int)sizeof(WarpTasks);
+
+template <int MODE>
 __global__ void __launch_bounds__(kHermiteSmemThreads, 1) k_hermite_smem(BatchPtrs b) {
-    extern __shared__ __align__(16) uint8_t stab[];  // the lookup tables
+    extern __shared__ __align__(16) uint8_t stab[];  // the lookup tables, the searches' densities and lists
     __shared__ __align__(16) float sg[64];
     if (b.bs->overflow) return;  // the same for every thread
     stage_gradients(sg, b.grad);
     const uint4* src = reinterpret_cast<const uint4*>(b.perm_t3);
     for (int i = threadIdx.x; i < kT3Bytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(stab)[i] = __ldg(src + i);
     __syncthreads();
-    hermite_list<VPC, MODE>(b, NoiseT<true>{stab, sg});
+    float* sval = reinterpret_cast<float*>(stab + kT3Bytes);
+    WarpTasks* wt = reinterpret_cast<WarpTasks*>(sval + 15 * kHermiteSmemThreads);
+    hermite_list<MODE, kHermiteSmemThreads>(b, NoiseT<true>{stab, sg}, sval + threadIdx.x, wt + (threadIdx.x >> 5));
+}
+
+// Batches too small to fill the GPU with an edge per thread: 16 lanes take an
+// edge together, one sample each, then one point of the normal each, so an
+// edge's 23 dependent density evaluations become two (three with a 3D term,
+// whose 17th sample has a turn of its own).
+template <int MODE>
+__global__ void __launch_bounds__(kThreads) k_hermite_wide(BatchPtrs b) {
+    const int FD2 = (b.vpc + 2) * (b.vpc + 2);
+    __shared__ __align__(16) float sg[64];
+    stage_gradients(sg, b.grad);
+    __syncthreads();
+    if (b.bs->overflow) return;
+    const Noise nz{b.perm_t3, sg};
+    const DensityParams& dp = b.density;
+    const int nplain = b.bs->total_xz + b.bs->total_y;
+    const int total = nplain + b.bs->total_created;
+    const int q = threadIdx.x & 15;
+    const int groups = (int)(gridDim.x * blockDim.x) >> 4;
+    // both groups of a warp stay in the loop together: w is the group's edge,
+    // clamped to the last one, whose result only its own group writes
+    for (int w1 = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; 2 * w1 < total; w1 += groups >> 1) {
+        const int wg = 2 * w1 + ((threadIdx.x >> 4) & 1), w = min(wg, total - 1);
+        const int i = b.edge_work[w];
+        const int c = b.edge_chunk[i];
+        const ChunkDesc& d = b.desc[c];
+        const int key = b.edge_keys[i];
+        const int slot = b.s_on ? b.sslot[c] : -1;
+        const bool plain = w < nplain && slot < 0;
+        if (!plain && q == 0 && wg == w)
+            b.edge_info[i] = w >= nplain ? hermite_brush(b, d, key) : hermite_sdens(b, slot, key);
+        if (!__any_sync(FULL, plain)) continue;
+        const HermiteEdge e = hermite_edge(b.vpc, d, key);
+        const float* hm = b.hmap ? b.hmap + (size_t)c * FD2 : nullptr;
+        const bool yedge = e.axis == 1;
+        float t = 0.f, hbest = 0.f;
+        if (b.crossing_mode) {
+            // lanes 0 and 1 the end points, then all of them the crossing's height
+            float x, y, z;
+            edge_point(e, (float)(q & 1), x, y, z);
+            const float v = dens_h<MODE>(nz, dp, height_m<MODE>(nz, dp, x, z), x, y, z);
+            const float e0 = __shfl_sync(FULL, v, threadIdx.x & 16), e1 = __shfl_sync(FULL, v, (threadIdx.x & 16) + 1);
+            const float den = e0 - e1;
+            t = fminf(fmaxf(den != 0.f ? e0 / den : 0.5f, 0.f), 1.f);
+            edge_point(e, t, x, y, z);
+            hbest = height_m<MODE>(nz, dp, x, z);
+        } else {
+            // lane q: sample q + 1, then sample 0; the first minimum wins
+            float minv = FLT_MAX, hy = 0.f;
+            int best = 0;
+            if (yedge) hy = hm ? hm[e.c0] : height_m<MODE>(nz, dp, e.px, e.pz);
+            for (int turn = 0; turn < 2; turn++) {
+                const int m = turn ? 0 : q + 1;
+                float x, y, z;
+                edge_point(e, (float)m * 0.0625f, x, y, z);
+                const float h = yedge ? hy
+                                : (hm && (m == 0 || m == 16)) ? hm[m == 0 ? e.c0 : e.c1]
+                                                              : height_m<MODE>(nz, dp, x, z);
+                const float a = fabsf(dens_h<MODE>(nz, dp, h, x, y, z));
+                if (a < minv || (a == minv && a < FLT_MAX)) minv = a, best = m, hbest = h;
+            }
+#pragma unroll
+            for (int o = 8; o; o >>= 1) {
+                const float a = __shfl_xor_sync(FULL, minv, o), h = __shfl_xor_sync(FULL, hbest, o);
+                const int m = __shfl_xor_sync(FULL, best, o);
+                if (a < minv || (a == minv && m < best)) minv = a, best = m, hbest = h;
+            }
+            if (!(minv < FLT_MAX)) best = 0, hbest = 0.f;
+            t = (float)best * 0.0625f;
+        }
+        // lanes 0-5: x + h, x - h, y + h, y - h, z + h, z - h
+        float px, py, pz;
+        edge_point(e, t, px, py, pz);
+        const int a = min(q >> 1, 2);
+        const float h = (q & 1) ? -0.001f : 0.001f;
+        const float x = a == 0 ? px + h : px, y = a == 1 ? py + h : py, z = a == 2 ? pz + h : pz;
+        const float hq = a == 1 ? hbest : height_m<MODE>(nz, dp, x, z);
+        const float v = dens_h<MODE>(nz, dp, hq, x, y, z);
+        const float diff = v - __shfl_down_sync(FULL, v, 1);
+        float nx = diff, ny = __shfl_down_sync(FULL, diff, 2), nzv = __shfl_down_sync(FULL, diff, 4);
+        if (q == 0 && plain && wg == w) {
+            normalize3(nx, ny, nzv);
+            b.edge_info[i] = make_float4(nx, ny, nzv, t);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2793,25 +3244,35 @@ cudaError_t launch_edge_scatter(const BatchPtrs& b, cudaStream_t s) {
 
 cudaError_t launch_hermite(const BatchPtrs& b, cudaStream_t s) {
     const int min_chunks = b.density.mode == LVN_DENSITY_CAVES ? kHermiteSmemMinChunksCaves : kHermiteSmemMinChunks;
-    const bool shared_tables = b.hermite_form == 1 || (b.hermite_form == 0 && b.n >= min_chunks);
-    if (shared_tables) {
-        // the tuned grid in 256-thread units per SM, as for the other stages:
-        // 4 units are one 1024-thread CTA per SM, 2 leave half the SMs free
-        const int per_sm = b.grid_per_sm[ST_HERMITE] > 0 ? b.grid_per_sm[ST_HERMITE] : 4;
-        const int g = std::max(1, b.num_sms * per_sm / (kHermiteSmemThreads / kThreads));
-        const int T = kHermiteSmemThreads, smem = kT3Bytes;
+    const int wide = b.density.mode == LVN_DENSITY_REFERENCE ? kHermiteWideFacesTerrain : kHermiteWideFaces;
+    if (b.hermite_form == 0 && b.n <= wide / (b.vpc * b.vpc)) {
+        const int g = persistent_grid(b, ST_HERMITE, 8);
         switch (b.density.mode) {
-            case LVN_DENSITY_REFERENCE: LVN_VPC_DISPATCH(b.vpc, (k_hermite_smem<V, LVN_DENSITY_REFERENCE><<<g, T, smem, s>>>(b))); break;
-            case LVN_DENSITY_FBM2D: LVN_VPC_DISPATCH(b.vpc, (k_hermite_smem<V, LVN_DENSITY_FBM2D><<<g, T, smem, s>>>(b))); break;
-            default: LVN_VPC_DISPATCH(b.vpc, (k_hermite_smem<V, LVN_DENSITY_CAVES><<<g, T, smem, s>>>(b))); break;
+            case LVN_DENSITY_REFERENCE: k_hermite_wide<LVN_DENSITY_REFERENCE><<<g, kThreads, 0, s>>>(b); break;
+            case LVN_DENSITY_FBM2D: k_hermite_wide<LVN_DENSITY_FBM2D><<<g, kThreads, 0, s>>>(b); break;
+            default: k_hermite_wide<LVN_DENSITY_CAVES><<<g, kThreads, 0, s>>>(b); break;
         }
         return cudaGetLastError();
     }
-    const int g = persistent_grid(b, ST_HERMITE, 8);
+    const bool shared_tables = b.hermite_form == 1 || (b.hermite_form == 0 && b.n >= min_chunks);
+    if (shared_tables) {
+        // one CTA per SM; a tuned shape of 2 (CTAs of other stages per SM) leaves
+        // half the SMs free
+        const int per_sm = b.grid_per_sm[ST_HERMITE] > 0 ? std::min(b.grid_per_sm[ST_HERMITE], 4) : 4;
+        const int g = std::max(1, b.num_sms * per_sm / 4);
+        const int T = kHermiteSmemThreads, smem = kHermiteSmemBytes;
+        switch (b.density.mode) {
+            case LVN_DENSITY_REFERENCE: k_hermite_smem<LVN_DENSITY_REFERENCE><<<g, T, smem, s>>>(b); break;
+            case LVN_DENSITY_FBM2D: k_hermite_smem<LVN_DENSITY_FBM2D><<<g, T, smem, s>>>(b); break;
+            default: k_hermite_smem<LVN_DENSITY_CAVES><<<g, T, smem, s>>>(b); break;
+        }
+        return cudaGetLastError();
+    }
+    const int g = persistent_grid(b, ST_HERMITE, kHermiteCtas);
     switch (b.density.mode) {
-        case LVN_DENSITY_REFERENCE: LVN_VPC_DISPATCH(b.vpc, (k_hermite<V, LVN_DENSITY_REFERENCE><<<g, kThreads, 0, s>>>(b))); break;
-        case LVN_DENSITY_FBM2D: LVN_VPC_DISPATCH(b.vpc, (k_hermite<V, LVN_DENSITY_FBM2D><<<g, kThreads, 0, s>>>(b))); break;
-        default: LVN_VPC_DISPATCH(b.vpc, (k_hermite<V, LVN_DENSITY_CAVES><<<g, kThreads, 0, s>>>(b))); break;
+        case LVN_DENSITY_REFERENCE: k_hermite<LVN_DENSITY_REFERENCE><<<g, kThreads, 0, s>>>(b); break;
+        case LVN_DENSITY_FBM2D: k_hermite<LVN_DENSITY_FBM2D><<<g, kThreads, 0, s>>>(b); break;
+        default: k_hermite<LVN_DENSITY_CAVES><<<g, kThreads, 0, s>>>(b); break;
     }
     return cudaGetLastError();
 }
@@ -2821,17 +3282,11 @@ cudaError_t launch_hermite(const BatchPtrs& b, cudaStream_t s) {
 cudaError_t set_kernel_attributes() {
     cudaError_t e = cudaSuccess;
     auto set = [&](const void* f) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kT3Bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kHermiteSmemBytes);
     };
-#define LVN_HERMITE_ATTR(V)                                        \
-    set((const void*)k_hermite_smem<V, LVN_DENSITY_REFERENCE>);    \
-    set((const void*)k_hermite_smem<V, LVN_DENSITY_FBM2D>);        \
-    set((const void*)k_hermite_smem<V, LVN_DENSITY_CAVES>);
-    LVN_HERMITE_ATTR(8)
-    LVN_HERMITE_ATTR(16)
-    LVN_HERMITE_ATTR(32)
-    LVN_HERMITE_ATTR(64)
-#undef LVN_HERMITE_ATTR
+    set((const void*)k_hermite_smem<LVN_DENSITY_REFERENCE>);
+    set((const void*)k_hermite_smem<LVN_DENSITY_FBM2D>);
+    set((const void*)k_hermite_smem<LVN_DENSITY_CAVES>);
     return e;
 }
 

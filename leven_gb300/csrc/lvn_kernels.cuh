@@ -106,6 +106,10 @@ struct BatchPtrs {
     // each chunk, written by the field kernels; null: hermite evaluates it
     float* hmap;                 // [n][FD * FD]
 
+    // the crossing search's interpolation bounds of each chunk, written by the
+    // reset kernel (null: the search evaluates every sample); see SearchBound
+    float4* search;              // [n][2 * kSearchLengths]
+
     // k_mesh_scatter writes triangles (scatter_what 1), seams (2) or both (0);
     // k_leaf and the vertex export take slice `slice` of `nslices` equal leaf
     // ranges (nslices <= 1: all of them)
@@ -121,6 +125,8 @@ struct BatchPtrs {
     const float4* prev_info;
     int prev_count;
 };
+
+constexpr int kSearchLengths = 4;   // interval lengths 2, 4, 8, 16 of the 17-sample search
 
 constexpr int kRowTile = 256;       // field / voxel rows per CTA in the dense stages
 constexpr int kTilePoints = 2048;

@@ -360,6 +360,133 @@ struct NoiseT {
         return fmaf(snoise3(px, py, pz), amplitude, noise);
     }
 
+    // ---- points close together ------------------------------------------------
+    // The central differences of a normal evaluate the terrain at points +-0.001
+    // apart, which nearly always lie in one simplex of every octave (its
+    // frequencies are no powers of two, so field points rarely meet a boundary;
+    // with the fBm densities they do at 5 to 40% of an octave's crossings, some
+    // lane of a warp nearly always, and sharing gains nothing there).  The
+    // functions below test that once, at the centre, and then share what the
+    // simplex alone decides (its lattice point, its corners, their gradients)
+    // among the points; every point's own arithmetic is that of snoise2,
+    // operation for operation, so the values keep their bits.  A lane whose
+    // points may straddle a simplex boundary takes the plain function.
+
+    // The distance to a cell or simplex boundary, in units of one octave's
+    // coordinates, beyond which a point `h` away along one axis decides its
+    // simplex as the centre does, in float arithmetic: an axis step of h moves a
+    // skewed coordinate by at most 4/3 h (the 2D skew: 1.37 h) and an offset
+    // difference by h, and the coordinates' products (`octave` + 2 roundings) and
+    // the sums on the way to a comparison err by a few 2^-24 of |coordinates|.
+    // NaN or infinite coordinates give a margin that no test passes.
+    __device__ __forceinline__ static float simplex_margin(float h, float abs_sum, int octave) {
+        return fmaf(1.8e-7f * (float)(octave + 10), abs_sum, 1.4f * h);
+    }
+
+    // snoise2 at (x2.x, y), (x2.y, y), (x, y2.x) and (x, y2.y), each within `h`
+    // of (x, y): the first two in nx, the others in ny
+    __device__ __forceinline__ void snoise2_near(float x, float y, float2 x2, float2 y2, float h, int octave, float2& nx,
+                                                 float2& ny) const {
+        const float F2 = 0.366025403784f;
+        const float G2 = 0.211324865405f;
+        const float C2 = 1.f - 2.f * G2;
+        const float s = (x + y) * F2;
+        const float ux = x + s, uy = y + s;
+        const float pix = floorf(ux), piy = floorf(uy);
+        const float t = (pix + piy) * G2;
+        const float ax = pix - t, ay = piy - t;
+        const float x0 = x - ax, y0 = y - ay;
+        const float fx = ux - pix, fy = uy - piy;
+        const float m = simplex_margin(h, fabsf(x) + fabsf(y), octave);
+        if (fminf(fx, fy) > m && fmaxf(fx, fy) < 1.f - m && fabsf(x0 - y0) > m) {
+            const bool xgt = x0 > y0;
+            const int b = ((int)piy & 255) * kT3Row + ((int)pix & 255);
+            const float2 ga = grad2(b), gb = grad2(b + (xgt ? 1 : kT3Row)), gc = grad2(b + kT3Row + 1);
+            const float2 X0 = sub2(x2, v2(ax)), Y0 = sub2(y2, v2(ay));
+            const float ox = xgt ? 1.f : 0.f, oy = xgt ? 0.f : 1.f;
+            const float2 n0x = corner2_x(ga, X0, y0), n0y = corner2_y(ga, x0, Y0);
+            const float2 n1x = corner2_x(gb, add2(sub2(X0, v2(ox)), v2(G2)), (y0 - oy) + G2);
+            const float2 n1y = corner2_y(gb, (x0 - ox) + G2, add2(sub2(Y0, v2(oy)), v2(G2)));
+            const float2 n2x = corner2_x(gc, sub2(X0, v2(C2)), y0 - C2);
+            const float2 n2y = corner2_y(gc, x0 - C2, sub2(Y0, v2(C2)));
+            nx = mul2s(v2(70.f), add2(add2(n0x, n1x), n2x));
+            ny = mul2s(v2(70.f), add2(add2(n0y, n1y), n2y));
+        } else {
+            nx = snoise2x2(x2, v2(y));
+            ny = snoise2x2(v2(x), y2);
+        }
+    }
+    // one snoise2 corner at two points that differ in x / in y
+    __device__ __forceinline__ float2 corner2_x(float2 g, float2 x, float y) const {
+        float2 t = max02(sub2(v2(0.5f), fma2(v2(y), v2(y), mul2(x, x))));
+        t = mul2(t, t);
+        return mul2s(mul2(t, t), fma2(v2(g.y), v2(y), mul2(v2(g.x), x)));
+    }
+    __device__ __forceinline__ float2 corner2_y(float2 g, float x, float2 y) const {
+        float2 t = max02(sub2(v2(0.5f), fma2(y, y, v2(__fmul_rn(x, x)))));
+        t = mul2(t, t);
+        return mul2s(mul2(t, t), fma2(v2(g.y), y, v2(__fmul_rn(g.x, x))));
+    }
+
+    // fbm2 at (x2.x, y), (x2.y, y) -> hx and (x, y2.x), (x, y2.y) -> hy, each
+    // within `h` of (x, y)
+    __device__ __forceinline__ void fbm2_near(int octaves, float frequency, float lacunarity, float persistence, float x,
+                                              float y, float2 x2, float2 y2, float h, float2& hx, float2& hy) const {
+        x = x * frequency, y = y * frequency;
+        x2 = mul2s(x2, v2(frequency)), y2 = mul2s(y2, v2(frequency));
+        h = h * fabsf(frequency);
+        float amplitude = 1.f;
+        hx = hy = v2(0.f);
+#pragma unroll 1
+        for (int i = 0; i < octaves; i++) {
+            float2 nx, ny;
+            snoise2_near(x, y, x2, y2, h, i, nx, ny);
+            hx = fma2(nx, v2(amplitude), hx);
+            hy = fma2(ny, v2(amplitude), hy);
+            amplitude = amplitude * persistence;
+            x = x * lacunarity, y = y * lacunarity;
+            x2 = mul2s(x2, v2(lacunarity)), y2 = mul2s(y2, v2(lacunarity));
+            h = h * fabsf(lacunarity);
+        }
+    }
+
+    // Whether one octave of 3D noise keeps its simplex over the 17 samples of an
+    // edge, in float arithmetic: p(w) are its points, w0 / w1 the ends' and wa /
+    // wb the first and last inner sample's coordinate along `axis`, o1 and o2 the
+    // other two coordinates in x, y, z order.  The inner samples lie between two
+    // whose cell and ranks agree with a margin; an end, which often lies on a
+    // boundary exactly (field points are multiples of a power of two), has to
+    // come out of snoise3's own comparisons alike.
+    __device__ __forceinline__ static bool same_simplex3(int axis, float w0, float wa, float wb, float w1, float o1,
+                                                         float o2, int octave) {
+        const float F3 = 0.333333333333f;
+        const float G3 = 0.166666666667f;
+        const float m = simplex_margin(0.f, fmaxf(fabsf(w0), fabsf(w1)) + fabsf(o1) + fabsf(o2), octave);
+        float cx = 0.f, cy = 0.f, cz = 0.f;  // the first inner sample's cell
+        int ranks = 0;
+        bool same = true;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float w = k == 0 ? wa : k == 1 ? wb : k == 2 ? w0 : w1;
+            const float x = axis == 0 ? w : o1, y = axis == 1 ? w : axis == 0 ? o1 : o2, z = axis == 2 ? w : o2;
+            const float s = ((x + y) + z) * F3;
+            const float ux = x + s, uy = y + s, uz = z + s;
+            const float pix = floorf(ux), piy = floorf(uy), piz = floorf(uz);
+            const float t = ((pix + piy) + piz) * G3;
+            const float x0 = x - (pix - t), y0 = y - (piy - t), z0 = z - (piz - t);
+            const int r = (x0 >= y0 ? 1 : 0) | (x0 >= z0 ? 2 : 0) | (y0 >= z0 ? 4 : 0);
+            if (k == 0) cx = pix, cy = piy, cz = piz, ranks = r;
+            same = same && pix == cx && piy == cy && piz == cz && r == ranks;
+            if (k < 2) {
+                const float fx = ux - pix, fy = uy - piy, fz = uz - piz;
+                // the two coordinates that stay give one and the same comparison
+                const float ra = axis == 2 ? fabsf(y0 - z0) : fabsf(x0 - y0), rb = axis == 1 ? fabsf(y0 - z0) : fabsf(x0 - z0);
+                same = same && fminf(fminf(fx, fy), fz) > m && fmaxf(fmaxf(fx, fy), fz) < 1.f - m && fminf(ra, rb) > m;
+            }
+        }
+        return same;
+    }
+
     // RidgedMultiFractal (noise.cl:42-81), RIDGED_MULTI_H == 1
     __device__ __forceinline__ float ridged(int octaves, float lacunarity, float gain, float offset, float x,
                                             float y) const {
@@ -399,6 +526,69 @@ struct NoiseT {
         float b2 = 0.6f * fbm2(2, 0.63f, 2.2f, 0.15f, px, pz);
         b2 = fmaf(b2, 0.5f, 0.5f);
         return fmaf(billow, r, b2);
+    }
+
+    // ridged at (x2.x, y), (x2.y, y) -> rx and (x, y2.x), (x, y2.y) -> ry, each
+    // within `h` of (x, y)
+    __device__ __forceinline__ void ridged_near(int octaves, float lacunarity, float gain, float offset, float x, float y,
+                                                float2 x2, float2 y2, float h, float2& rx, float2& ry) const {
+        float sig[4], noise[4];
+        float frequency = 1.f;
+#pragma unroll 1
+        for (int i = 0; i <= octaves; i++) {
+            if (i) {
+                x = x * lacunarity, y = y * lacunarity;
+                x2 = mul2s(x2, v2(lacunarity)), y2 = mul2s(y2, v2(lacunarity));
+                h = h * lacunarity;
+            }
+            float2 nx, ny;
+            snoise2_near(x, y, x2, y2, h, i, nx, ny);
+            const float n[4] = {nx.x, nx.y, ny.x, ny.y};
+            const float exponent = 1.f / frequency;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float s = offset - fabsf(n[k]);
+                if (i == 0) {
+                    sig[k] = s * s;
+                    noise[k] = sig[k];
+                } else {
+                    const float weight = fminf(fmaxf(sig[k] * gain, 0.f), 1.f);
+                    sig[k] = s * weight;
+                    noise[k] = fmaf(sig[k], exponent, noise[k]);
+                }
+            }
+            if (i) frequency = frequency * lacunarity;
+        }
+        const float inv = 1.f / (float)octaves;
+        rx = make_float2(noise[0] * inv, noise[1] * inv);
+        ry = make_float2(noise[2] * inv, noise[3] * inv);
+    }
+
+    // terrain at (x2.x, z), (x2.y, z) -> hx and (x, z2.x), (x, z2.y) -> hz, each
+    // within `h` of (x, z)
+    __device__ __forceinline__ void terrain_near(float x, float z, float2 x2, float2 z2, float h, float2& hx,
+                                                 float2& hz) const {
+        const float S = 1.f / 2000.f;
+        const float px = x * S, pz = z * S;
+        const float2 px2 = mul2s(x2, v2(S)), pz2 = mul2s(z2, v2(S));
+        h = h * S;
+        float2 rx, rz, bx, bz, cx, cz;
+        ridged_near(7, 2.114352f, 1.5241f, 1.f, px, pz, px2, pz2, h, rx, rz);
+        fbm2_near(4, 0.24f, 1.8754f, 0.433f, -4.33f * px, 7.98f * pz, mul2s(v2(-4.33f), px2), mul2s(v2(7.98f), pz2),
+                  7.98f * h, bx, bz);
+        fbm2_near(2, 0.63f, 2.2f, 0.15f, px, pz, px2, pz2, h, cx, cz);
+        const float r[4] = {rx.x, rx.y, rz.x, rz.y}, bl[4] = {bx.x, bx.y, bz.x, bz.y}, c[4] = {cx.x, cx.y, cz.x, cz.y};
+        float out[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float rr = 0.8f * r[k];
+            rr = fminf(fmaxf(rr, 0.f), 1.f);
+            const float billow = fmaf(0.5f, 0.6f * bl[k], 0.5f);
+            const float b2 = fmaf(0.6f * c[k], 0.5f, 0.5f);
+            out[k] = fmaf(billow, rr, b2);
+        }
+        hx = make_float2(out[0], out[1]);
+        hz = make_float2(out[2], out[3]);
     }
 
     // The height term h(x,z) of a heightfield density d = y - amp*h (+ caves)

@@ -157,7 +157,7 @@ struct BatchState {
     int32_t total_created;
     int32_t total_simp_verts;  // simplified mesh totals
     int32_t total_simp_tris;
-    int32_t pad[1];
+    int32_t hermite_next;      // next block of the hermite work list
 };
 
 // Octree simplification: a node's QEF in its own frame (origin at the node's
