@@ -438,7 +438,7 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
     LVN_CK(m->mats.ensure((size_t)F * n));
     LVN_CK(m->planes.ensure(sizeof(uint4) * 3 * (size_t)field_rows(m->vpc) * n));
     LVN_CK(m->hmap.ensure(sizeof(float) * (size_t)field_rows(m->vpc) * n));
-    LVN_CK(m->search.ensure(sizeof(float4) * 2 * kSearchLengths * (size_t)n));
+    LVN_CK(m->search.ensure(sizeof(float4) * kSearchEntries * (size_t)n));
     LVN_CK(m->edge_tiles.ensure(sizeof(int4) * (size_t)edge_tiles_per_chunk(m->vpc) * n));
     LVN_CK(m->vox_tiles.ensure(sizeof(int) * (size_t)vox_tiles_per_chunk(m->vpc) * n));
     LVN_CK(m->chunk_tile_off.ensure(sizeof(int) * (size_t)(n + 1)));
@@ -2034,17 +2034,18 @@ int lvn_debug_cuckoo(const uint32_t* keys, int32_t n, uint32_t prime, int32_t fl
 namespace lvn {
 
 // A bound on |amp3 * fbm3| as the kernels compute it, for the cave density
-// (0 for the heightfield densities, which have no 3D term).
-// |snoise3| <= 1.2972: each of a point's four simplex corners adds at most
-// (0.6 - r^2)^4 r |g| to the sum before the factor 32, with |g| <= 1.42532 for
-// the gradient table; the corners are among the lattice points within
-// sqrt(0.6) of the point, and the largest sum of (0.6 - r^2)^4 r over those
-// lattice points, over a 200^3 grid of one skewed cell, is 0.025074, plus
-// 0.003367 for the grid spacing (6 lattice points in range, each changing by at
-// most 0.6^4 per unit of distance).  32 * 1.42532 * 0.028441 = 1.2972.  fbm3
-// sums the octaves scaled by amplitudes 1, gain3, gain3^2, ...; the 0.1% on
-// top covers single-precision rounding of those sums and products.
-static float cave_band(const DensityParams& d) {
+// (0 for the heightfield densities, which have no 3D term), from a bound on
+// |snoise3|.  kNoise3Bound: a point's four simplex corners are among the
+// lattice points within sqrt(0.6) of it; the sum over those of the largest
+// 32 (0.6 - r^2)^4 |g . p| any gradient of the table gives is at most 0.9825 in
+// a cell (tests/test_search_bounds.py).  kSampleBound takes |g| r for |g . p|,
+// which no gradient reaches at every corner at once: 1.2972
+// (tests/test_cave_bound.py); the surrogate's samples are drawn by it.  fbm3
+// sums the octaves scaled by amplitudes 1, gain3, gain3^2, ...; the 0.1% on top
+// covers single-precision rounding of those sums and products.
+constexpr double kNoise3Bound = 1.0, kSampleBound = 1.2972;
+
+static float cave_band(const DensityParams& d, double bound) {
     if (d.mode != LVN_DENSITY_CAVES) return 0.f;
     double sum = 0.0;
     float a = 1.f;
@@ -2052,10 +2053,12 @@ static float cave_band(const DensityParams& d) {
         sum += std::fabs((double)a);
         a = a * d.gain3;
     }
-    const double band = std::fabs((double)d.amp3) * 1.2972 * sum * 1.001;
+    const double band = std::fabs((double)d.amp3) * bound * sum * 1.001;
     if (!(band < 1e30)) return INFINITY;  // non-finite parameters: every point is evaluated
     return std::nextafter((float)band, INFINITY);
 }
+
+float sample_band(const DensityParams& d) { return cave_band(d, kSampleBound); }
 
 // rem[s] = the same bound over fbm3's octaves 2s and up only (the octaves the
 // field kernel has not evaluated after s steps of two), plus 4e-3 for the
@@ -2074,14 +2077,14 @@ static void cave_remainders(const DensityParams& d, float* rem) {
         double sum = 0.0;
         for (size_t i = 2 * (size_t)s; i < amp.size(); i++) sum += amp[i];
         if (sum == 0.0) break;
-        const double r = std::fabs((double)d.amp3) * 1.2972 * sum * 1.001 + 4e-3;
+        const double r = std::fabs((double)d.amp3) * kNoise3Bound * sum * 1.001 + 4e-3;
         rem[s] = r < 1e30 ? std::nextafter((float)r, INFINITY) : INFINITY;
     }
 }
 
 void density_fields(const DensityParams& d, int32_t default_material, float* band, float* rem,
                     int32_t dom_by_solid[9]) {
-    *band = cave_band(d);
+    *band = cave_band(d, kNoise3Bound);
     cave_remainders(d, rem);
     for (int n = 0; n <= 8; n++) {
         int mats[8];

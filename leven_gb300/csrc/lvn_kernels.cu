@@ -469,7 +469,7 @@ __device__ __forceinline__ float simp_solve(const SimpQef& q, float s, float& ox
 // stage 0: reset per-chunk state
 // ---------------------------------------------------------------------------
 
-// Interpolation bounds of the crossing search (search_edges).  Along an edge
+// Interpolation bounds of the crossing search (EdgeSearch).  Along an edge
 // the density is a sum of octaves; between two samples `len` density units
 // apart an octave of 2D or 3D simplex noise of frequency f and amplitude a
 // stays within min(a H (f len)^2 u (1 - u) / 2, 2 a A) of the line through its
@@ -501,7 +501,8 @@ constexpr float kNoise3Slope = 14.f, kNoise2Slope = 11.5f;  // the gradient's 1-
 constexpr float kNoise3Jump = 0.0054f;                      // B
 constexpr int kJumpOctaves = 3;
 
-__device__ __forceinline__ void search_bounds(const DensityParams& dp, const ChunkDesc& d, int vpc, float4* out) {
+__device__ __forceinline__ void search_bounds(const DensityParams& dp, const ChunkDesc& d, int vpc, float cave_rem1,
+                                              float4* out) {
     float reach = 0.f;  // largest coordinate of the chunk's field
     for (int a = 0; a < 3; a++)
         reach = fmaxf(reach, fmaxf(fabsf((float)d.off[a]), fabsf((float)d.off[a] + (float)d.scale * (float)(vpc + 2))));
@@ -529,7 +530,7 @@ __device__ __forceinline__ void search_bounds(const DensityParams& dp, const Chu
         }
     }
     // y's rounding beyond 2^20; the rounding of the sums y - amp2 h + amp3 n is
-    // relative to their values (the 1e-6 of search_edges, and 1e-4 here)
+    // relative to their values (the 1e-6 of EdgeSearch, and 1e-4 here)
     const float round = far * 2.f * eps * reach + 1e-4f;
     for (int e = 0; e < 2 * kSearchLengths; e++) {
         const bool xz = e >= kSearchLengths;
@@ -557,6 +558,33 @@ __device__ __forceinline__ void search_bounds(const DensityParams& dp, const Chu
         if (!(Q + C < 1e30f)) Q = 0.f, C = __int_as_float(0x7f800000);
         out[e] = make_float4(Q, C, Q > 1e-30f ? 1.f / (8.f * Q) : 1e30f, 0.f);
     }
+    // The cave field's grid (k_field_caves), (T, stride in field points): over a
+    // grid of `len` density units the first two octaves lie within T - cave_rem1
+    // of the bilinear interpolation of their values at the grid points (a
+    // curvature term per axis, then jumps and rounding as above), so where y -
+    // amp2 h plus that interpolation exceeds T it has the density's sign.  The
+    // longest of 8, 4 and 2 units whose curvature terms stay below 0.35 of the
+    // other octaves' bound is taken (4 at 6 octaves of 1/64: 1.5 of 5.7 in T): a
+    // grid point costs what evaluating a point does, a larger T decides fewer.
+    float T = __int_as_float(0x7f800000), stride = 1.f;
+    if (dp.mode == LVN_DENSITY_CAVES && far == 0.f) {
+        float c1 = 0.f, fix = 0.f;
+        float f = fabsf(dp.freq3), a = fabsf(dp.amp3);
+        const float prod = pow2(dp.freq3) && pow2(dp.lacunarity3) ? 0.f : 1.f;
+        for (int k = 0; k < min(2, dp.octaves3); k++) {
+            c1 += a * kNoise3Curve * f * f * 0.25f;  // both axes, at one unit
+            fix += 2.f * a * (kNoise3Jump + kNoise3Slope * (2.2f + prod * (float)(k + 1)) * eps * f * reach + 1e-5f);
+            f *= fabsf(dp.lacunarity3);
+            a *= fabsf(dp.gain3);
+        }
+        int len = 8;
+        while (len >= 2 && !(c1 * (float)(len * len) <= 0.35f * cave_rem1)) len >>= 1;
+        if (len >= 2 && len > d.scale && len % d.scale == 0) {
+            stride = (float)(len / d.scale);
+            T = 1.001f * (c1 * (float)(len * len) + fix) + cave_rem1 + 1e-3f;
+        }
+    }
+    out[2 * kSearchLengths] = make_float4(T, stride, 0.f, 0.f);
 }
 
 __global__ void k_reset(BatchPtrs b) {
@@ -566,7 +594,7 @@ __global__ void k_reset(BatchPtrs b) {
         memset(&z, 0, sizeof(z));
         b.cs[i] = z;
         if (b.search && b.density.mode != LVN_DENSITY_REFERENCE)
-            search_bounds(b.density, b.desc[i], b.vpc, b.search + (size_t)2 * kSearchLengths * i);
+            search_bounds(b.density, b.desc[i], b.vpc, b.cave_rem[1], b.search + (size_t)kSearchEntries * i);
     }
     if (i == 0) {
         BatchState z;
@@ -717,10 +745,16 @@ __global__ void __launch_bounds__(96) k_field(BatchPtrs b) {
 // sign of base.  base rounds monotonically in y, so each column is solid below
 // a first row ya (base < -band) and air from a first row yb (base > band),
 // both found by bisection like the heightfield's crossing; only the rows
-// [ya, yb) between them need the 3D term.  Those points go to a shared list
-// that all lanes then evaluate, two octaves at a time, until the octaves left
-// cannot change the sign; their solid bits are gathered into the row words
-// with shared-memory atomics.
+// [ya, yb) between them need the 3D term.  On fine chunks the first two octaves
+// are evaluated on a coarse grid of the slice first (every fourth point and row
+// at LOD0, every second at LOD1), and their interpolation decides most of those
+// points (search_bounds).  On the 4096-chunk caves batch's LOD0 slices 70 M band
+// points become 8 M grid points and 24 M listed ones, 52 M paired octave
+// evaluations instead of 90 M; the kernel went from 2.50 to 2.24 ms (issue 70%
+// active), the heights and the row loop being the rest.
+// The points left go to a shared list that all lanes then evaluate, two octaves
+// at a time, until the octaves left cannot change the sign; their solid bits are
+// gathered into the row words with shared-memory atomics.
 constexpr int kCaveBatch = 1024;  // listed points per batch of the stepped evaluation
 
 template <int VPC>
@@ -730,7 +764,8 @@ __global__ void __launch_bounds__(96) k_field_caves(BatchPtrs b) {
     __shared__ float hs[G::FD];
     __shared__ uint32_t words[3][G::FD];
     __shared__ uint16_t list[G::FD * G::FD];
-    __shared__ int wsum[3];
+    __shared__ int wsum[3], wlo[3], whi[3], lcount;
+    __shared__ uint16_t bandrows[G::FD], gridrows[G::FD];  // a column's band rows; a grid column's first row, rows
     __shared__ uint16_t bidx[2][kCaveBatch];  // the undecided points of a batch, ping-pong
     __shared__ float bnoise[2][kCaveBatch];   // their fBm partial sums
     __shared__ int bcount[2];
@@ -774,78 +809,157 @@ __global__ void __launch_bounds__(96) k_field_caves(BatchPtrs b) {
         }
         yb = lo;
     }
-    // the warp's row words of the rows decided solid: every valid column is
-    // solid below the warp's lowest ya and none from its highest, so only the
-    // rows between need a ballot.  Lane l keeps rows l, l + 32 and l + 64.
-    {
-        const unsigned vmask = __ballot_sync(FULL, valid);
-        const int ymin = __reduce_min_sync(FULL, valid ? ya : G::FD);
-        const int ymax = __reduce_max_sync(FULL, valid ? ya : 0);
-        uint32_t w0 = 0, w1 = 0, w2 = 0;
-        for (int y = ymin; y < ymax; y++) {
-            const unsigned sb = __ballot_sync(FULL, y < ya);
-            if ((y & 31) == lane) {
-                w0 = y < 32 ? sb : w0;
-                w1 = y >= 32 && y < 64 ? sb : w1;
-                w2 = y >= 64 ? sb : w2;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int y = lane + 32 * k;
-            if (y < G::FD) words[warp][y] = y < ymin ? vmask : y >= ymax ? 0u : k == 0 ? w0 : k == 1 ? w1 : w2;
-        }
-    }
-    // list the band rows of every column: an exclusive scan of the counts
     const int cnt = valid ? yb - ya : 0;
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += v;
+    // rows with band points, over the CTA, and how many points there are
+    {
+        const int rlo = __reduce_min_sync(FULL, cnt > 0 ? ya : G::FD), rhi = __reduce_max_sync(FULL, cnt > 0 ? yb : 0);
+        const int sum = __reduce_add_sync(FULL, cnt);
+        if (lane == 0) wlo[warp] = rlo, whi[warp] = rhi, wsum[warp] = sum;
+        if (threadIdx.x == 0) lcount = 0;
     }
-    if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    int off = incl - cnt;
-    for (int w = 0; w < warp; w++) off += wsum[w];
-    const int nl = wsum[0] + wsum[1] + wsum[2];
-    for (int k = 0; k < cnt; k++) list[off + k] = (uint16_t)(x + G::FD * (ya + k));
-    __syncthreads();
-    // The listed points, a batch at a time, two fBm octaves a step.  After a
-    // step, a point whose partial density fma(amp3, noise, base) exceeds the
-    // bound on the octaves still to come (b.cave_rem) in magnitude keeps that
-    // sign whatever they add, so it is decided; the others carry their partial
-    // sum (the exact float the full loop holds there) to the next step through
-    // a compacted batch list, and the last step decides by the full density.
+    const int rlo = min(min(wlo[0], wlo[1]), wlo[2]), rhi = max(max(whi[0], whi[1]), whi[2]);
+    int nl = wsum[0] + wsum[1] + wsum[2];
+    float T = 0.f;
+    int S = 1;
+    if (b.search) {
+        const float4 q = b.search[(size_t)kSearchEntries * c + 2 * kSearchLengths];
+        T = q.x, S = (int)q.y;
+    }
+    // The grid: columns 0, S, .. past the last, rows from j0 past rhi; of each
+    // column only the rows around the band rows of the field columns it
+    // interpolates.
+    const int gx = (G::FD - 1) / S + 2, j0 = rlo / S, gy = nl > 0 ? (rhi - 1) / S + 2 - j0 : 0;
+    float* coarse = &bnoise[0][0];
+    static_assert((G::FD / 2 + 2) * (G::FD / 2 + 2) <= 2 * kCaveBatch, "the grid fits the partial sums' space");
+    bool grid = S > 1 && nl > 0;
+    if (grid) {  // the same for every thread
+        if (valid) bandrows[x] = cnt > 0 ? ya << 8 | yb : 0xff00;
+        __syncthreads();
+        int glo = 255, ghi = 0;
+        if (x < gx) {
+            for (int k = max(0, (x - 1) * S + 1); k <= min(G::FD - 1, (x + 1) * S - 1); k++) {
+                glo = min(glo, (int)bandrows[k] >> 8);
+                ghi = max(ghi, (int)bandrows[k] & 0xff);
+            }
+            glo /= S;
+            gridrows[x] = ghi > 0 ? glo << 8 | ((ghi - 1) / S + 2 - glo) : 0;
+        }
+        // evaluating a grid point has to save several band points
+        const int points = __reduce_add_sync(FULL, x < gx && ghi > 0 ? (ghi - 1) / S + 2 - glo : 0);
+        if (lane == 0) wlo[warp] = points;
+        __syncthreads();
+        grid = nl >= 3 * (wlo[0] + wlo[1] + wlo[2]);
+    }
     const int steps = dp.octaves3 > 0 ? (dp.octaves3 + 1) / 2 : 1;
-    for (int b0 = 0; b0 < nl; b0 += kCaveBatch) {
-        const int nb = min(kCaveBatch, nl - b0);
-        for (int st = 0; st < steps; st++) {
-            const int src = st & 1, dst = src ^ 1;
-            const int n_in = st == 0 ? nb : bcount[src];
-            __syncthreads();  // every thread has read n_in
-            if (threadIdx.x == 0) bcount[dst] = 0;
-            __syncthreads();
-            const bool last = st + 1 == steps;
-            const float rem = b.cave_rem[st + 1];
-            for (int k = threadIdx.x; k < n_in; k += blockDim.x) {
-                const int i = st == 0 ? list[b0 + k] : bidx[src][k];
-                const int y = i / G::FD, px = i - G::FD * y;
-                const float wy = (float)(y * scale + oy);
-                const float base = fmaf(-amp2, hs[px], wy);
-                const float noise = nz.fbm3_step(st, dp.octaves3, dp.freq3, dp.lacunarity3, dp.gain3,
-                                                 (float)(px * scale + ox), wy, wz, st == 0 ? 0.f : bnoise[src][k]);
-                const float v = fmaf(dp.amp3, noise, base);
-                if (last || !(fabsf(v) <= rem)) {
-                    if (v < 0.f) atomicOr(&words[px >> 5][y], 1u << (px & 31));
-                } else {
-                    const int slot = atomicAdd(&bcount[dst], 1);
-                    bidx[dst][slot] = (uint16_t)i;
-                    bnoise[dst][slot] = noise;
+    // Pass 0 evaluates the grid's points, pass 1 the listed points, a batch at a
+    // time, two fBm octaves a step (one call site for both: a second copy of the
+    // noise code outgrows the instruction cache).  After a step, a point whose
+    // partial density fma(amp3, noise, base) exceeds the bound on the octaves
+    // still to come (b.cave_rem) in magnitude keeps that sign whatever they add,
+    // so it is decided; the others carry their partial sum (the exact float the
+    // full loop holds there) to the next step through a compacted batch list, and
+    // the last step decides by the full density.
+    for (int pass = grid ? 0 : 1; pass < 2; pass++) {
+        if (pass == 1) {
+            // The warp's row words of the points decided: every valid column is
+            // solid below the warp's lowest ya and air from its highest yb (its
+            // highest ya where there is no grid), so only the rows between need a
+            // ballot.  Lane l keeps rows l, l + 32 and l + 64.  With a grid the
+            // undecided points are listed on the way, else every band point is.
+            const unsigned vmask = __ballot_sync(FULL, valid);
+            const int ymin = __reduce_min_sync(FULL, valid ? ya : G::FD);
+            const int ymax = __reduce_max_sync(FULL, valid ? (grid ? yb : ya) : 0);
+            uint32_t w0 = 0, w1 = 0, w2 = 0;
+            const int i = min(x, G::FD - 1) / S;
+            const float fx = (float)(min(x, G::FD - 1) - i * S) / (float)S, fs = 1.f / (float)S;
+            float lo = 0.f, hi = 0.f;
+            int row = -1;
+            for (int y = ymin; y < ymax; y++) {
+                bool solid = y < ya, open = false;
+                if (grid) {
+                    const int j = y / S;
+                    if (j != row) {  // the grid rows around y at this column
+                        row = j;
+                        const float* g0 = coarse + gx * min(max(j - j0, 0), gy - 2) + i;
+                        lo = fmaf(g0[1] - g0[0], fx, g0[0]);
+                        hi = fmaf(g0[gx + 1] - g0[gx], fx, g0[gx]);
+                    }
+                    const float v = fmaf(dp.amp3, fmaf(hi - lo, (float)(y - j * S) * fs, lo),
+                                         fmaf(-amp2, h, (float)(y * scale + oy)));
+                    const bool in = valid && y >= ya && y < yb, sure = fabsf(v) > T;
+                    solid = solid || (in && sure && v < 0.f);
+                    open = in && !sure;
+                    const unsigned ob = __ballot_sync(FULL, open);
+                    if (ob) {
+                        int at = 0;
+                        if (lane == 0) at = atomicAdd(&lcount, __popc(ob));
+                        at = __shfl_sync(FULL, at, 0) + __popc(ob & ((1u << lane) - 1u));
+                        if (open) list[at] = (uint16_t)(x + G::FD * y);
+                    }
+                }
+                const unsigned sb = __ballot_sync(FULL, valid && solid);
+                if ((y & 31) == lane) {
+                    w0 = y < 32 ? sb : w0;
+                    w1 = y >= 32 && y < 64 ? sb : w1;
+                    w2 = y >= 64 ? sb : w2;
                 }
             }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const int y = lane + 32 * k;
+                if (y < G::FD) words[warp][y] = y < ymin ? vmask : y >= ymax ? 0u : k == 0 ? w0 : k == 1 ? w1 : w2;
+            }
+            if (!grid) {
+                // list the band rows of every column: an exclusive scan of the counts
+                int off = warp_inclusive(cnt) - cnt;
+                for (int w = 0; w < warp; w++) off += wsum[w];
+                for (int k = 0; k < cnt; k++) list[off + k] = (uint16_t)(x + G::FD * (ya + k));
+            }
             __syncthreads();
-            if (bcount[dst] == 0) break;
+            if (grid) nl = lcount;
+        }
+        const int n = pass == 0 ? gx * gy : nl;
+        for (int b0 = 0; b0 < n; b0 += pass == 0 ? n : kCaveBatch) {
+            const int nb = pass == 0 ? n : min(kCaveBatch, n - b0);
+            for (int st = 0; st < (pass == 0 ? 1 : steps); st++) {
+                const int src = st & 1, dst = src ^ 1;
+                const int n_in = st == 0 ? nb : bcount[src];
+                __syncthreads();  // every thread has read n_in
+                if (threadIdx.x == 0) bcount[dst] = 0;
+                __syncthreads();
+                const bool last = st + 1 == steps;
+                const float rem = b.cave_rem[st + 1];
+                for (int k = threadIdx.x; k < n_in; k += blockDim.x) {
+                    int i = 0, px, y;
+                    if (pass == 0) {
+                        const int gj = k / gx, gi = k - gx * gj, rows = gridrows[gi];
+                        if (gj >= (rows & 0xff)) continue;
+                        i = ((rows >> 8) + gj - j0) * gx + gi;
+                        px = gi * S, y = ((rows >> 8) + gj) * S;
+                    } else {
+                        i = st == 0 ? list[b0 + k] : bidx[src][k];
+                        y = i / G::FD, px = i - G::FD * y;
+                    }
+                    const float wy = (float)(y * scale + oy);
+                    const float noise = nz.fbm3_step(st, dp.octaves3, dp.freq3, dp.lacunarity3, dp.gain3,
+                                                     (float)(px * scale + ox), wy, wz, st == 0 ? 0.f : bnoise[src][k]);
+                    if (pass == 0) {
+                        coarse[i] = noise;
+                        continue;
+                    }
+                    const float v = fmaf(dp.amp3, noise, fmaf(-amp2, hs[px], wy));
+                    if (last || !(fabsf(v) <= rem)) {
+                        if (v < 0.f) atomicOr(&words[px >> 5][y], 1u << (px & 31));
+                    } else {
+                        const int slot = atomicAdd(&bcount[dst], 1);
+                        bidx[dst][slot] = (uint16_t)i;
+                        bnoise[dst][slot] = noise;
+                    }
+                }
+                __syncthreads();
+                if (bcount[dst] == 0) break;
+            }
         }
     }
     __syncthreads();
@@ -1600,7 +1714,7 @@ __device__ __forceinline__ void hermite_edges(const BatchPtrs& b, const N& nz, i
             idx = i;
             e = hermite_edge(b.vpc, b.desc[c], key);
             hm = b.hmap ? b.hmap + (size_t)c * (b.vpc + 2) * (b.vpc + 2) : nullptr;
-            bound = b.search ? b.search + (size_t)2 * kSearchLengths * c + (yseg ? 0 : kSearchLengths) : nullptr;
+            bound = b.search ? b.search + (size_t)kSearchEntries * c + (yseg ? 0 : kSearchLengths) : nullptr;
         }
     }
     if (!__any_sync(FULL, idx >= 0)) return;

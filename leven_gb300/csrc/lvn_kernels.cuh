@@ -106,9 +106,10 @@ struct BatchPtrs {
     // each chunk, written by the field kernels; null: hermite evaluates it
     float* hmap;                 // [n][FD * FD]
 
-    // the crossing search's interpolation bounds of each chunk, written by the
-    // reset kernel (null: the search evaluates every sample); see SearchBound
-    float4* search;              // [n][2 * kSearchLengths]
+    // interpolation bounds of each chunk, written by the reset kernel (null: the
+    // crossing search evaluates every sample, the field kernel every band point);
+    // see search_bounds
+    float4* search;              // [n][kSearchEntries]
 
     // k_mesh_scatter writes triangles (scatter_what 1), seams (2) or both (0);
     // k_leaf and the vertex export take slice `slice` of `nslices` equal leaf
@@ -127,6 +128,7 @@ struct BatchPtrs {
 };
 
 constexpr int kSearchLengths = 4;   // interval lengths 2, 4, 8, 16 of the 17-sample search
+constexpr int kSearchEntries = 2 * kSearchLengths + 1;  // the search's two edge classes, the cave field's grid
 
 constexpr int kRowTile = 256;       // field / voxel rows per CTA in the dense stages
 constexpr int kTilePoints = 2048;

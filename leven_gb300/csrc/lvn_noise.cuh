@@ -350,14 +350,13 @@ struct NoiseT {
             pz = (pz * lacunarity) * lacunarity;
             amplitude = (amplitude * persistence) * persistence;
         }
-        if (2 * s + 1 < octaves) {
-            const float qx = px * lacunarity, qy = py * lacunarity, qz = pz * lacunarity;
-            const float2 n = snoise3x2(make_float2(px, qx), make_float2(py, qy), make_float2(pz, qz));
-            noise = fmaf(n.x, amplitude, noise);
-            amplitude = amplitude * persistence;
-            return fmaf(n.y, amplitude, noise);
-        }
-        return fmaf(snoise3(px, py, pz), amplitude, noise);
+        // the last octave of an odd number takes the paired code too, its second
+        // lane unused: one copy of the noise in the kernel
+        const float qx = px * lacunarity, qy = py * lacunarity, qz = pz * lacunarity;
+        const float2 n = snoise3x2(make_float2(px, qx), make_float2(py, qy), make_float2(pz, qz));
+        noise = fmaf(n.x, amplitude, noise);
+        amplitude = amplitude * persistence;
+        return 2 * s + 1 < octaves ? fmaf(n.y, amplitude, noise) : noise;
     }
 
     // ---- points close together ------------------------------------------------

@@ -37,6 +37,9 @@ void lod_colour_for(int min_leaf_size, float c[3]);
 // for n = 0..8.
 void density_fields(const DensityParams& d, int32_t default_material, float* band, float* rem,
                     int32_t dom_by_solid[9]);
+// The width about the heightfield's surface in which the surrogate's samples of
+// a density with a 3D term look for its zero set.
+float sample_band(const DensityParams& d);
 // Field-index box holding every point the operations can change.
 void csg_box_for(const Brush* ops, int n, const int32_t off[3], int scale, int fd, int32_t lo[3], int32_t hi[3]);
 
