@@ -139,6 +139,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 columns, not waited for: the registers hold them after tmem_wait16
+__device__ __forceinline__ void tmem_issue16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+// waits for this thread's loads; the operands keep their uses behind it
+__device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+
 // 16-byte global -> shared copies that stay in flight together
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
@@ -163,10 +181,22 @@ __device__ __forceinline__ float2 sigmoid2(float2 z) {
 __device__ __forceinline__ float2 silu_grad2(float2 z, float2 s) {  // s = sigmoid2(z)
     return mul2(s, fma2(z, sub2(v2(1.f), s), v2(1.f)));
 }
+// two values rounded to BF16, the first in the low half
+__device__ __forceinline__ uint32_t bf2_bits(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
 // sin(pi r), cos(pi r): r reduced to [-1, 1] exactly (an even number of half
 // turns removed), then the fast intrinsics on a small argument
 __device__ __forceinline__ void sincos_pi(float r, float& s, float& c) {
     r -= 2.f * rintf(0.5f * r);
+    __sincosf(3.14159265358979f * r, &s, &c);
+}
+// the same for |r| < 2^22: adding and subtracting 1.5 * 2^23 rounds r / 2 as
+// rintf does, off the special-function unit, which rintf shares with the sine
+// and cosine
+__device__ __forceinline__ void sincos_pi_small(float r, float& s, float& c) {
+    r -= 2.f * __fsub_rn(__fadd_rn(0.5f * r, 12582912.f), 12582912.f);
     __sincosf(3.14159265358979f * r, &s, &c);
 }
 
@@ -250,18 +280,26 @@ __global__ void k_to_bf16(const float* p, int n, __nv_bfloat16* wb, LayerMap lm)
 // ---------------------------------------------------------------------------
 // Fused inference: the whole network on 128-point tiles in one CTA.  The four
 // hidden layers' BF16 weights stay in shared memory for the kernel's life.
-// Three warpgroups each own a tile stream, a 128-column TMEM accumulator and an
-// activation tile: a warpgroup computes its tile's features into the tile,
-// its elected thread issues the layer's MMAs and commits to its mbarrier, and
-// its epilogue turns the accumulator into the next layer's operand (bias,
-// SiLU, BF16) in place, or into the density after the last layer.  While one
-// warpgroup is in an epilogue the tensor core works on the other's layer.
+// Three tile streams each own a 128-column TMEM accumulator, an activation tile
+// and two warpgroups: thread `row` of each owns tile row `row` (its TMEM lane),
+// the first in columns 0-63, the second in 64-127.  A stream computes its tile's
+// features into the tile, its elected thread issues the layer's MMAs and commits
+// to its mbarrier, and its epilogue turns the accumulator into the next layer's
+// operand (bias, SiLU, BF16) in place, or into the density after the last layer.
+// While one stream is in an epilogue the tensor core works on another's layer.
+// The special-function unit bounds it: 512 tanh and 96 sines and cosines a point,
+// 16 a clock and SM, are 1.2 ms of 9.2 M points, which take 1.81 ms (2.03 with one
+// warpgroup a stream, the accumulator loaded 32 columns at a time and waited for,
+// and rintf, also a special-function instruction, in the features).  ex2 runs at
+// twice that rate, but SiLU from four ex2 and a shared reciprocal cost 1.96 ms in
+// FP32 arithmetic; starting the streams out of phase changed nothing.
 // ---------------------------------------------------------------------------
 
 constexpr int kWbBytes = 2 * kWb;                 // 120 KB of weights
 constexpr int kActBytes = kTile * kHidden * 2;    // 32 KB per activation tile
-constexpr int kInferWG = 3;                       // warpgroups (tile streams) per CTA
-constexpr int kInferSmem = kWbBytes + kInferWG * kActBytes + (kLayers * kHidden + kHidden + 1) * 4;
+constexpr int kInferWG = 3;                       // tile streams per CTA, two warpgroups each
+constexpr int kInferThreads = 256 * kInferWG;
+constexpr int kInferSmem = kWbBytes + kInferWG * kActBytes + (kLayers * kHidden + kHidden + 4 + kInferWG * kTile) * 4;
 static_assert(kInferSmem <= 227 * 1024, "one CTA per SM");
 
 struct InferArgs {
@@ -278,29 +316,31 @@ struct InferArgs {
     int* status;
 };
 
-__device__ __forceinline__ void wg_sync(int wg) {  // named barrier of one warpgroup
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
+__device__ __forceinline__ void wg_sync(int wg) {  // named barrier of one stream's two warpgroups
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + wg) : "memory");
 }
-// named barrier of one warpgroup that also ORs a predicate across it
+// the same, which also ORs a predicate across the stream
 __device__ __forceinline__ bool wg_any(int wg, bool v) {
     uint32_t r;
     asm volatile(
-        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}"
+        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, 256, p;\nselp.u32 %0, 1, 0, q;\n}"
         : "=r"(r)
         : "r"((uint32_t)v), "r"(1 + wg)
         : "memory");
     return r != 0;
 }
 
-__global__ void __launch_bounds__(128 * kInferWG, 1) k_mlp_infer(InferArgs a) {
+__global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(InferArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bars[kInferWG];
     __shared__ uint32_t tmem_base;
     uint8_t* sW = smem;
     uint8_t* sAct = smem + kWbBytes;
     float* sBias = reinterpret_cast<float*>(sAct + kInferWG * kActBytes);  // [4][128] biases, w4[128], b4
+    float* sHead = sBias + kLayers * kHidden + kHidden + 4;  // the second halves' head sums
     const int warp = threadIdx.x >> 5;
-    const int wg = warp >> 2;
+    const int wg = warp >> 3;           // tile stream
+    const int half = (warp >> 2) & 1;   // columns 64 half .. + 63
     const int row = threadIdx.x & 127;  // tile row = TMEM lane
     // weights: layer l is N = 128 rows (out) x K = in_l, K-major core matrices
     constexpr uint32_t kLbo = (kTile / 8) * 128;  // 2048: 128 rows per K column of core matrices
@@ -358,31 +398,35 @@ __global__ void __launch_bounds__(128 * kInferWG, 1) k_mlp_infer(InferArgs a) {
         const float yc = fminf(fmaxf(c[1], a.dom.lo[1]), a.dom.hi[1]);
         const float y_out = c[1] - yc;
         c[1] = yc;
-        // features -> this row of the activation tile (12 core-matrix columns)
+        // features -> this row of the activation tile (12 core-matrix columns: 4
+        // an axis, sines then cosines), frequencies 8 half .. + 7
 #pragma unroll
         for (int ax = 0; ax < 3; ax++) {
             const float u = 2.f * (c[ax] - a.dom.lo[ax]) / (a.dom.hi[ax] - a.dom.lo[ax]) - 1.f;
-            __align__(16) __nv_bfloat16 sv[16], cv[16];
+            uint32_t sv[4], cv[4];
+            auto fill = [&](auto sincos) {
 #pragma unroll
-            for (int k = 0; k < kFreqs; k++) {
-                float s, co;
-                sincos_pi(a.ff.f[ax][k] * u, s, co);
-                sv[k] = __float2bfloat16_rn(s);
-                cv[k] = __float2bfloat16_rn(co);
-            }
-            const int c0 = ax * 4;  // 32 features = 4 core columns per axis
-            *reinterpret_cast<uint4*>(act + (c0 + 0) * kLbo + row * 16) = *reinterpret_cast<uint4*>(sv);
-            *reinterpret_cast<uint4*>(act + (c0 + 1) * kLbo + row * 16) = *reinterpret_cast<uint4*>(sv + 8);
-            *reinterpret_cast<uint4*>(act + (c0 + 2) * kLbo + row * 16) = *reinterpret_cast<uint4*>(cv);
-            *reinterpret_cast<uint4*>(act + (c0 + 3) * kLbo + row * 16) = *reinterpret_cast<uint4*>(cv + 8);
+                for (int k = 0; k < 8; k += 2) {
+                    float s0, c0, s1, c1;
+                    sincos(a.ff.f[ax][8 * half + k] * u, s0, c0);
+                    sincos(a.ff.f[ax][8 * half + k + 1] * u, s1, c1);
+                    sv[k / 2] = bf2_bits(s0, s1);
+                    cv[k / 2] = bf2_bits(c0, c1);
+                }
+            };
+            // the frequencies rise with k
+            if (fabsf(a.ff.f[ax][kFreqs - 1] * u) < 4194304.f) fill(sincos_pi_small);
+            else fill(sincos_pi);
+            *reinterpret_cast<uint4*>(act + (4 * ax + half) * kLbo + row * 16) = make_uint4(sv[0], sv[1], sv[2], sv[3]);
+            *reinterpret_cast<uint4*>(act + (4 * ax + 2 + half) * kLbo + row * 16) = make_uint4(cv[0], cv[1], cv[2], cv[3]);
         }
-        float y = b4;
+        float y = half ? 0.f : b4;
         for (int l = 0; l < kLayers && ok; l++) {
             fence_proxy_async();
             tc_fence_before();
             wg_sync(wg);
             tc_fence_after();
-            if (row == 0) {
+            if (row == 0 && half == 0) {
                 const uint64_t ad = umma_desc(act_addr, kLbo, 128), bd = umma_desc(w_addr + 2 * wb_off(l), kLbo, 128);
                 if (l == 0) umma_chain<kIn / 16>(tmem, ad, 2 * kLbo, bd, 2 * kLbo, kIdesc, false);
                 else umma_chain<kHidden / 16>(tmem, ad, 2 * kLbo, bd, 2 * kLbo, kIdesc, false);
@@ -396,33 +440,54 @@ __global__ void __launch_bounds__(128 * kInferWG, 1) k_mlp_infer(InferArgs a) {
                     break;
                 }
             phase ^= 1u;
-            ok = !wg_any(wg, late);  // the whole warpgroup takes the same path
+            ok = !wg_any(wg, late);  // the whole stream takes the same path
             tc_fence_after();
             if (!ok) break;
-            const float* bias = sBias + l * kHidden;
-#pragma unroll 1
-            for (int cc = 0; cc < kHidden / 32; cc++) {
-                float v[32];
-                tmem_ld32(tmem + lane_base + (uint32_t)(cc * 32), v);
+            const float4* bias = reinterpret_cast<const float4*>(sBias + l * kHidden);
+            // 16 columns at a time, the next 16 loaded from tensor memory meanwhile
+            const uint32_t acc = tmem + lane_base + (uint32_t)(64 * half);
+            uint32_t v[2][16];
+            tmem_issue16(acc, v[0]);
+            tmem_wait16(v[0]);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint32_t(&r)[16] = v[q & 1];
+                if (q < 3) tmem_issue16(acc + 16 * (q + 1), v[(q + 1) & 1]);
+                const int c0 = 64 * half + 16 * q;  // the first column
+                uint32_t h[8];
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 bj = bias[(c0 + j) / 4];
+                    const float2 z0 = add2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(bj.x, bj.y));
+                    const float2 z1 = add2(make_float2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])), make_float2(bj.z, bj.w));
+                    const float2 s0 = mul2(z0, sigmoid2(z0)), s1 = mul2(z1, sigmoid2(z1));
+                    h[j / 2] = bf2_bits(s0.x, s0.y);
+                    h[j / 2 + 1] = bf2_bits(s1.x, s1.y);
+                }
                 if (l < kLayers - 1) {
-                    __align__(16) __nv_bfloat16 h[32];
-#pragma unroll
-                    for (int j = 0; j < 32; j++) h[j] = __float2bfloat16_rn(silu(v[j] + bias[cc * 32 + j]));
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        *reinterpret_cast<uint4*>(act + (cc * 4 + q) * kLbo + row * 16) =
-                            *reinterpret_cast<uint4*>(h + 8 * q);
+                    *reinterpret_cast<uint4*>(act + (c0 / 8) * kLbo + row * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+                    *reinterpret_cast<uint4*>(act + (c0 / 8 + 1) * kLbo + row * 16) = make_uint4(h[4], h[5], h[6], h[7]);
                 } else {
+                    const float4* w = reinterpret_cast<const float4*>(w4);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        // the head reads the BF16 activation, as in training
-                        const float x = __bfloat162float(__float2bfloat16_rn(silu(v[j] + bias[cc * 32 + j])));
-                        y = fmaf(x, w4[cc * 32 + j], y);
+                    for (int j = 0; j < 16; j += 4) {  // the head reads the BF16 activation, as in training
+                        const float4 wj = w[(c0 + j) / 4];
+                        y = fmaf(__uint_as_float(h[j / 2] << 16), wj.x, y);
+                        y = fmaf(__uint_as_float(h[j / 2] & 0xffff0000u), wj.y, y);
+                        y = fmaf(__uint_as_float(h[j / 2 + 1] << 16), wj.z, y);
+                        y = fmaf(__uint_as_float(h[j / 2 + 1] & 0xffff0000u), wj.w, y);
                     }
                 }
+                if (q < 3) tmem_wait16(v[(q + 1) & 1]);
             }
         }
-        if (ok && p < a.n) a.out[p] = fmaf(y, a.out_scale, y_out);
+        if (!ok) break;
+        if (half) sHead[wg * kTile + row] = y;
+        wg_sync(wg);
+        if (!half) {
+            y += sHead[wg * kTile + row];
+            if (p < a.n) a.out[p] = fmaf(y, a.out_scale, y_out);
+        }
     }
     if (!ok) {
         // The MMAs this warpgroup committed did not signal within the poll
@@ -433,7 +498,7 @@ __global__ void __launch_bounds__(128 * kInferWG, 1) k_mlp_infer(InferArgs a) {
         // (a CTA that never frees them would stall every later allocation on
         // this SM), and the status flag makes the host discard the call's
         // results (LVN_ERR_DEVICE_STATUS), including anything a late MMA wrote.
-        if ((threadIdx.x & 127) == 0) atomicExch(a.status, 1);
+        if (row == 0 && half == 0) atomicExch(a.status, 1);
         uint32_t polls = 0;
         while (!mbar_try_wait(&bars[wg], phase ^ 1u) && ++polls < 4 * kWaitLimit) {
         }
@@ -517,10 +582,6 @@ struct TrainArgs {
 // byte offset of core-matrix column c (8 elements), row r of a 128-row image
 __device__ __forceinline__ uint32_t img_off(int c, int r) { return (uint32_t)c * kCoreCol + (uint32_t)r * 16u; }
 
-__device__ __forceinline__ uint32_t bf2_bits(float a, float b) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
 __device__ __forceinline__ uint4 pack8(const float* v) {
     return make_uint4(bf2_bits(v[0], v[1]), bf2_bits(v[2], v[3]), bf2_bits(v[4], v[5]), bf2_bits(v[6], v[7]));
 }
@@ -1099,7 +1160,7 @@ struct lvn_surrogate {
         a.status = status.as<int>();
         const int64_t tiles = (n + kTile - 1) / kTile;
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(num_sms, (tiles + kInferWG - 1) / kInferWG));
-        k_mlp_infer<<<grid, 128 * kInferWG, kInferSmem, stream>>>(a);
+        k_mlp_infer<<<grid, kInferThreads, kInferSmem, stream>>>(a);
         SG_CK(cudaGetLastError());
         return LVN_OK;
     }
