@@ -51,8 +51,10 @@ constexpr int kSmemQuads = 14336;   // hosts with more quads sort them in global
 constexpr int kQuadBlock = 256;     // leaves per CTA of the quad enumeration (hosts up to kSmemLeaves)
 constexpr int kBigQuadBlock = 512;  // leaves per CTA of the quad enumeration (larger hosts)
 constexpr size_t kLeafSmem = (size_t)kSortLeaves * 8;
-constexpr size_t kQuadSmem = (size_t)kSmemLeaves * 8;
-constexpr size_t kBigQuadSmem = (size_t)kSortLeaves * 8;
+constexpr int kBigSmemLeaves = 27136;  // of the larger class
+constexpr size_t kQuadSmem = (size_t)kSmemLeaves * 8 + (size_t)kQuadBlock * 12 * 2;
+constexpr size_t kBigQuadSmem = (size_t)kBigSmemLeaves * 8 + (size_t)kBigQuadBlock * 12 * 2;
+static_assert(kBigQuadSmem <= 226 * 1024 && kBigQuadBlock * 12 <= 65536, "shared memory, 16-bit list entries");
 constexpr size_t kSortSmem = (size_t)kSmemQuads * 16;
 constexpr int kSmallLeaves = 2048;  // leaf sorts up to this size run several CTAs per SM
 constexpr int kBucketBits = 6;      // leaves of larger hosts are sorted in 64 Morton-prefix buckets
@@ -86,6 +88,7 @@ struct SeamHost {
     int32_t size;
     int32_t unit;        // smallest leaf size among the gathered chunks
     int32_t lev;         // log2(2 size / unit)
+    int32_t inside;      // 1: no gathered leaf reaches out of its CLIPMAP_LEAF_SIZE block
     int32_t pair_begin;  // gathered (chunk, neighbour mask) pairs
     int32_t pair_end;
     int64_t sel_off;     // the host's selected seam nodes (room for every node of its pairs)
@@ -410,35 +413,92 @@ __global__ void __launch_bounds__(1024) k_seam_leaves(SeamArgs A, int cap) {
     }
 }
 
+// The 12 edges of a leaf that may carry a quad: those with a sign change and,
+// where `inside` says that no gathered leaf reaches out of its CLIPMAP_LEAF_SIZE
+// block, those around which the four regions of the leaf's size do not all lie
+// in one block.  (A leaf found for a region contains it, so it lies in the
+// region's block, and the straddle test below would drop the segment.)
+__device__ __forceinline__ uint32_t open_edges(int corners, const int32_t pos[3], int32_t s, bool inside) {
+    uint32_t cross = inside ? 0u : 0x3fu;  // bit 2 a + side: blocks change at that face of axis a
+    for (int a = 0; a < 3; a++)
+        for (int side = 0; side < 2; side++) {
+            const uint32_t line = (uint32_t)(pos[a] + side * s);
+            if ((line - (uint32_t)s) / CLIPMAP_LEAF_SIZE != line / CLIPMAP_LEAF_SIZE) cross |= 1u << (2 * a + side);
+        }
+    uint32_t out = 0;
+#pragma unroll
+    for (int e = 0; e < 12; e++) {
+        const int dir = e >> 2, a1 = dir == 0 ? 1 : 0, a2 = dir == 2 ? 1 : 2;
+        const int c0 = (int)((0x642054103210ull >> (4 * e)) & 15), c1 = c0 | (4 >> dir);
+        const bool sign = ((corners >> c0) ^ (corners >> c1)) & 1;
+        const bool reach = (cross >> (2 * a1 + cbit(c0, a1)) | cross >> (2 * a2 + cbit(c0, a2))) & 1;
+        if (sign && reach) out |= 1u << e;
+    }
+    return out;
+}
+
 // The quads of the leaves [first, first + block) of one host, unsorted,
 // with their recursion path keys.  The host's sorted entries are copied to
-// shared memory when they fit `cap`, else searched in global memory.
+// shared memory when they fit `cap`, else searched in global memory.  One thread
+// a leaf lists the edges that may carry a quad, a small part of the twelve (of a
+// 428-chunk frame's 6.5 M about 1 in 10); the searches then run over the list
+// with every lane busy.  Searched edge by edge in place, the two launches took
+// 0.62 ms.
 __global__ void __launch_bounds__(1024) k_seam_quads(SeamArgs A, int block, int cap) {
     extern __shared__ uint64_t smem[];
+    __shared__ int s_open;
+    uint16_t* open = reinterpret_cast<uint16_t*>(smem + cap);  // leaf of the block * 12 + edge
     const int2 it = A.items[blockIdx.x];
     const SeamHost h = A.hosts[it.x];
     const int n = A.counts[it.x];
     const uint64_t* ent = A.ent + h.leaf_off;
+    const int unit_log = log2_units(h.unit, 1);
+    const int r_end = min(n, it.y + block);
+    if (threadIdx.x == 0) s_open = 0;
+    __syncthreads();
+    for (int r0 = it.y + (threadIdx.x & ~31); r0 < r_end; r0 += blockDim.x) {
+        const int r = r0 + (threadIdx.x & 31);
+        uint32_t edges = 0;
+        if (r < r_end) {
+            const uint64_t me = ent[r];
+            int32_t pos[3];
+            unmorton(ent_code(me), h.lev, unit_log, pos);
+            for (int a = 0; a < 3; a++) pos[a] += h.min[a];
+            edges = open_edges(A.seams[A.leaves[h.leaf_off + r]].localspace_min[3] & 0xff, pos,
+                               h.unit << ent_size_log(me), h.inside != 0);
+        }
+        int inc = __popc(edges);
+        const int own = inc;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if ((threadIdx.x & 31) >= o) inc += t;
+        }
+        int at = 0;
+        if ((threadIdx.x & 31) == 31 && inc) at = atomicAdd(&s_open, inc);
+        at = __shfl_sync(0xffffffffu, at, 31) + inc - own;
+        for (; edges; edges &= edges - 1) open[at++] = (uint16_t)((r - it.y) * 12 + __ffs(edges) - 1);
+    }
+    __syncthreads();
+    const int n_open = s_open;
+    if (n_open == 0) return;  // the same for every thread
     if (n <= cap) {  // binary searches in shared memory
         for (int i = threadIdx.x; i < n; i += blockDim.x) smem[i] = ent[i];
         __syncthreads();
         ent = smem;
     }
-    const int unit_log = log2_units(h.unit, 1);
     LeafView v;
     v.ent = ent;
     v.n = n;
     v.lev = h.lev;
     v.unit_log = unit_log;
     v.root = 2 * h.size;
-    const int r_end = min(n, it.y + block);
-    for (int item = it.y * 12 + threadIdx.x; item < r_end * 12; item += blockDim.x) {
-        const int r = item / 12, e = item - 12 * r;
+    for (int k = threadIdx.x; k < n_open; k += blockDim.x) {
+        const int item = open[k];
+        const int r = it.y + item / 12, e = item % 12;
         const uint64_t me = ent[r];
-        const int corners = A.seams[A.leaves[h.leaf_off + r]].localspace_min[3] & 0xff;
         const int c0 = cEdgeVMap[e][0], c1 = cEdgeVMap[e][1];
-        const int m0 = (corners >> c0) & 1, m1 = (corners >> c1) & 1;
-        if (m0 == m1) continue;  // no sign change on the edge of the smallest leaf: no quad
+        const int corners = A.seams[A.leaves[h.leaf_off + r]].localspace_min[3] & 0xff;
+        const int m1 = (corners >> c1) & 1;
         const int dir = e >> 2;
         int j = 0;
         for (int q = 0; q < 4; q++)
@@ -775,15 +835,20 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         }
         std::sort(found.begin(), found.end());
         int unit = d.size / vpc;
+        // blocks are counted from world 0: a leaf of up to their size lies in one when the root is aligned to them
+        bool inside = true;
+        for (int a = 0; a < 3; a++) inside &= root_min[a] % CLIPMAP_LEAF_SIZE == 0;
         for (size_t k = 0; k < found.size();) {
             int mask = 0;
             const int c = found[k].first;
             for (; k < found.size() && found[k].first == c; k++) mask |= 1 << found[k].second;
             pairs.push_back(make_int4(c, mask, hi, 0));
             unit = std::min(unit, chunks[c].size / vpc);
+            inside &= chunks[c].size / vpc <= CLIPMAP_LEAF_SIZE;
         }
         h.pair_end = (int32_t)pairs.size();
         h.unit = unit;
+        h.inside = inside ? 1 : 0;
         h.lev = 0;
         while ((unit << h.lev) < 2 * d.size) h.lev++;
         if (h.lev > kMaxLevels) return LVN_ERR_INVALID;
@@ -958,7 +1023,7 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     if (!big_items.empty()) {
         SeamArgs B = A;
         B.items = w.items.p + n_small;
-        k_seam_quads<<<(int)big_items.size(), 1024, kBigQuadSmem, w.side>>>(B, kBigQuadBlock, kSortLeaves);
+        k_seam_quads<<<(int)big_items.size(), 1024, kBigQuadSmem, w.side>>>(B, kBigQuadBlock, kBigSmemLeaves);
         SM_TRY(cudaGetLastError());
         SM_TRY(cudaEventRecord(w.ev_join, w.side));
     }
