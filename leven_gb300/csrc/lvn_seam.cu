@@ -12,8 +12,7 @@
 // host, without building the tree:
 //   * the depth-first leaf order is the Morton order of the leaves' minimum
 //     corners (children are visited x << 2 | y << 1 | z), so the leaves are
-//     sorted by Morton key (in shared memory when they fit, else in global
-//     memory, which the L2 holds) and numbered by rank;
+//     sorted by Morton key (in parts that fit shared memory) and numbered by rank;
 //   * the recursion emits one quad per final edge segment: an edge of the
 //     smallest of the four leaves around it, all four present, not all four
 //     in one CLIPMAP_LEAF_SIZE block (the straddle test of ContourEdgeProc /
@@ -45,21 +44,19 @@ constexpr int kSlotBits = 15;                    // leaf sort entry: (morton << 
 constexpr int kRankBits = 15;                    // quad payload: 4 ranks of 15 bits, flip at bit 60
 static_assert(kMaxLeaves <= (1 << kRankBits) && kMaxLeaves <= (1 << kSlotBits), "rank bits");
 constexpr int kMaxLevels = 12;    // log2(2 host size / smallest leaf): path keys of 5 bits per level fit 64 bits
-constexpr int kSortLeaves = 28672;  // hosts with more leaves sort them in global memory
 constexpr int kSmemLeaves = 8192;   // hosts with more leaves search them in global memory
-constexpr int kSmemQuads = 14336;   // hosts with more quads sort them in global memory
 constexpr int kQuadBlock = 256;     // leaves per CTA of the quad enumeration (hosts up to kSmemLeaves)
 constexpr int kBigQuadBlock = 512;  // leaves per CTA of the quad enumeration (larger hosts)
-constexpr size_t kLeafSmem = (size_t)kSortLeaves * 8;
 constexpr int kBigSmemLeaves = 27136;  // of the larger class
 constexpr size_t kQuadSmem = (size_t)kSmemLeaves * 8 + (size_t)kQuadBlock * 12 * 2;
 constexpr size_t kBigQuadSmem = (size_t)kBigSmemLeaves * 8 + (size_t)kBigQuadBlock * 12 * 2;
 static_assert(kBigQuadSmem <= 226 * 1024 && kBigQuadBlock * 12 <= 65536, "shared memory, 16-bit list entries");
-constexpr size_t kSortSmem = (size_t)kSmemQuads * 16;
 constexpr int kSmallLeaves = 2048;  // leaf sorts up to this size run several CTAs per SM
 constexpr int kBucketBits = 6;      // leaves of larger hosts are sorted in 64 Morton-prefix buckets
 constexpr int kBuckets = 1 << kBucketBits;
-constexpr int kSmallQuads = 2048;   // as do quad sorts up to this size
+constexpr int kSmallQuads = 2048;   // as do quad sorts up to this size; larger sorts are split in kParts
+constexpr int kParts = 256;
+static_assert(kSmallLeaves == kSmallQuads, "k_seam_parts' shared memory");
 constexpr size_t kSmallLeafSmem = (size_t)kSmallLeaves * 8;
 constexpr size_t kSmallSortSmem = (size_t)kSmallQuads * 16;
 
@@ -116,6 +113,8 @@ struct SeamArgs {
     uint64_t* qkey;     // quad path keys
     uint64_t* qval;     // quad payloads (sorted by key after the sort kernel)
     const int2* items;  // quad enumeration: (host, first leaf)
+    int4* parts;        // split sorts' parts: (host, first, count, dealt)
+    int32_t* n_parts;
     // emit
     const int64_t* vout_off;
     const int64_t* tout_off;
@@ -389,27 +388,134 @@ __device__ uint64_t path_key(int32_t root, int dir, const int32_t line[3], int32
     return key;
 }
 
-// Leaf sort lsort[blockIdx.x] = (host, first, count): the host's slots
-// [first, first + count) sorted (in shared memory when they fit `cap`) to
-// A.ent and A.leaves at the same positions of the host's leaf range.  A
-// small host is one sort; a larger one a sort per Morton-prefix bucket, which
-// together order the whole host.
-__global__ void __launch_bounds__(1024) k_seam_leaves(SeamArgs A, int cap) {
+// Leaf sort lsort[blockIdx.x] = (host, first, count <= kSmallLeaves): the host's
+// slots [first, first + count) sorted in shared memory to A.ent and A.leaves at
+// the same positions of the host's leaf range.  A small host is one sort; a larger
+// one a sort per Morton-prefix bucket, which together order the whole host.
+__global__ void __launch_bounds__(256) k_seam_leaves(SeamArgs A) {
     extern __shared__ uint64_t smem[];
     const int4 it = A.lsort[blockIdx.x];
     const SeamHost h = A.hosts[it.x];
     const int n = it.z;
-    uint64_t* ent = A.sel + h.sel_off + it.y;
-    if (n <= cap) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) smem[i] = ent[i];
-        __syncthreads();
-        ent = smem;
-    }
-    block_sort<false>(ent, nullptr, n);
+    const uint64_t* ent = A.sel + h.sel_off + it.y;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) smem[i] = ent[i];
+    __syncthreads();
+    block_sort<false>(smem, nullptr, n);
     for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        const uint64_t e = ent[r];
+        const uint64_t e = smem[r];
         A.ent[h.leaf_off + it.y + r] = e;
         A.leaves[h.leaf_off + it.y + r] = A.slots[h.sel_off + (e & ((1u << kSlotBits) - 1))];
+    }
+}
+
+// Sorts too large for that are split first: one CTA deals a sort's entries into
+// 256 parts by the eight bits below their common prefix, and lists the parts that
+// are not empty for k_seam_parts.  (In one CTA a frame's largest leaf and quad
+// sorts, 10 to 20 thousand entries, took 172 and 143 us, on the call's critical
+// path.)  Leaves (Quads = false): sort lsort[blockIdx.x], dealt to A.ent.  Quads:
+// those of host list[blockIdx.x] when they are more than kSmallQuads, dealt to the
+// unused half of the host's quad range; without one (2 quads > 12 leaves) the
+// host is a single part where it lies.
+template <bool Quads>
+__global__ void __launch_bounds__(1024) k_seam_split(SeamArgs A, const int32_t* list) {
+    __shared__ unsigned long long lo, hi;
+    __shared__ int cursor[kParts], warp_sum[kParts / 32];
+    int host, first = 0, n;
+    if (Quads) {
+        host = list[blockIdx.x];
+        n = A.qcounts[host];
+        if (n <= kSmallQuads) return;
+    } else {
+        const int4 it = A.lsort[blockIdx.x];
+        host = it.x, first = it.y, n = it.z;
+    }
+    const SeamHost h = A.hosts[host];
+    const uint64_t* key = Quads ? A.qkey + h.quad_off : A.sel + h.sel_off + first;
+    const int t = threadIdx.x;
+    if (Quads && 2 * (int64_t)n > 12 * (int64_t)A.counts[host]) {
+        if (t == 0) A.parts[atomicAdd(A.n_parts, 1)] = make_int4(host, 0, n, 0);
+        return;
+    }
+    if (t == 0) lo = ~0ull, hi = 0ull;
+    if (t < kParts) cursor[t] = 0;
+    __syncthreads();
+    unsigned long long mn = ~0ull, mx = 0ull;
+    for (int i = t; i < n; i += blockDim.x) {
+        mn = min(mn, (unsigned long long)key[i]);
+        mx = max(mx, (unsigned long long)key[i]);
+    }
+    atomicMin(&lo, mn);
+    atomicMax(&hi, mx);
+    __syncthreads();
+    const int top = lo == hi ? 0 : 63 - __clzll((long long)(lo ^ hi));  // highest bit that differs
+    const int shift = max(0, top - 7);
+    for (int i = t; i < n; i += blockDim.x) atomicAdd(&cursor[(key[i] >> shift) & (kParts - 1)], 1);
+    __syncthreads();
+    int count = 0, inc = 0;
+    if (t < kParts) {
+        count = inc = cursor[t];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if ((t & 31) >= o) inc += v;
+        }
+        if ((t & 31) == 31) warp_sum[t >> 5] = inc;
+    }
+    __syncthreads();
+    if (t < kParts) {
+        int start = inc - count;
+        for (int w = 0; w < (t >> 5); w++) start += warp_sum[w];
+        cursor[t] = start;
+        if (count) A.parts[atomicAdd(A.n_parts, 1)] = make_int4(host, first + start, count, 1);
+    }
+    __syncthreads();
+    for (int i = t; i < n; i += blockDim.x) {
+        const uint64_t k = key[i];
+        const int at = atomicAdd(&cursor[(k >> shift) & (kParts - 1)], 1);
+        if (Quads) {
+            A.qkey[h.quad_off + n + at] = k;
+            A.qval[h.quad_off + n + at] = A.qval[h.quad_off + i];
+        } else {
+            A.ent[h.leaf_off + first + at] = k;
+        }
+    }
+}
+
+// The listed parts (host, first, count, dealt), each sorted to its place: leaf
+// entries and seam indices, or quad payloads.  A part that does not fit shared
+// memory (keys that crowd below a long common prefix more than once) is sorted
+// where it lies.
+template <bool Quads>
+__global__ void __launch_bounds__(256) k_seam_parts(SeamArgs A) {
+    extern __shared__ uint64_t smem[];
+    const int parts = *A.n_parts;
+    for (int p = blockIdx.x; p < parts; p += gridDim.x) {
+        const int4 it = A.parts[p];
+        const SeamHost h = A.hosts[it.x];
+        const int n = it.z;
+        const int64_t dealt = Quads && it.w ? A.qcounts[it.x] : 0;
+        uint64_t* key = Quads ? A.qkey + h.quad_off + dealt + it.y : A.ent + h.leaf_off + it.y;
+        uint64_t* val = Quads ? A.qval + h.quad_off + dealt + it.y : nullptr;
+        uint64_t *sk = key, *sv = val;
+        if (n <= kSmallLeaves) {
+            sk = smem;
+            sv = smem + kSmallLeaves;
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                sk[i] = key[i];
+                if (Quads) sv[i] = val[i];
+            }
+            __syncthreads();
+        }
+        block_sort<Quads>(sk, sv, n);
+        for (int r = threadIdx.x; r < n; r += blockDim.x) {
+            if (Quads) {
+                A.qval[h.quad_off + it.y + r] = sv[r];
+            } else {
+                const uint64_t e = sk[r];
+                key[r] = e;
+                A.leaves[h.leaf_off + it.y + r] = A.slots[h.sel_off + (e & ((1u << kSlotBits) - 1))];
+            }
+        }
+        __syncthreads();  // shared memory is reused
     }
 }
 
@@ -557,30 +663,25 @@ __global__ void __launch_bounds__(1024) k_seam_quads(SeamArgs A, int block, int 
     }
 }
 
-// The quads of host list[blockIdx.x] in the recursion's order: payloads
-// sorted in place, in shared memory when they fit `cap`.  With `only_above`,
-// hosts with at most that many quads are left to the other size class.
-__global__ void __launch_bounds__(1024) k_seam_qsort(SeamArgs A, const int32_t* list, int cap, int only_above) {
+// The quads of host list[blockIdx.x], at most kSmallQuads, in the recursion's
+// order: payloads sorted in place.
+__global__ void __launch_bounds__(256) k_seam_qsort(SeamArgs A, const int32_t* list) {
     extern __shared__ uint64_t smem[];
     const int hi = list[blockIdx.x];
     const SeamHost h = A.hosts[hi];
     const int nq = A.qcounts[hi];
-    if (nq <= only_above || (only_above < 0 && nq > kSmallQuads)) return;
+    if (nq > kSmallQuads) return;
     uint64_t* key = A.qkey + h.quad_off;
     uint64_t* val = A.qval + h.quad_off;
-    if (nq <= cap) {
-        uint64_t* sk = smem;
-        uint64_t* sv = smem + cap;
-        for (int i = threadIdx.x; i < nq; i += blockDim.x) {
-            sk[i] = key[i];
-            sv[i] = val[i];
-        }
-        __syncthreads();
-        block_sort<true>(sk, sv, nq);
-        for (int i = threadIdx.x; i < nq; i += blockDim.x) val[i] = sv[i];
-    } else {
-        block_sort<true>(key, val, nq);
+    uint64_t* sk = smem;
+    uint64_t* sv = smem + kSmallQuads;
+    for (int i = threadIdx.x; i < nq; i += blockDim.x) {
+        sk[i] = key[i];
+        sv[i] = val[i];
     }
+    __syncthreads();
+    block_sort<true>(sk, sv, nq);
+    for (int i = threadIdx.x; i < nq; i += blockDim.x) val[i] = sv[i];
 }
 
 // vertices (hosts with triangles only) and triangles, back to back by host;
@@ -646,9 +747,9 @@ struct Grow {
 
 struct SeamWork {
     std::mutex mu;
-    int device = -1;
+    int device = -1, num_sms = 0;
     cudaStream_t stream = nullptr, side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr, ev_sorted = nullptr;
     Grow<SeamHost> hosts;
     Grow<int4> pairs;
     Grow<int4> chunks;
@@ -658,7 +759,8 @@ struct SeamWork {
     Grow<uint32_t> slots, leaves;
     Grow<int2> items;
     Grow<int32_t> lists, bcount, bstart, cursor;
-    Grow<int4> lsort;
+    Grow<int4> lsort, parts;
+    Grow<int32_t> n_parts;  // leaf parts, quad parts
     Grow<int32_t, true> hbuckets;  // pinned
     Grow<int64_t> offs;  // vertex offsets, triangle offsets
     Grow<lvn_mesh_vertex> vstage;
@@ -865,9 +967,9 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         SM_TRY(cudaEventCreateWithFlags(&w.ev_join, cudaEventDisableTiming));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_fork2, cudaEventDisableTiming));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_join2, cudaEventDisableTiming));
-        SM_TRY(cudaFuncSetAttribute(k_seam_leaves, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafSmem));
+        SM_TRY(cudaEventCreateWithFlags(&w.ev_sorted, cudaEventDisableTiming));
         SM_TRY(cudaFuncSetAttribute(k_seam_quads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBigQuadSmem));
-        SM_TRY(cudaFuncSetAttribute(k_seam_qsort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem));
+        SM_TRY(cudaDeviceGetAttribute(&w.num_sms, cudaDevAttrMultiProcessorCount, dev));
         w.device = dev;
     }
     if (num_hosts == 0) {
@@ -1004,29 +1106,39 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     SM_TRY(cudaMemcpyAsync(w.hosts.p, hv.data(), sizeof(SeamHost) * nh, cudaMemcpyHostToDevice, st));
     SM_TRY(cudaMemcpyAsync(w.items.p, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, st));
     SM_TRY(cudaMemsetAsync(w.qcounts.p, 0, sizeof(int32_t) * nh, st));
+    // a host has at most one split sort of quads; the quads' parts reuse the list of the leaves'
+    SM_TRY(w.parts.fit(kParts * std::max<size_t>(big_sorts.size(), nh)));
+    SM_TRY(w.n_parts.fit(2));
+    SM_TRY(cudaMemsetAsync(w.n_parts.p, 0, sizeof(int32_t) * 2, st));
+    A.parts = w.parts.p;
+    A.n_parts = w.n_parts.p;
     // the large hosts' sorts and enumeration beside the small hosts', on the second stream
     SM_TRY(cudaEventRecord(w.ev_fork, st));
     SM_TRY(cudaStreamWaitEvent(w.side, w.ev_fork, 0));
+    SeamArgs B = A;
+    B.lsort = w.lsort.p + small_sorts.size();
+    const int part_ctas = 4 * w.num_sms;
     if (!big_sorts.empty()) {
-        SeamArgs B = A;
-        B.lsort = w.lsort.p + small_sorts.size();
-        k_seam_leaves<<<(int)big_sorts.size(), 1024, kLeafSmem, w.side>>>(B, kSortLeaves);
+        k_seam_split<false><<<(int)big_sorts.size(), 1024, 0, w.side>>>(B, nullptr);
+        k_seam_parts<false><<<part_ctas, 256, kSmallSortSmem, w.side>>>(B);
         SM_TRY(cudaGetLastError());
+        SM_TRY(cudaEventRecord(w.ev_sorted, w.side));
     }
     if (!small_sorts.empty()) {
         A.lsort = w.lsort.p;
-        k_seam_leaves<<<(int)small_sorts.size(), 256, kSmallLeafSmem, st>>>(A, kSmallLeaves);
+        k_seam_leaves<<<(int)small_sorts.size(), 256, kSmallLeafSmem, st>>>(A);
         SM_TRY(cudaGetLastError());
     }
     SM_TRY(cudaEventRecord(w.ev_fork2, st));
     SM_TRY(cudaStreamWaitEvent(w.side, w.ev_fork2, 0));  // the enumeration reads every host's sorted leaves
     if (!big_items.empty()) {
-        SeamArgs B = A;
         B.items = w.items.p + n_small;
         k_seam_quads<<<(int)big_items.size(), 1024, kBigQuadSmem, w.side>>>(B, kBigQuadBlock, kBigSmemLeaves);
         SM_TRY(cudaGetLastError());
         SM_TRY(cudaEventRecord(w.ev_join, w.side));
     }
+    // a host of the small class may have had one of its buckets sorted on the side stream
+    if (!big_sorts.empty()) SM_TRY(cudaStreamWaitEvent(st, w.ev_sorted, 0));
     if (n_small) {
         k_seam_quads<<<n_small, 256, kQuadSmem, st>>>(A, kQuadBlock, kSmemLeaves);
         SM_TRY(cudaGetLastError());
@@ -1034,10 +1146,12 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     if (!big_items.empty()) SM_TRY(cudaStreamWaitEvent(st, w.ev_join, 0));
     SM_TRY(cudaEventRecord(w.ev_join, st));
     SM_TRY(cudaStreamWaitEvent(w.side, w.ev_join, 0));
-    // quad sorts: up to kSmallQuads quads in the small class, the rest (any host) on the side stream
-    k_seam_qsort<<<num_hosts, 256, kSmallSortSmem, st>>>(A, w.lists.p, kSmallQuads, -1);
+    // quad sorts: hosts of up to kSmallQuads quads here, the others in parts on the side stream
+    k_seam_qsort<<<num_hosts, 256, kSmallSortSmem, st>>>(A, w.lists.p);
     SM_TRY(cudaGetLastError());
-    k_seam_qsort<<<num_hosts, 1024, kSortSmem, w.side>>>(A, w.lists.p, kSmemQuads, kSmallQuads);
+    B.n_parts = w.n_parts.p + 1;
+    k_seam_split<true><<<num_hosts, 1024, 0, w.side>>>(B, w.lists.p);
+    k_seam_parts<true><<<part_ctas, 256, kSmallSortSmem, w.side>>>(B);
     SM_TRY(cudaGetLastError());
     SM_TRY(cudaEventRecord(w.ev_join2, w.side));
     SM_TRY(cudaStreamWaitEvent(st, w.ev_join2, 0));
