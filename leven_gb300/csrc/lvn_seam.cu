@@ -44,13 +44,7 @@ constexpr int kSlotBits = 15;                    // leaf sort entry: (morton << 
 constexpr int kRankBits = 15;                    // quad payload: 4 ranks of 15 bits, flip at bit 60
 static_assert(kMaxLeaves <= (1 << kRankBits) && kMaxLeaves <= (1 << kSlotBits), "rank bits");
 constexpr int kMaxLevels = 12;    // log2(2 host size / smallest leaf): path keys of 5 bits per level fit 64 bits
-constexpr int kSmemLeaves = 8192;   // hosts with more leaves search them in global memory
-constexpr int kQuadBlock = 256;     // leaves per CTA of the quad enumeration (hosts up to kSmemLeaves)
-constexpr int kBigQuadBlock = 512;  // leaves per CTA of the quad enumeration (larger hosts)
-constexpr int kBigSmemLeaves = 27136;  // of the larger class
-constexpr size_t kQuadSmem = (size_t)kSmemLeaves * 8 + (size_t)kQuadBlock * 12 * 2;
-constexpr size_t kBigQuadSmem = (size_t)kBigSmemLeaves * 8 + (size_t)kBigQuadBlock * 12 * 2;
-static_assert(kBigQuadSmem <= 226 * 1024 && kBigQuadBlock * 12 <= 65536, "shared memory, 16-bit list entries");
+constexpr int kQuadBlock = 256;     // leaves per CTA of the quad enumeration
 constexpr int kSmallLeaves = 2048;  // leaf sorts up to this size run several CTAs per SM
 constexpr int kBucketBits = 6;      // leaves of larger hosts are sorted in 64 Morton-prefix buckets
 constexpr int kBuckets = 1 << kBucketBits;
@@ -543,23 +537,22 @@ __device__ __forceinline__ uint32_t open_edges(int corners, const int32_t pos[3]
     return out;
 }
 
-// The quads of the leaves [first, first + block) of one host, unsorted,
-// with their recursion path keys.  The host's sorted entries are copied to
-// shared memory when they fit `cap`, else searched in global memory.  One thread
-// a leaf lists the edges that may carry a quad, a small part of the twelve (of a
-// 428-chunk frame's 6.5 M about 1 in 10); the searches then run over the list
-// with every lane busy.  Searched edge by edge in place, the two launches took
-// 0.62 ms.
-__global__ void __launch_bounds__(1024) k_seam_quads(SeamArgs A, int block, int cap) {
-    extern __shared__ uint64_t smem[];
+// The quads of the leaves [first, first + kQuadBlock) of one host, unsorted,
+// with their recursion path keys.  One thread a leaf lists the edges that may
+// carry a quad, a small part of the twelve (of a 428-chunk frame's 6.5 M about 1
+// in 10); the searches then run over the list with every lane busy (0.62 ms when
+// each edge was searched in place).  So few searches do not pay for a copy of the
+// host's entries in shared memory (0.09 ms for the hosts up to 8192 leaves beside
+// 0.09 for the others, against 0.13 for all).
+__global__ void __launch_bounds__(kQuadBlock) k_seam_quads(SeamArgs A) {
+    __shared__ uint16_t open[kQuadBlock * 12];  // leaf of the block * 12 + edge
     __shared__ int s_open;
-    uint16_t* open = reinterpret_cast<uint16_t*>(smem + cap);  // leaf of the block * 12 + edge
     const int2 it = A.items[blockIdx.x];
     const SeamHost h = A.hosts[it.x];
     const int n = A.counts[it.x];
     const uint64_t* ent = A.ent + h.leaf_off;
     const int unit_log = log2_units(h.unit, 1);
-    const int r_end = min(n, it.y + block);
+    const int r_end = min(n, it.y + kQuadBlock);
     if (threadIdx.x == 0) s_open = 0;
     __syncthreads();
     for (int r0 = it.y + (threadIdx.x & ~31); r0 < r_end; r0 += blockDim.x) {
@@ -586,12 +579,6 @@ __global__ void __launch_bounds__(1024) k_seam_quads(SeamArgs A, int block, int 
     }
     __syncthreads();
     const int n_open = s_open;
-    if (n_open == 0) return;  // the same for every thread
-    if (n <= cap) {  // binary searches in shared memory
-        for (int i = threadIdx.x; i < n; i += blockDim.x) smem[i] = ent[i];
-        __syncthreads();
-        ent = smem;
-    }
     LeafView v;
     v.ent = ent;
     v.n = n;
@@ -749,7 +736,7 @@ struct SeamWork {
     std::mutex mu;
     int device = -1, num_sms = 0;
     cudaStream_t stream = nullptr, side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr, ev_sorted = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_sorted = nullptr;
     Grow<SeamHost> hosts;
     Grow<int4> pairs;
     Grow<int4> chunks;
@@ -965,10 +952,8 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         SM_TRY(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_fork, cudaEventDisableTiming));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_join, cudaEventDisableTiming));
-        SM_TRY(cudaEventCreateWithFlags(&w.ev_fork2, cudaEventDisableTiming));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_join2, cudaEventDisableTiming));
         SM_TRY(cudaEventCreateWithFlags(&w.ev_sorted, cudaEventDisableTiming));
-        SM_TRY(cudaFuncSetAttribute(k_seam_quads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBigQuadSmem));
         SM_TRY(cudaDeviceGetAttribute(&w.num_sms, cudaDevAttrMultiProcessorCount, dev));
         w.device = dev;
     }
@@ -1067,7 +1052,7 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     }
     int64_t leaf_total = 0, quad_total = 0;
     bool limit = false;
-    std::vector<int2> items, big_items;  // (host, first leaf) of the quad enumeration's CTAs
+    std::vector<int2> items;  // (host, first leaf) of the quad enumeration's CTAs
     for (size_t i = 0; i < nh; i++) {
         const int n = w.hcounts.p[i];
         limit |= n > kMaxLeaves;
@@ -1075,10 +1060,7 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         hv[i].quad_off = quad_total;
         leaf_total += n;
         quad_total += 12 * (int64_t)n;
-        if (n <= kSmemLeaves)
-            for (int r = 0; r < n; r += kQuadBlock) items.push_back(make_int2((int)i, r));
-        else
-            for (int r = 0; r < n; r += kBigQuadBlock) big_items.push_back(make_int2((int)i, r));
+        for (int r = 0; r < n; r += kQuadBlock) items.push_back(make_int2((int)i, r));
     }
     if (limit) return LVN_ERR_DEVICE_STATUS;
     // 2: sorted leaves, quads, quads in order
@@ -1086,7 +1068,7 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     SM_TRY(w.leaves.fit(std::max<int64_t>(leaf_total, 1)));
     SM_TRY(w.qkey.fit(std::max<int64_t>(quad_total, 1)));
     SM_TRY(w.qval.fit(std::max<int64_t>(quad_total, 1)));
-    SM_TRY(w.items.fit(std::max<size_t>(items.size() + big_items.size(), 1)));
+    SM_TRY(w.items.fit(std::max<size_t>(items.size(), 1)));
     SM_TRY(w.lists.fit(nh));
     std::vector<int32_t> lists(nh);
     for (size_t i = 0; i < nh; i++) lists[i] = (int32_t)i;
@@ -1096,8 +1078,6 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     std::vector<int4> sorts(small_sorts);
     sorts.insert(sorts.end(), big_sorts.begin(), big_sorts.end());
     SM_TRY(cudaMemcpyAsync(w.lsort.p, sorts.data(), sizeof(int4) * n_sorts, cudaMemcpyHostToDevice, st));
-    items.insert(items.end(), big_items.begin(), big_items.end());
-    const int n_small = (int)(items.size() - big_items.size());
     A.ent = w.ent.p;
     A.leaves = w.leaves.p;
     A.qkey = w.qkey.p;
@@ -1112,7 +1092,7 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     SM_TRY(cudaMemsetAsync(w.n_parts.p, 0, sizeof(int32_t) * 2, st));
     A.parts = w.parts.p;
     A.n_parts = w.n_parts.p;
-    // the large hosts' sorts and enumeration beside the small hosts', on the second stream
+    // the large sorts beside the small ones, on the second stream
     SM_TRY(cudaEventRecord(w.ev_fork, st));
     SM_TRY(cudaStreamWaitEvent(w.side, w.ev_fork, 0));
     SeamArgs B = A;
@@ -1129,21 +1109,11 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         k_seam_leaves<<<(int)small_sorts.size(), 256, kSmallLeafSmem, st>>>(A);
         SM_TRY(cudaGetLastError());
     }
-    SM_TRY(cudaEventRecord(w.ev_fork2, st));
-    SM_TRY(cudaStreamWaitEvent(w.side, w.ev_fork2, 0));  // the enumeration reads every host's sorted leaves
-    if (!big_items.empty()) {
-        B.items = w.items.p + n_small;
-        k_seam_quads<<<(int)big_items.size(), 1024, kBigQuadSmem, w.side>>>(B, kBigQuadBlock, kBigSmemLeaves);
-        SM_TRY(cudaGetLastError());
-        SM_TRY(cudaEventRecord(w.ev_join, w.side));
-    }
-    // a host of the small class may have had one of its buckets sorted on the side stream
     if (!big_sorts.empty()) SM_TRY(cudaStreamWaitEvent(st, w.ev_sorted, 0));
-    if (n_small) {
-        k_seam_quads<<<n_small, 256, kQuadSmem, st>>>(A, kQuadBlock, kSmemLeaves);
+    if (!items.empty()) {
+        k_seam_quads<<<(int)items.size(), kQuadBlock, 0, st>>>(A);
         SM_TRY(cudaGetLastError());
     }
-    if (!big_items.empty()) SM_TRY(cudaStreamWaitEvent(st, w.ev_join, 0));
     SM_TRY(cudaEventRecord(w.ev_join, st));
     SM_TRY(cudaStreamWaitEvent(w.side, w.ev_join, 0));
     // quad sorts: hosts of up to kSmallQuads quads here, the others in parts on the side stream
