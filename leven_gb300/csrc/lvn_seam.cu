@@ -771,93 +771,131 @@ int cuda_rc(cudaError_t e) {
         if (rc__ != LVN_OK) return rc__; \
     } while (0)
 
-// Open-addressing hash table of 64-bit keys (linear probing, never full).
-class FlatTable {
-   public:
-    void reserve(size_t n) {
-        size_t cap = 16;
-        while (cap < 4 * n) cap <<= 1;
-        keys_.assign(cap, kEmpty);
-        vals_.assign(cap, -1);
-        mask_ = cap - 1;
-    }
-    // inserts (key, val) unless key is present; returns false when it was
-    bool insert(uint64_t key, int32_t val) {
-        for (size_t i = slot(key);; i = (i + 1) & mask_) {
-            if (keys_[i] == key) return false;
-            if (keys_[i] == kEmpty) {
-                keys_[i] = key;
-                vals_[i] = val;
-                return true;
-            }
-        }
-    }
-    int32_t find(uint64_t key) const {  // -1 when absent
-        for (size_t i = slot(key);; i = (i + 1) & mask_) {
-            if (keys_[i] == key) return vals_[i];
-            if (keys_[i] == kEmpty) return -1;
-        }
-    }
-
-   private:
-    static constexpr uint64_t kEmpty = ~0ull;
-    size_t slot(uint64_t key) const { return (size_t)((key * 0x9e3779b97f4a7c15ull) >> 20) & mask_; }
-    std::vector<uint64_t> keys_;
-    std::vector<int32_t> vals_;
-    size_t mask_ = 0;
-};
-
 // The clipmap's active nodes (the chunks) and the nodes above them;
 // FindNode / FindActiveNodes (clipmap.cpp:982-1013, 1449-1479) over the
-// complete octree rooted at (root_min, root_size).  A node is keyed by its
-// root-relative position in CLIPMAP_LEAF_SIZE units (19 bits per axis: roots
-// up to 2^27) and log2(size / CLIPMAP_LEAF_SIZE).
-struct ActiveSet {
-    int32_t root_min[3];
-    int32_t root_size;
-    FlatTable active;  // -> chunk index
-    FlatTable above;   // nodes with an active node below them (value unused)
+// complete octree rooted at (root_min, root_size).  A node is its level
+// log2(size / CLIPMAP_LEAF_SIZE) and its root-relative position in units of its
+// size (19 bits per axis: roots up to 2^27); one open-addressing table maps both
+// kinds, so that a lookup tells an active node, a node above active ones and
+// nothing apart (two tables and a division per axis and level took 0.33 ms for
+// the 442 hosts of a frame).
+class ActiveSet {
+   public:
+    static constexpr int32_t kNone = -1, kAbove = -2;
 
-    uint64_t key(const int32_t mn[3], int32_t size) const {
-        int lg = 0;
-        while ((CLIPMAP_LEAF_SIZE << lg) < size) lg++;
-        uint64_t k = 0;
-        for (int a = 0; a < 3; a++) k = (k << 19) | (uint64_t)(((int64_t)mn[a] - root_min[a]) / CLIPMAP_LEAF_SIZE);
-        return (k << 5) | (uint64_t)lg;
+    ActiveSet(const int32_t rmin[3], int32_t rsize, int32_t num_chunks) : root_size_(rsize) {
+        for (int a = 0; a < 3; a++) root_min_[a] = rmin[a];
+        root_level_ = level(rsize);
+        size_t cap = 64;
+        while (cap < 8 * (size_t)num_chunks) cap <<= 1;
+        slots_.assign(cap, Slot{kEmpty, kNone});
+    }
+    static int level(int32_t size) {
+        int l = 0;
+        while ((CLIPMAP_LEAF_SIZE << l) < size) l++;
+        return l;
     }
     bool in_root(const int32_t mn[3], int32_t size) const {
         for (int a = 0; a < 3; a++) {
-            const int64_t rel = (int64_t)mn[a] - root_min[a];
-            if (rel < 0 || rel + size > root_size || rel % size) return false;
+            const int64_t rel = (int64_t)mn[a] - root_min_[a];
+            if (rel < 0 || rel + size > root_size_ || (rel & (size - 1))) return false;
         }
         return true;
     }
-    // the active nodes FindActiveNodes lists for the node (mn, size)
-    void find_active(const int32_t mn[3], int32_t size, std::vector<int>& out) const {
-        // an active node containing mn (the node itself or above it)
-        for (int32_t s = size; s <= root_size; s *= 2) {
-            int32_t a[3];
-            for (int k = 0; k < 3; k++) a[k] = root_min[k] + (int32_t)(((int64_t)mn[k] - root_min[k]) / s * s);
-            const int32_t c = active.find(key(a, s));
-            if (c >= 0) {
-                out.push_back(c);
-                return;
+    // adds chunk c; false when it is listed twice
+    bool add_active(const lvn_chunk_desc& d, int32_t c) {
+        const int l = level(d.size);
+        uint32_t u[3];
+        cell(d.min, l, u);
+        return insert(key(l, u[0], u[1], u[2]), c) == kNone;
+    }
+    // marks the nodes above an active one; false when one of them is active itself
+    bool add_above(const lvn_chunk_desc& d) {
+        int l = level(d.size);
+        uint32_t u[3];
+        cell(d.min, l, u);
+        for (l++; l <= root_level_; l++) {
+            for (uint32_t& x : u) x >>= 1;
+            const int32_t was = insert(key(l, u[0], u[1], u[2]), kAbove);
+            if (was >= 0) return false;
+            if (was == kAbove) break;
+        }
+        return true;
+    }
+    // visits the active nodes FindActiveNodes lists for the node (mn, size)
+    template <class F>
+    void find_active(const int32_t mn[3], int32_t size, F&& visit) const {
+        int l = level(size);
+        uint32_t u[3];
+        cell(mn, l, u);
+        int32_t v = find(key(l, u[0], u[1], u[2]));
+        if (v == kAbove) return descend(l, u[0], u[1], u[2], visit);
+        // else an active node containing it, where there is one
+        while (v == kNone && l < root_level_) {
+            l++;
+            for (uint32_t& x : u) x >>= 1;
+            v = find(key(l, u[0], u[1], u[2]));
+        }
+        if (v >= 0) visit(v);
+    }
+
+   private:
+    struct Slot {
+        uint64_t key;
+        int32_t val;
+    };
+    static constexpr uint64_t kEmpty = ~0ull;
+
+    void cell(const int32_t mn[3], int l, uint32_t u[3]) const {
+        for (int a = 0; a < 3; a++) u[a] = (uint32_t)(((int64_t)mn[a] - root_min_[a]) / CLIPMAP_LEAF_SIZE) >> l;
+    }
+    static uint64_t key(int l, uint32_t x, uint32_t y, uint32_t z) {
+        return (((((uint64_t)x << 19) | y) << 19) | z) << 5 | (uint64_t)l;
+    }
+    size_t slot(uint64_t k) const { return (size_t)((k * 0x9e3779b97f4a7c15ull) >> 20) & (slots_.size() - 1); }
+    int32_t find(uint64_t k) const {
+        for (size_t i = slot(k);; i = (i + 1) & (slots_.size() - 1)) {
+            if (slots_[i].key == k) return slots_[i].val;
+            if (slots_[i].key == kEmpty) return kNone;
+        }
+    }
+    // inserts (k, val) unless k is present; returns what was there
+    int32_t insert(uint64_t k, int32_t val) {
+        for (size_t i = slot(k);; i = (i + 1) & (slots_.size() - 1)) {
+            if (slots_[i].key == k) return slots_[i].val;
+            if (slots_[i].key == kEmpty) {
+                slots_[i] = Slot{k, val};
+                if (2 * ++used_ > slots_.size()) grow();
+                return kNone;
             }
         }
-        descend(mn, size, out);
     }
-    void descend(const int32_t mn[3], int32_t size, std::vector<int>& out) const {
-        if (size <= CLIPMAP_LEAF_SIZE || above.find(key(mn, size)) < 0) return;
-        const int32_t h = size / 2;
-        for (int i = 0; i < 8; i++) {
-            const int32_t c[3] = {mn[0] + ((i >> 2) & 1) * h, mn[1] + ((i >> 1) & 1) * h, mn[2] + (i & 1) * h};
-            const int32_t ci = active.find(key(c, h));
-            if (ci >= 0)
-                out.push_back(ci);
-            else
-                descend(c, h, out);
+    void grow() {
+        std::vector<Slot> old(2 * slots_.size(), Slot{kEmpty, kNone});
+        old.swap(slots_);
+        for (const Slot& s : old) {
+            if (s.key == kEmpty) continue;
+            size_t i = slot(s.key);
+            while (slots_[i].key != kEmpty) i = (i + 1) & (slots_.size() - 1);
+            slots_[i] = s;
         }
     }
+    template <class F>
+    void descend(int l, uint32_t x, uint32_t y, uint32_t z, F&& visit) const {
+        if (l == 0) return;
+        for (int i = 0; i < 8; i++) {
+            const uint32_t cx = 2 * x + ((i >> 2) & 1), cy = 2 * y + ((i >> 1) & 1), cz = 2 * z + (i & 1);
+            const int32_t v = find(key(l - 1, cx, cy, cz));
+            if (v >= 0) visit(v);
+            else if (v == kAbove) descend(l - 1, cx, cy, cz, visit);
+        }
+    }
+
+    int32_t root_min_[3];
+    int32_t root_size_;
+    int root_level_;
+    size_t used_ = 0;
+    std::vector<Slot> slots_;
 };
 
 }  // namespace
@@ -879,33 +917,24 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
     if (root_size < CLIPMAP_LEAF_SIZE || (root_size & (root_size - 1))) return LVN_ERR_INVALID;
     const int vpc = voxels_per_chunk;
     if (root_size > (1 << 27)) return LVN_ERR_INVALID;
-    ActiveSet act;
-    for (int a = 0; a < 3; a++) act.root_min[a] = root_min[a];
-    act.root_size = root_size;
-    act.active.reserve((size_t)num_chunks);
-    act.above.reserve((size_t)num_chunks * 4 + 16);
+    ActiveSet act(root_min, root_size, num_chunks);
     for (int c = 0; c < num_chunks; c++) {
         const lvn_chunk_desc& d = chunks[c];
         if (d.size < CLIPMAP_LEAF_SIZE || (d.size & (d.size - 1)) || !act.in_root(d.min, d.size) ||
             seam_offsets[c + 1] < seam_offsets[c])
             return LVN_ERR_INVALID;
-        if (!act.active.insert(act.key(d.min, d.size), c)) return LVN_ERR_INVALID;  // listed twice
+        if (!act.add_active(d, c)) return LVN_ERR_INVALID;  // listed twice
     }
-    for (int c = 0; c < num_chunks; c++) {
-        const lvn_chunk_desc& d = chunks[c];
-        for (int32_t s = d.size * 2; s <= root_size; s *= 2) {
-            int32_t a[3];
-            for (int k = 0; k < 3; k++) a[k] = root_min[k] + (int32_t)(((int64_t)d.min[k] - root_min[k]) / s * s);
-            // the clipmap's active nodes never overlap: an active node above an active node is an error
-            if (act.active.find(act.key(a, s)) >= 0) return LVN_ERR_INVALID;
-            if (!act.above.insert(act.key(a, s), 0)) break;
-        }
-    }
+    // the clipmap's active nodes never overlap: an active node above an active node is an error
+    for (int c = 0; c < num_chunks; c++)
+        if (!act.add_above(chunks[c])) return LVN_ERR_INVALID;
     const int64_t num_seams = num_chunks ? seam_offsets[num_chunks] : 0;
     if (seam_offsets && num_chunks && seam_offsets[0] != 0) return LVN_ERR_INVALID;
     // the gathered (chunk, neighbour mask) pairs of every host
     std::vector<SeamHost> hv(num_hosts);
     std::vector<int4> pairs;
+    std::vector<uint8_t> mask_of((size_t)num_chunks, 0);  // neighbour indices a chunk was reached through
+    std::vector<int32_t> touched;
     for (int hi = 0; hi < num_hosts; hi++) {
         if (hosts[hi] < 0 || hosts[hi] >= num_chunks) return LVN_ERR_INVALID;
         const lvn_chunk_desc& d = chunks[hosts[hi]];
@@ -913,25 +942,23 @@ int lvn_seam_generate(const lvn_chunk_desc* chunks, const int32_t* seam_offsets,
         for (int a = 0; a < 3; a++) h.min[a] = d.min[a];
         h.size = d.size;
         h.pair_begin = (int32_t)pairs.size();
-        std::vector<std::pair<int, int>> found;  // (chunk, neighbour index)
+        touched.clear();
         for (int i = 0; i < 8; i++) {
             const int32_t nmin[3] = {d.min[0] + ((i >> 2) & 1) * d.size, d.min[1] + ((i >> 1) & 1) * d.size,
                                      d.min[2] + (i & 1) * d.size};
             if (!act.in_root(nmin, d.size)) continue;  // Clipmap::findNode finds no node there
-            std::vector<int> cs;
-            act.find_active(nmin, d.size, cs);
-            for (int c : cs) found.push_back({c, i});
+            act.find_active(nmin, d.size, [&](int32_t c) {
+                if (!mask_of[c]) touched.push_back(c);
+                mask_of[c] |= (uint8_t)(1 << i);
+            });
         }
-        std::sort(found.begin(), found.end());
         int unit = d.size / vpc;
         // blocks are counted from world 0: a leaf of up to their size lies in one when the root is aligned to them
         bool inside = true;
         for (int a = 0; a < 3; a++) inside &= root_min[a] % CLIPMAP_LEAF_SIZE == 0;
-        for (size_t k = 0; k < found.size();) {
-            int mask = 0;
-            const int c = found[k].first;
-            for (; k < found.size() && found[k].first == c; k++) mask |= 1 << found[k].second;
-            pairs.push_back(make_int4(c, mask, hi, 0));
+        for (const int32_t c : touched) {
+            pairs.push_back(make_int4(c, mask_of[c], hi, 0));
+            mask_of[c] = 0;
             unit = std::min(unit, chunks[c].size / vpc);
             inside &= chunks[c].size / vpc <= CLIPMAP_LEAF_SIZE;
         }
