@@ -366,6 +366,12 @@ struct lvn_meshgen {
     DevBuf probe_pts, probe_plain, probe_s, gate_ok, sslot, sdens, lattices;
     HostBuf h_gate, h_sslot, h_lattices;
     HostBuf h_desc, h_brushes, h_cs, h_bs;
+    HostBuf h_mesh;  // where the kernels leave a single chunk's mesh for the host (mesh_stage)
+    // the last batch's field and edges for debug fetches, where they lie in a
+    // cached field (null: in the pools)
+    const uint8_t* dbg_mats = nullptr;
+    const int32_t* dbg_keys = nullptr;
+    const float4* dbg_info = nullptr;
     int64_t ecap = 0, vcap = 0, eslot_cap = 0, nslot_cap = 0, ntile_cap = 0;
     int64_t vert_cap = 0, tri_cap = 0, seam_cap = 0;
     int chunk_cap = 0;
@@ -561,6 +567,9 @@ std::array<int, 4> tune_key(const lvn_meshgen* m, int n) {
 BatchPtrs make_ptrs(lvn_meshgen* m, int n) {
     BatchPtrs b;
     std::memset(&b, 0, sizeof(b));
+    m->dbg_mats = nullptr;
+    m->dbg_keys = nullptr;
+    m->dbg_info = nullptr;
     std::array<int, ST_COUNT> shape{};
     if (stage_shapes(m, tune_key(m, n), &shape, nullptr))
         for (int st = 0; st < ST_COUNT; st++) b.grid_per_sm[st] = shape[st];
@@ -687,6 +696,7 @@ int enqueue_octree_stages(lvn_meshgen* m, const BatchPtrs& b) {
 struct DirectOut {
     void* dst[3];
     int64_t cap[3];
+    bool optional = false;  // an array that is too small is no error: the pools hold the mesh too
 };
 
 // All three outputs, in order, on one stream.
@@ -1122,7 +1132,7 @@ int run_fresh_batch(lvn_meshgen* m, std::vector<ChunkDesc>& descs, const std::ve
         m->last_fresh = true;
         m->last_desc = descs;
         const BatchState& bs = *m->h_bs.as<BatchState>();
-        if (direct && bs.status) return LVN_ERR_CAPACITY;  // a caller array was too small
+        if (direct && bs.status && !direct->optional) return LVN_ERR_CAPACITY;  // a caller array was too small
         if (bs.overflow) {
             const bool user_short = dev_out && ((bs.overflow & (OVF_QUADS | OVF_SEAMS)) ||
                                                 ((bs.overflow & OVF_NODES) && bs.total_nodes > b.vertex_cap &&
@@ -1168,6 +1178,106 @@ int copy_out(lvn_meshgen* m, void* dst, const void* src, size_t bytes, int memor
     if (bytes == 0) return LVN_OK;
     LVN_CK(cudaMemcpyAsync(dst, src, bytes, memory == LVN_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                            m->stream));
+    return LVN_OK;
+}
+
+// The side stream and events of pinned host outputs.
+int ensure_side(lvn_meshgen* m) {
+    if (m->side) return LVN_OK;
+    // exports take free SM slots ahead of the compute kernels they overlap
+    int lo = 0, hi = 0;
+    LVN_CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    LVN_CK(cudaStreamCreateWithPriority(&m->side, cudaStreamNonBlocking, hi));
+    LVN_CK(cudaEventCreateWithFlags(&m->ev_leaf, cudaEventDisableTiming));
+    LVN_CK(cudaEventCreateWithFlags(&m->ev_side, cudaEventDisableTiming));
+    return LVN_OK;
+}
+
+// ---- one chunk's mesh to the host -------------------------------------------
+
+// A single chunk's mesh is small, and copying its three arrays out of the pools
+// after the batch's synchronisation costs more than making them: 50 us of a 64^3
+// chunk's 170, 29 of a 16^3 chunk's 115 (and the second copy, from vectors to the
+// caller's arrays by cudaMemcpy, 40 and 21).  So the kernels write it to a pinned
+// buffer of the context as they do to pinned caller arrays, and a plain copy takes
+// it from there: 74 us and 121 us a call.  Sized for four times the vertices of a
+// level surface through the chunk; a mesh that does not fit is pulled from the
+// pools, which hold it as well.
+bool mesh_stage(lvn_meshgen* m, DirectOut* d) {
+    if (!m->host_writes) return false;
+    const int64_t face = (int64_t)m->vpc * m->vpc;
+    const int64_t nv = 4 * face, nt = 8 * face, ns = 2 * face;
+    const size_t bytes = sizeof(lvn_mesh_vertex) * (nv + ns) + sizeof(lvn_mesh_triangle) * nt;
+    if (!m->h_mesh.p) {
+        if (m->h_mesh.ensure(bytes) != cudaSuccess || ensure_side(m) != LVN_OK) {
+            cudaGetLastError();
+            m->h_mesh.release();
+            return false;
+        }
+    }
+    char* p = m->h_mesh.as<char>();  // vertices, seam nodes, triangles: each 16-byte aligned
+    d->dst[0] = p;
+    d->dst[2] = p + sizeof(lvn_mesh_vertex) * nv;
+    d->dst[1] = p + sizeof(lvn_mesh_vertex) * (nv + ns);
+    d->cap[0] = nv, d->cap[1] = nt, d->cap[2] = ns;
+    d->optional = true;
+    return true;
+}
+
+// The sizes of chunk 0's mesh, and where it lies in the pools.
+struct MeshView {
+    int32_t nv, nt, ns;
+    const lvn_mesh_vertex* v;
+    const lvn_mesh_triangle* t;
+    const lvn_seam_node* s;
+};
+MeshView pool_mesh(const lvn_meshgen* m) {
+    const ChunkState& cs = m->last_cs[0];
+    const bool simp = m->simp_threshold >= 0.f;
+    MeshView w;
+    w.nt = simp ? cs.simp_tris : 2 * cs.quads;
+    w.nv = w.nt > 0 ? (simp ? cs.simp_verts : cs.nodes) : 0;
+    w.ns = cs.seams;
+    w.v = m->vertices.as<lvn_mesh_vertex>() + (simp ? cs.simp_vert_off : cs.node_off);
+    w.t = m->triangles.as<lvn_mesh_triangle>() + (simp ? (size_t)cs.simp_tri_off : 2 * (size_t)cs.quad_off);
+    w.s = m->seams.as<lvn_seam_node>() + cs.seam_off;
+    return w;
+}
+
+// Host memory to a caller's host array: a plain copy (cudaMemcpy takes 7 us a
+// call before it moves a byte).  A null or device pointer is left to cudaMemcpy.
+int host_store(void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return LVN_OK;
+    cudaPointerAttributes at;
+    if (!dst || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeDevice) {
+        LVN_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToHost));
+        return LVN_OK;
+    }
+    std::memcpy(dst, src, bytes);
+    return LVN_OK;
+}
+
+// Chunk 0's mesh to the caller's arrays: from the staging buffer, or from the pools.
+int deliver_mesh(lvn_meshgen* m, const DirectOut* staged, lvn_mesh_out* out) {
+    const MeshView w = pool_mesh(m);
+    out->num_vertices = w.nv;
+    out->num_triangles = w.nt;
+    out->num_seams = w.ns;
+    if (w.nv > out->vertex_capacity || w.nt > out->triangle_capacity || w.ns > out->seam_capacity)
+        return LVN_ERR_CAPACITY;
+    const size_t bv = sizeof(lvn_mesh_vertex) * w.nv, bt = sizeof(lvn_mesh_triangle) * w.nt,
+                 bs = sizeof(lvn_seam_node) * w.ns;
+    if (staged) {
+        int rc = host_store(out->vertices, staged->dst[0], bv);
+        if (!rc) rc = host_store(out->triangles, staged->dst[1], bt);
+        if (!rc) rc = host_store(out->seams, staged->dst[2], bs);
+        return rc;
+    }
+    int rc = copy_out(m, out->vertices, w.v, bv, out->memory);
+    if (!rc) rc = copy_out(m, out->triangles, w.t, bt, out->memory);
+    if (!rc) rc = copy_out(m, out->seams, w.s, bs, out->memory);
+    if (rc) return rc;
+    LVN_CK(cudaStreamSynchronize(m->stream));
     return LVN_OK;
 }
 
@@ -1301,7 +1411,7 @@ int load_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry** 
 }
 
 // ConstructOctreeFromField + mesh + seams for one cached field
-int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry& f) {
+int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry& f, const DirectOut* staged) {
     std::vector<ChunkDesc> descs;
     int rc = one_desc(m, min, size, descs);
     if (rc) return rc;
@@ -1312,14 +1422,6 @@ int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEnt
     for (int attempt = 0; attempt < kMaxHashRetries; attempt++) {
         if ((rc = ensure_pools(m, 1, cap))) return rc;
         if ((rc = upload(m, descs, none))) return rc;
-        const size_t F = (size_t)field_size(m->vpc);
-        LVN_CK(cudaMemcpyAsync(m->mats.p, f.mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
-        LVN_CK(cudaMemcpyAsync(m->planes.p, f.planes.p, sizeof(uint4) * 3 * (size_t)field_rows(m->vpc),
-                               cudaMemcpyDeviceToDevice, m->stream));
-        LVN_CK(cudaMemcpyAsync(m->edge_keys.p, f.keys.p, sizeof(int32_t) * f.num_edges, cudaMemcpyDeviceToDevice,
-                               m->stream));
-        LVN_CK(cudaMemcpyAsync(m->edge_info.p, f.info.p, sizeof(float4) * f.num_edges, cudaMemcpyDeviceToDevice,
-                               m->stream));
         LVN_CK(cudaMemsetAsync(m->edge_chunk.p, 0, sizeof(int32_t) * std::max(1, f.num_edges), m->stream));
         ChunkState cs;
         std::memset(&cs, 0, sizeof(cs));
@@ -1344,7 +1446,16 @@ int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEnt
         LVN_CK(cudaMemcpyAsync(m->bs.p, m->h_bs.p, sizeof(bs), cudaMemcpyHostToDevice, m->stream));
         BatchPtrs b = make_ptrs(m, 1);
         b.derive_mats = 0;  // the cached field may hold CSG materials
+        // the octree stages only read the field and its edges: no copy to the pools
+        b.mats = f.mats.as<uint8_t>();
+        b.planes = f.planes.as<uint4>();
+        b.edge_keys = f.keys.as<int32_t>();
+        b.edge_info = f.info.as<float4>();
+        m->dbg_mats = b.mats;
+        m->dbg_keys = b.edge_keys;
+        m->dbg_info = b.edge_info;
         if ((rc = enqueue_octree_stages(m, b))) return rc;
+        if (staged && (rc = enqueue_exports(m, b, staged, m->stream))) return rc;
         if ((rc = read_states(m, 1))) return rc;
         m->last_fresh = false;
         const BatchState& hb = *m->h_bs.as<BatchState>();
@@ -1365,35 +1476,40 @@ int export_chunk(lvn_meshgen* m, const OctreeEntry& o, lvn_mesh_out* out) {
     if (out->num_vertices > out->vertex_capacity || out->num_triangles > out->triangle_capacity ||
         out->num_seams > out->seam_capacity)
         return LVN_ERR_CAPACITY;
-    const cudaMemcpyKind kind = out->memory == LVN_MEMORY_DEVICE ? cudaMemcpyHostToDevice : cudaMemcpyHostToHost;
-    if (out->num_vertices)
-        LVN_CK(cudaMemcpy(out->vertices, o.vertices.data(), sizeof(lvn_mesh_vertex) * out->num_vertices, kind));
-    if (out->num_triangles)
-        LVN_CK(cudaMemcpy(out->triangles, o.triangles.data(), sizeof(lvn_mesh_triangle) * out->num_triangles, kind));
-    if (out->num_seams) LVN_CK(cudaMemcpy(out->seams, o.seams.data(), sizeof(lvn_seam_node) * out->num_seams, kind));
+    const size_t bv = sizeof(lvn_mesh_vertex) * out->num_vertices, bt = sizeof(lvn_mesh_triangle) * out->num_triangles,
+                 bs = sizeof(lvn_seam_node) * out->num_seams;
+    if (out->memory != LVN_MEMORY_DEVICE) {
+        int rc = host_store(out->vertices, o.vertices.data(), bv);
+        if (!rc) rc = host_store(out->triangles, o.triangles.data(), bt);
+        if (!rc) rc = host_store(out->seams, o.seams.data(), bs);
+        return rc;
+    }
+    if (bv) LVN_CK(cudaMemcpy(out->vertices, o.vertices.data(), bv, cudaMemcpyHostToDevice));
+    if (bt) LVN_CK(cudaMemcpy(out->triangles, o.triangles.data(), bt, cudaMemcpyHostToDevice));
+    if (bs) LVN_CK(cudaMemcpy(out->seams, o.seams.data(), bs, cudaMemcpyHostToDevice));
     return LVN_OK;
 }
 
-// Pull chunk 0's mesh out of the pools into host vectors.
-int pull_chunk(lvn_meshgen* m, OctreeEntry& o) {
-    const ChunkState& cs = m->last_cs[0];
-    const bool simp = m->simp_threshold >= 0.f;
-    const int ntri = simp ? cs.simp_tris : 2 * cs.quads;
-    o.num_vertices = ntri > 0 ? (simp ? cs.simp_verts : cs.nodes) : 0;
-    o.vertices.resize(o.num_vertices);
-    o.triangles.resize((size_t)ntri);
-    o.seams.resize(cs.seams);
-    if (o.num_vertices)
-        LVN_CK(cudaMemcpyAsync(o.vertices.data(),
-                               m->vertices.as<lvn_mesh_vertex>() + (simp ? cs.simp_vert_off : cs.node_off),
-                               sizeof(lvn_mesh_vertex) * o.num_vertices, cudaMemcpyDeviceToHost, m->stream));
-    if (ntri)
-        LVN_CK(cudaMemcpyAsync(o.triangles.data(),
-                               m->triangles.as<lvn_mesh_triangle>() + (simp ? (size_t)cs.simp_tri_off : 2 * (size_t)cs.quad_off),
-                               sizeof(lvn_mesh_triangle) * o.triangles.size(), cudaMemcpyDeviceToHost, m->stream));
-    if (cs.seams)
-        LVN_CK(cudaMemcpyAsync(o.seams.data(), m->seams.as<lvn_seam_node>() + cs.seam_off,
-                               sizeof(lvn_seam_node) * cs.seams, cudaMemcpyDeviceToHost, m->stream));
+// Chunk 0's mesh into host vectors: from the staging buffer, or from the pools.
+int pull_chunk(lvn_meshgen* m, const DirectOut* staged, OctreeEntry& o) {
+    const MeshView w = pool_mesh(m);
+    o.num_vertices = w.nv;
+    if (staged) {
+        const auto* v = static_cast<const lvn_mesh_vertex*>(staged->dst[0]);
+        const auto* t = static_cast<const lvn_mesh_triangle*>(staged->dst[1]);
+        const auto* s = static_cast<const lvn_seam_node*>(staged->dst[2]);
+        o.vertices.assign(v, v + w.nv);
+        o.triangles.assign(t, t + w.nt);
+        o.seams.assign(s, s + w.ns);
+        return LVN_OK;
+    }
+    o.vertices.resize(w.nv);
+    o.triangles.resize(w.nt);
+    o.seams.resize(w.ns);
+    int rc = copy_out(m, o.vertices.data(), w.v, sizeof(lvn_mesh_vertex) * w.nv, LVN_MEMORY_HOST);
+    if (!rc) rc = copy_out(m, o.triangles.data(), w.t, sizeof(lvn_mesh_triangle) * w.nt, LVN_MEMORY_HOST);
+    if (!rc) rc = copy_out(m, o.seams.data(), w.s, sizeof(lvn_seam_node) * w.ns, LVN_MEMORY_HOST);
+    if (rc) return rc;
     LVN_CK(cudaStreamSynchronize(m->stream));
     return LVN_OK;
 }
@@ -1524,6 +1640,7 @@ void lvn_meshgen_destroy(lvn_meshgen* m) {
     m->h_gate.release();
     m->h_sslot.release();
     m->h_lattices.release();
+    m->h_mesh.release();
     for (auto& kv : m->fields) {
         kv.second.mats.release();
         kv.second.planes.release();
@@ -1740,14 +1857,7 @@ int lvn_meshgen_generate_chunks(lvn_meshgen* m, const lvn_chunk_desc* chunks, in
     const bool dev = out->memory == LVN_MEMORY_DEVICE;
     DirectOut direct;
     const bool use_direct = !dev && m->host_writes && direct_addresses(out, &direct);
-    if (use_direct && !m->side) {
-        // exports take free SM slots ahead of the compute kernels they overlap
-        int lo = 0, hi = 0;
-        LVN_CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-        LVN_CK(cudaStreamCreateWithPriority(&m->side, cudaStreamNonBlocking, hi));
-        LVN_CK(cudaEventCreateWithFlags(&m->ev_leaf, cudaEventDisableTiming));
-        LVN_CK(cudaEventCreateWithFlags(&m->ev_side, cudaEventDisableTiming));
-    }
+    if (use_direct && (rc = ensure_side(m))) return rc;
     rc = run_fresh_batch(m, descs, brushes, dev ? out : nullptr, use_direct ? &direct : nullptr);
     out->total_vertices = out->total_triangles = out->total_seams = 0;
     if (m->h_bs.p) {  // absent when the first pool allocation failed
@@ -1811,10 +1921,12 @@ int lvn_meshgen_generate_chunk_mesh(lvn_meshgen* m, const int32_t min[3], int32_
         std::vector<Brush> brushes;
         int rc = build_descs(m, &cd, 1, descs, brushes, true);
         if (rc) return rc;
-        if ((rc = run_fresh_batch(m, descs, brushes, nullptr))) return rc;
-        OctreeEntry o;
-        if ((rc = pull_chunk(m, o))) return rc;
-        return export_chunk(m, o, out);
+        DirectOut direct;
+        const bool staged = out->memory != LVN_MEMORY_DEVICE && mesh_stage(m, &direct);
+        rc = run_fresh_batch(m, descs, brushes, nullptr, staged ? &direct : nullptr);
+        if (rc) return rc;
+        const bool fits = staged && m->h_bs.as<BatchState>()->status == 0;
+        return deliver_mesh(m, fits ? &direct : nullptr, out);
     }
     // LoadOctree (compute_octree.cpp:154-181)
     const ChunkKey k = key_of(min, size);
@@ -1826,8 +1938,11 @@ int lvn_meshgen_generate_chunk_mesh(lvn_meshgen* m, const int32_t min[3], int32_
         f = &m->fields[k];
         OctreeEntry o;
         if (f->num_edges > 0) {
-            if ((rc = mesh_from_field(m, min, size, *f))) return rc;
-            if ((rc = pull_chunk(m, o))) return rc;
+            DirectOut direct;
+            const bool staged = mesh_stage(m, &direct);
+            if ((rc = mesh_from_field(m, min, size, *f, staged ? &direct : nullptr))) return rc;
+            const bool fits = staged && m->h_bs.as<BatchState>()->status == 0;
+            if ((rc = pull_chunk(m, fits ? &direct : nullptr, o))) return rc;
         }
         it = m->octrees.emplace(k, std::move(o)).first;
     }
@@ -1879,12 +1994,14 @@ int64_t lvn_meshgen_debug_fetch(lvn_meshgen* m, int32_t what, int32_t chunk, voi
     const size_t F = (size_t)field_size(m->vpc);
     const void* src = nullptr;
     int64_t count = 0, elem = 0;
-    std::vector<uint8_t> mats;
+    const int32_t* keys = m->dbg_keys ? m->dbg_keys : m->edge_keys.as<int32_t>();
+    const float4* info = m->dbg_info ? m->dbg_info : m->edge_info.as<float4>();
     switch (what) {
         case LVN_DEBUG_MATERIALS: {
             if (cap < (int64_t)F) return LVN_ERR_CAPACITY;
             uint8_t* out = static_cast<uint8_t*>(host);
-            if (cudaMemcpy(out, m->mats.as<uint8_t>() + F * chunk, F, cudaMemcpyDeviceToHost) != cudaSuccess)
+            const uint8_t* mats = m->dbg_mats ? m->dbg_mats : m->mats.as<uint8_t>();
+            if (cudaMemcpy(out, mats + F * chunk, F, cudaMemcpyDeviceToHost) != cudaSuccess)
                 return LVN_ERR_CUDA;
             if (m->last_fresh && chunk < (int)m->last_desc.size()) {
                 // fresh fields hold byte materials only inside the CSG box; the
@@ -1911,8 +2028,8 @@ int64_t lvn_meshgen_debug_fetch(lvn_meshgen* m, int32_t what, int32_t chunk, voi
             }
             return (int64_t)F;
         }
-        case LVN_DEBUG_EDGE_KEYS: src = m->edge_keys.as<int32_t>() + cs.edge_off; count = cs.num_edges; elem = 4; break;
-        case LVN_DEBUG_EDGE_INFO: src = m->edge_info.as<float4>() + cs.edge_off; count = cs.num_edges; elem = 16; break;
+        case LVN_DEBUG_EDGE_KEYS: src = keys + cs.edge_off; count = cs.num_edges; elem = 4; break;
+        case LVN_DEBUG_EDGE_INFO: src = info + cs.edge_off; count = cs.num_edges; elem = 16; break;
         case LVN_DEBUG_NODE_CODES: src = m->node_codes.as<uint32_t>() + cs.node_off; count = cs.nodes; elem = 4; break;
         case LVN_DEBUG_NODE_INFO: src = m->node_info.as<int32_t>() + cs.node_off; count = cs.nodes; elem = 4; break;
         case LVN_DEBUG_EDGE_TABLE:
