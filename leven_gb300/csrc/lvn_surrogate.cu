@@ -49,9 +49,15 @@ constexpr int kHeadB = kHeadW + kHidden;
 constexpr int kParams = kHeadB + 1;
 static_assert(w_off(2) == w_off(1) + kHidden * kHidden + kHidden && b_off(0) == kHidden * kIn, "layout");
 static_assert(kParams == 62081, "4 x 128 SiLU MLP on 96 features");
-// BF16 copies W_l (out x in)
+// BF16 copies W_l (out x in), each laid out as the kernels' shared-memory operand
+// image (K-major core matrices of 8 outputs x 8 inputs, all of an input octet's
+// outputs first), so that a CTA reads its 120 KB of weights in order
 __host__ __device__ constexpr int wb_off(int l) { return l == 0 ? 0 : kHidden * kIn + (l - 1) * kHidden * kHidden; }
 constexpr int kWb = wb_off(kLayers);
+__device__ __forceinline__ int wb_pos(int rel, int in) {  // place of element `rel` of the row-major W_l
+    const int r = rel / in, c = rel % in;
+    return (c >> 3) * (8 * kHidden) + 8 * r + (c & 7);
+}
 
 // ---------------------------------------------------------------------------
 // tcgen05 / mbarrier primitives (inline PTX, sm_100 family)
@@ -163,6 +169,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Programmatic dependent launch: the next kernel of the stream may start once
+// every CTA has called launch_next; start_wait returns when the kernels before
+// this one are complete and their writes visible.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void start_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // SiLU through sigmoid(z) = (1 + tanh(z / 2)) / 2: one special-function
 // instruction (tanh.approx, relative error about 2^-11, below BF16's 2^-8)
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -170,10 +182,8 @@ __device__ __forceinline__ float tanh_approx(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float sigmoid(float z) { return fmaf(0.5f, tanh_approx(0.5f * z), 0.5f); }
-__device__ __forceinline__ float silu(float z) { return z * sigmoid(z); }
-// the same on two values at once: the FP32 arithmetic in the two-lane forms
-// (one instruction for both), the hyperbolic tangent per lane
+// on two values at once: the FP32 arithmetic in the two-lane forms (one
+// instruction for both), the hyperbolic tangent per lane
 __device__ __forceinline__ float2 sigmoid2(float2 z) {
     const float2 h = mul2(z, v2(0.5f));
     return fma2(v2(0.5f), make_float2(tanh_approx(h.x), tanh_approx(h.y)), v2(0.5f));
@@ -266,13 +276,13 @@ struct LayerMap {
     int w[kLayers], b[kLayers], in[kLayers], wb[kLayers];
 };
 
-// the BF16 copies W_l (out x in, row-major) of the FP32 hidden weights
+// the BF16 copies W_l of the FP32 hidden weights
 __global__ void k_to_bf16(const float* p, int n, __nv_bfloat16* wb, LayerMap lm) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #pragma unroll
         for (int l = 0; l < kLayers; l++) {
             const int rel = i - lm.w[l];
-            if (rel >= 0 && rel < kHidden * lm.in[l]) wb[lm.wb[l] + rel] = __float2bfloat16_rn(p[i]);
+            if (rel >= 0 && rel < kHidden * lm.in[l]) wb[lm.wb[l] + wb_pos(rel, in_dim(l))] = __float2bfloat16_rn(p[i]);
         }
     }
 }
@@ -344,14 +354,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(InferArgs a) {
     const int row = threadIdx.x & 127;  // tile row = TMEM lane
     // weights: layer l is N = 128 rows (out) x K = in_l, K-major core matrices
     constexpr uint32_t kLbo = (kTile / 8) * 128;  // 2048: 128 rows per K column of core matrices
-    for (int l = 0; l < kLayers; l++) {
-        const int in = in_dim(l), cores = in / 8;
-        uint8_t* dst = sW + 2 * wb_off(l);
-        for (int i = threadIdx.x; i < kHidden * cores; i += blockDim.x) {
-            const int r = i % kHidden, c = i / kHidden;
-            cp_async16(dst + c * kLbo + r * 16, a.wb + wb_off(l) + (size_t)r * in + 8 * c);
-        }
-    }
+    for (int i = threadIdx.x; i < kWbBytes / 16; i += kInferThreads) cp_async16(sW + 16 * i, a.wb + 8 * i);
     for (int i = threadIdx.x; i < kLayers * kHidden; i += blockDim.x)
         sBias[i] = a.params[b_off(i / kHidden) + (i % kHidden)];
     for (int i = threadIdx.x; i <= kHidden; i += blockDim.x) sBias[kLayers * kHidden + i] = a.params[kHeadW + i];
@@ -513,33 +516,51 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(InferArgs a) {
 // gradients of 128-row tiles in one persistent kernel, one launch per step.
 //
 // Each CTA (16 warps) takes a run of tiles.  The four hidden layers' BF16
-// weights stay in shared memory, with two activation images, one dZ image and
-// a 128 x 16 image of ones (220 KB).  A thread owns TMEM lane / tile row
-// 32 (warp & 3) + lane and the 32-column chunk 32 (warp >> 2) .. + 31.
+// weights stay in shared memory, with two activation images, each with 16
+// columns of ones behind it, and one dZ image (224 KB).  A thread owns TMEM lane
+// / tile row 32 (warp & 3) + lane and the 32-column chunk 32 (warp >> 2) .. + 31.
 //
 // Per tile:
-//   features -> XA (and the X0 image to the tile's slot in scratch)
+//   features -> XA (and the X0 image in the tile's slot in scratch)
 //   layer l: acc = X_l W_l^T; z = acc + b_l -> BF16 z image (scratch);
 //            X_{l+1} = BF16 silu(z) -> the other image (X1 also to the slot)
 //   head:    y = X4 . w4 + b4 (four chunk sums), r = y - t / s, dy = 2 r / n,
 //            dZ3 = dy w4 silu'(z3) -> the dZ image
-//   l = 3, 2: dW_l += dZ_l^T X_l, db_l += dZ_l^T 1 and acc = dZ_l W_l in one
-//            commit; dZ_{l-1} = acc silu'(z_{l-1}) -> the dZ image (dZ1 also
-//            to the slot)
-//   l = 1:   acc = dZ1 W1; dZ0 = acc silu'(z0) -> the slot
+//   l = 3, 2: acc = dZ_l W_l, then [dW_l db_l] += dZ_l^T [X_l 1];
+//            dZ_{l-1} = acc silu'(z_{l-1}) -> the dZ image (dZ1 also to the slot)
+//   l = 1:   acc = dZ1 W1; dZ0 = acc silu'(z0) -> the dZ image and the slot
 // dW_3, dW_2 and their bias sums accumulate in tensor memory over the CTA's
-// tiles.  After the last tile they are written out and the freed columns take
-// dW_1, dW_0 and their bias sums, contracted from the slots' X1 / dZ1 and
-// X0 / dZ0 images (about 480 KB of scratch per CTA, in L2).
+// tiles.  After the last tile [dW_1 db_1] and [dW_0 db_0] are contracted from the
+// slots' images (about 480 KB of scratch per CTA, in L2).
+//
+// A tile is a chain of seven products and epilogues, none of which can start
+// before the one ahead of it, and shared memory has no room for a second tile,
+// so everything else is kept off that chain: the weight gradients run after the
+// input gradient, under the epilogue's arithmetic (that waits for them only to
+// write over dZ_l); the copy engine takes X1, dZ1 and dZ0 to the slot; the next
+// tile's features and w4's column sums are computed while products run.  The
+// products read 8 KB of shared memory per 64 clocks, its whole rate, which slows
+// what runs beside them: a feature axis takes 1500 clocks there, 500 alone.  After
+// the last tile the images come back through three stages while the finished
+// gradients are written out.  65,536 rows (four tiles for each of 128 CTAs) take
+// 72 us, of them 13 after the last tile (92 us before, the chain's 2.6 us a link
+// with the tail's 22 us of row-major gradient stores and waited-for copies); the
+// seven products' own time is about 4 us a tile.  Moving z2 from scratch to
+// tensor memory took 34 MB of 370 off the L2 and no time.
 //
 // The weight-gradient products read the dZ and X images as MN-major operands
 // (the same core matrices, K running over the tile's rows) and the input
 // gradient reads W_l as an MN-major B, so no transposed copy is made.  A bias
-// gradient is the product of dZ^T with the ones image (column 0 of 16 kept).
+// gradient is the product of dZ^T with the ones (column 0 of 16 kept).
 // The head's weight gradient is a column sum over rows on the CUDA cores (a
 // butterfly that leaves column L's sum of a warp's rows in lane L).  The CTA
 // writes its gradient and loss to its own row of `partial`; k_adam_partials
 // sums the rows in a fixed order, so a step is deterministic.
+//
+// k_mlp_train may start while the previous step's k_adam_partials still runs: its
+// first tile's features need none of the weights.  (k_adam_partials started
+// early in its turn lands on the few SMs without a k_mlp_train CTA and sums there:
+// 94 us a step instead of 77.)
 // ---------------------------------------------------------------------------
 
 constexpr uint32_t kCoreCol = (kTile / 8) * 128;  // bytes between core-matrix columns of a 128-row image
@@ -547,22 +568,31 @@ constexpr int kTrainThreads = 512;  // 16 warps: lane quarter warp & 3, column q
 constexpr int kX0Bytes = kTile * kIn * 2;       // 24 KB feature image
 constexpr int kImgBytes = kTile * kHidden * 2;  // 32 KB activation image
 constexpr int kOnesBytes = kTile * 16 * 2;      // 4 KB: 128 rows x 16 columns of 1.0
-constexpr int kTrainSmem = kWbBytes + 3 * kImgBytes + kOnesBytes;
+constexpr int kXBytes = kImgBytes + kOnesBytes;  // an activation image and the ones behind it
+constexpr int kTrainSmem = kWbBytes + 2 * kXBytes + kImgBytes;
 static_assert(kTrainSmem + 4 * kTile * 4 + 64 <= 227 * 1024, "one CTA per SM");
+constexpr int kStageBytes = kXBytes + kImgBytes;  // the last contractions' stages: X, ones, dZ
+static_assert(3 * kStageBytes <= kTrainSmem, "three stages");
 // per tile slot: the X0, X1, dZ0 and dZ1 images, contracted after the last tile
 constexpr size_t kSlotBytes = (size_t)kX0Bytes + 3 * (size_t)kImgBytes;
 constexpr size_t kTransientBytes = 3 * (size_t)kImgBytes;  // z0, z1, z2 of the tile in hand
 constexpr int kPartStride = (kParams + 1 + 3) / 4 * 4;     // gradient, then the loss; 16-byte rows
+// A weight gradient's place in a row of `partial`: four columns of output 0,
+// of output 1, ... of output 127, then the next four columns, so that a warp,
+// whose lanes hold one output each, stores 512 bytes in order.  (Row-major
+// stores of 16 bytes every 512 took 16 of a step's 92 us.)
+static_assert(kHidden == 128 && w_off(1) % 4 == 0 && b_off(0) % 4 == 0 && kHeadW % 4 == 0, "groups of four");
 // tensor-memory columns
 constexpr uint32_t kTmWork = 0;    // forward and input-gradient accumulator
-constexpr uint32_t kTmDW2 = 128;   // dW_2 over the CTA's tiles; dW_1 after the last tile
-constexpr uint32_t kTmDW3 = 256;   // dW_3; dW_0 (96 columns) after the last tile
-constexpr uint32_t kTmDB = 384;    // db_2 / db_1 (16 columns), then db_3 / db_0 (16 columns)
+constexpr uint32_t kTmDW2 = 144;   // dW_2 and db_2 (16 columns) over the CTA's tiles
+constexpr uint32_t kTmDW3 = 288;   // dW_3 and db_3
+constexpr uint32_t kTmDW1 = 0;     // after the last tile: dW_1 and db_1
+constexpr uint32_t kTmDW0 = 144;   // and, once dW_2 is out, dW_0 (96 columns) and db_0
 constexpr uint32_t kIdescFwd = umma_idesc(kTile, kHidden);
 constexpr uint32_t kIdescDX = umma_idesc(kTile, kHidden) | (1u << 16);                 // B MN-major
-constexpr uint32_t kIdescDW = umma_idesc(kHidden, kHidden) | (1u << 15) | (1u << 16);  // A and B MN-major
-constexpr uint32_t kIdescDW0 = umma_idesc(kHidden, kIn) | (1u << 15) | (1u << 16);
-constexpr uint32_t kIdescDB = umma_idesc(kHidden, 16) | (1u << 15) | (1u << 16);
+// A and B MN-major; the ones behind the X image make 16 more columns
+constexpr uint32_t kIdescDW = umma_idesc(kHidden, kHidden + 16) | (1u << 15) | (1u << 16);
+constexpr uint32_t kIdescDW0 = umma_idesc(kHidden, kIn + 16) | (1u << 15) | (1u << 16);
 
 struct TrainArgs {
     const float4* pool;  // samples (x, y, z, density); row i of the batch is pool[(first + i) % pool_n]
@@ -596,12 +626,13 @@ __device__ __forceinline__ void unpack8(uint4 u, float* v) {
 }
 
 // Column sums of a warp's 32 rows: lane L holds row L's 32 values in v (which
-// this overwrites) and gets back the sum of column L over the 32 rows.  Each
-// of the five halvings keeps half of the remaining columns and adds the
-// partner lane's copy of them (31 shuffles in all).
-__device__ __forceinline__ float warp_column_sums(float (&v)[32], int lane) {
+// this overwrites) and v[0] ends as the sum of column L over the 32 rows.  Each
+// of the five halvings, off = 16 .. 1, keeps half of the remaining columns and
+// adds the partner lane's copy of them (31 shuffles in all).
+template <int FROM, int TO>
+__device__ __forceinline__ void column_halvings(float (&v)[32], int lane) {
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
+    for (int off = FROM; off >= TO; off >>= 1) {
         const bool up = (lane & off) != 0;
 #pragma unroll
         for (int j = 0; j < off; j++) {
@@ -610,31 +641,29 @@ __device__ __forceinline__ float warp_column_sums(float (&v)[32], int lane) {
             v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
     }
-    return v[0];
 }
 
-// every thread waits for the commit; false for the whole CTA when it did not
-// arrive within the poll limit
-__device__ __forceinline__ bool cta_wait(uint64_t* bar, uint32_t& phase) {
+// this thread's wait for a commit; false when it did not arrive within the poll limit
+__device__ __forceinline__ bool arrived(uint64_t* bar, uint32_t& phase) {
     uint32_t polls = 0;
-    bool late = false;
+    bool in_time = true;
     while (!mbar_try_wait(bar, phase))
         if (++polls == kWaitLimit) {
-            late = true;
+            in_time = false;
             break;
         }
     phase ^= 1u;
-    const bool ok = !__syncthreads_or(late);
     tc_fence_after();
-    return ok;
+    return in_time;
 }
 
-// shared-memory writes of this CTA made visible to the tensor core, then one
-// barrier; thread 0 issues next
-__device__ __forceinline__ void to_tensor_core() {
+// shared-memory writes of this CTA made visible to the tensor core and the copy
+// engine, then one barrier; thread 0 issues next.  False for the whole CTA when
+// some thread's wait came `late`: what it computed since is discarded.
+__device__ __forceinline__ bool to_tensor_core(bool late) {
     fence_proxy_async();
     tc_fence_before();
-    __syncthreads();
+    return !__syncthreads_or(late);
 }
 
 // 32 consecutive floats (16-byte aligned, the same for every lane) into registers
@@ -650,94 +679,125 @@ __device__ __forceinline__ void load32(const float* p, float (&v)[32]) {
     }
 }
 
-__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(TrainArgs a) {
+// a finished image to global memory on the copy engine (both addresses 16-byte
+// aligned), its group committed; the waits are for the issuing thread's groups
+__device__ __forceinline__ void bulk_store(void* gmem, uint32_t saddr, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem), "r"(saddr), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const __grid_constant__ TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar, bar_dw;
     __shared__ uint32_t tmem_base;
     __shared__ float ypart[4][kTile];
     uint8_t* sW = smem;
     uint8_t* sXA = smem + kWbBytes;
-    uint8_t* sXB = sXA + kImgBytes;
-    uint8_t* sDZ = sXB + kImgBytes;
-    uint8_t* sOnes = sDZ + kImgBytes;
+    uint8_t* sXB = sXA + kXBytes;
+    uint8_t* sDZ = sXB + kXBytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = warp & 3, cq = warp >> 2;
     const int row = 32 * q + lane;  // tile row = TMEM lane; columns 32 cq .. 32 cq + 31
     const uint32_t tl = ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * cq);  // this thread's lane and chunk
-    for (int l = 0; l < kLayers; l++) {
-        const int in = in_dim(l), cores = in / 8;
-        uint8_t* dst = sW + 2 * wb_off(l);
-        for (int i = threadIdx.x; i < kHidden * cores; i += blockDim.x) {
-            const int r = i % kHidden, c = i / kHidden;
-            cp_async16(dst + img_off(c, r), a.wb + wb_off(l) + (size_t)r * in + 8 * c);
+    const bool copier = threadIdx.x == 32;  // hands finished images to the copy engine
+    auto ones = [](uint8_t* at) {  // kOnesBytes of BF16 1.0
+        if (threadIdx.x < kOnesBytes / 16)
+            reinterpret_cast<uint4*>(at)[threadIdx.x] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    };
+    ones(sXA + kImgBytes);
+    ones(sXB + kImgBytes);
+    if (warp == 0) tmem_alloc(&tmem_base, 512);
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        mbar_init(&bar_dw, 1);
+    }
+    const uint32_t w_addr = smem_u32(sW), xa_addr = smem_u32(sXA), xb_addr = smem_u32(sXB), dz_addr = smem_u32(sDZ);
+    uint8_t* scr = a.scratch + (size_t)blockIdx.x * ((size_t)a.tiles_per_cta * kSlotBytes + kTransientBytes);
+    auto zimg = [scr](int l) { return scr + (size_t)l * kImgBytes; };  // z_l, l = 0, 1, 2
+    uint8_t* slots = scr + kTransientBytes;  // per tile: X0, X1, dZ0, dZ1
+    const int ntiles = a.n / kTile;
+    const int t0 = blockIdx.x * a.tiles_per_cta, t1 = min(ntiles, t0 + a.tiles_per_cta);
+    auto sample = [&](int t) {  // this thread's row of tile t
+        int64_t si = a.first + (int64_t)t * kTile + row;  // < 2 pool_n
+        if (si >= a.pool_n) si -= a.pool_n;
+        return a.pool[si];
+    };
+    // core column cq + 4 ax of the features: sin (cq < 2) or cos of axis ax's
+    // frequencies 8 (cq & 1) .. + 7, the angle's even half turns taken off as
+    // sincos_pi or, where every frequency's angle allows it, sincos_pi_small do
+    auto feature8 = [&](const float4& p, int ax) {
+        const float c = ax == 0 ? p.x : ax == 1 ? p.y : p.z;
+        const float u = 2.f * (c - a.dom.lo[ax]) / (a.dom.hi[ax] - a.dom.lo[ax]) - 1.f;
+        float f8[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) f8[k] = a.ff.f[ax][8 * (cq & 1) + k] * u;
+        if (fabsf(a.ff.f[ax][kFreqs - 1] * u) < 4194304.f) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) f8[k] -= 2.f * __fsub_rn(__fadd_rn(0.5f * f8[k], 12582912.f), 12582912.f);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) f8[k] -= 2.f * rintf(0.5f * f8[k]);
+        }
+        if (cq < 2) {  // warp-uniform
+#pragma unroll
+            for (int k = 0; k < 8; k++) f8[k] = __sinf(3.14159265358979f * f8[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) f8[k] = __cosf(3.14159265358979f * f8[k]);
+        }
+        return pack8(f8);
+    };
+    float target = 0.f;
+    if (t0 < t1) {  // the first tile's features, while the last step's weights are finished
+        const float4 p = sample(t0);
+        target = p.w / a.out_scale;
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+            const uint4 u = feature8(p, ax);
+            *reinterpret_cast<uint4*>(sXA + img_off(4 * ax + cq, row)) = u;
+            *reinterpret_cast<uint4*>(slots + img_off(4 * ax + cq, row)) = u;
         }
     }
-    for (int i = threadIdx.x; i < kOnesBytes / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(sOnes)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-    if (warp == 0) tmem_alloc(&tmem_base, 512);
-    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    // nothing before this line reads the weights, which the previous step's
+    // k_adam_partials may still be writing
+    start_wait();
+    for (int i = threadIdx.x; i < kWbBytes / 16; i += kTrainThreads) cp_async16(sW + 16 * i, a.wb + 8 * i);
+    const float b4 = a.params[kHeadB];
     cp_async_wait_all();
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const uint32_t w_addr = smem_u32(sW), xa_addr = smem_u32(sXA), xb_addr = smem_u32(sXB), dz_addr = smem_u32(sDZ);
-    const uint32_t ones_addr = smem_u32(sOnes);
-    uint8_t* scr = a.scratch + (size_t)blockIdx.x * ((size_t)a.tiles_per_cta * kSlotBytes + kTransientBytes);
-    auto zimg = [scr](int l) { return scr + (size_t)l * kImgBytes; };  // z_l, l = 0, 1, 2
-    uint8_t* slots = scr + kTransientBytes;  // per tile: X0, X1, dZ0, dZ1
-    const int ntiles = a.n / kTile;
-    const int t0 = blockIdx.x * a.tiles_per_cta, t1 = min(ntiles, t0 + a.tiles_per_cta);
-    const float b4 = a.params[kHeadB];
     float gw4 = 0.f, lsum = 0.f, gb4 = 0.f;  // w4 column 32 cq + lane over the warp's rows; loss and b4 per row
-    uint32_t phase = 0;
-    bool ok = true;
-    // dW_l (+)= dZ^T X over one tile's rows (M = 128 outputs, N = `n_in` inputs,
-    // both operands MN-major) and db_l (+)= dZ^T 1, issued by thread 0
-    const uint64_t dz_mn = umma_desc(dz_addr, 128, kCoreCol), ones_mn = umma_desc(ones_addr, 128, kCoreCol);
-    auto weight_grads = [&](uint32_t dw, uint32_t db, uint32_t x_addr, uint32_t idesc, bool acc) {
-        umma_chain<kTile / 16>(tmem + dw, dz_mn, 256, umma_desc(x_addr, 128, kCoreCol), 256, idesc, acc);
-        umma_chain<kTile / 16>(tmem + db, dz_mn, 256, ones_mn, 256, kIdescDB, acc);
+    uint32_t phase = 0, phase_dw = 0;
+    bool ok = true, late = false;
+    // [dW_l db_l] (+)= dZ^T [X 1] over one tile's rows (M = 128 outputs, N =
+    // inputs and 16 ones, both operands MN-major), issued by thread 0
+    auto weight_grads = [&](uint32_t dw, uint32_t d_addr, uint32_t x_addr, uint32_t idesc, bool acc) {
+        umma_chain<kTile / 16>(tmem + dw, umma_desc(d_addr, 128, kCoreCol), 256, umma_desc(x_addr, 128, kCoreCol), 256,
+                               idesc, acc);
     };
-    // the features of tile t -> XA and its slot's X0 image; its targets
-    auto features = [&](int t, float& target) {
-        uint8_t* x0img = slots + (size_t)(t - t0) * kSlotBytes;
-        int64_t si = a.first + (int64_t)t * kTile + row;  // < 2 pool_n
-        if (si >= a.pool_n) si -= a.pool_n;
-        const float4 p = a.pool[si];
-        target = p.w / a.out_scale;
-        // core column cq + 4 ax of each axis: sin (cq < 2) or cos of
-        // frequencies 8 (cq & 1) .. + 7
-        const float c[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int ax = 0; ax < 3; ax++) {
-            const float u = 2.f * (c[ax] - a.dom.lo[ax]) / (a.dom.hi[ax] - a.dom.lo[ax]) - 1.f;
-            float f8[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                float sv, cv;
-                sincos_pi(a.ff.f[ax][8 * (cq & 1) + k] * u, sv, cv);
-                f8[k] = cq < 2 ? sv : cv;
-            }
-            const uint4 u8 = pack8(f8);
-            *reinterpret_cast<uint4*>(sXA + img_off(4 * ax + cq, row)) = u8;
-            *reinterpret_cast<uint4*>(x0img + img_off(4 * ax + cq, row)) = u8;
-        }
-    };
-    float target = 0.f;
-    if (t0 < t1) features(t0, target);
     for (int t = t0; t < t1 && ok; t++) {
         uint8_t* x0img = slots + (size_t)(t - t0) * kSlotBytes;
         uint8_t* x1img = x0img + kX0Bytes;
-        uint8_t* dz0img = x1img + kImgBytes;
-        uint8_t* dz1img = dz0img + kImgBytes;
-        // forward
+        uint8_t* dz1img = x1img + 2 * kImgBytes;
+        // the next tile's features: an axis is computed while each forward
+        // product runs and waits in the slot for XA to be free
+        const bool more = t + 1 < t1;
+        uint8_t* x0next = x0img + kSlotBytes;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (more) p = sample(t + 1);
+        // forward: X0 in XA, X1 in XB, X2 in XA, X3 in XB
         uint8_t* src = sXA;
         uint8_t* dst = sXB;
 #pragma unroll 1
-        for (int l = 0; l < kLayers && ok; l++) {
-            to_tensor_core();
+        for (int l = 0; l < kLayers - 1; l++) {
+            if (copier && l == 2) bulk_wait_read();  // X1, which this layer's epilogue writes over
+            if (!(ok = to_tensor_core(late))) break;
             if (threadIdx.x == 0) {
                 tc_fence_after();
                 const uint64_t ad = umma_desc(smem_u32(src), kCoreCol, 128);
@@ -746,11 +806,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(TrainArgs a) {
                 else umma_chain<kHidden / 16>(tmem + kTmWork, ad, 2 * kCoreCol, bd, 2 * kCoreCol, kIdescFwd, false);
                 umma_commit(&bar);
             }
-            float bv[32], w4c[32];
+            if (copier) {  // the previous tile's dZ0 and this one's X1 leave while the products run
+                if (l == 0 && t > t0) bulk_store(dz1img - kImgBytes - kSlotBytes, dz_addr, kImgBytes);
+                if (l == 1) bulk_store(x1img, xb_addr, kImgBytes);
+            }
+            float bv[32];
             load32(a.params + b_off(l) + 32 * cq, bv);
-            if (l == kLayers - 1) load32(a.params + kHeadW + 32 * cq, w4c);
-            ok = cta_wait(&bar, phase);
-            if (!ok) break;
+            if (more) *reinterpret_cast<uint4*>(x0next + img_off(4 * l + cq, row)) = feature8(p, l);
+            late |= !arrived(&bar, phase);
             float v[32];
             tmem_ld32(tmem + kTmWork + tl, v);
 #pragma unroll
@@ -759,174 +822,204 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(TrainArgs a) {
                 v[j] = z.x;
                 v[j + 1] = z.y;
             }
-            if (l < kLayers - 1) {
 #pragma unroll
-                for (int g = 0; g < 4; g++)
-                    *reinterpret_cast<uint4*>(zimg(l) + img_off(4 * cq + g, row)) = pack8(v + 8 * g);
+            for (int g = 0; g < 4; g++)
+                *reinterpret_cast<uint4*>(zimg(l) + img_off(4 * cq + g, row)) = pack8(v + 8 * g);
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float2 z = make_float2(v[j], v[j + 1]);
-                    const float2 x = mul2(z, sigmoid2(z));
-                    v[j] = x.x;
-                    v[j + 1] = x.y;
-                }
-#pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    const uint4 u = pack8(v + 8 * g);
-                    *reinterpret_cast<uint4*>(dst + img_off(4 * cq + g, row)) = u;
-                    if (l == 0) *reinterpret_cast<uint4*>(x1img + img_off(4 * cq + g, row)) = u;
-                }
-                uint8_t* tmp = src;
-                src = dst;
-                dst = tmp;
-            } else {
-                // head: y from the BF16 activations, as in inference; the
-                // four column quarters' sums meet in shared memory
-                float2 y2 = v2(0.f);
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float2 z = make_float2(v[j], v[j + 1]);
-                    const float2 sg = sigmoid2(z);
-                    const float2 x = __bfloat1622float2(__float22bfloat162_rn(mul2(z, sg)));  // X4
-                    const float2 w = make_float2(w4c[j], w4c[j + 1]);
-                    y2 = fma2(x, w, y2);
-                    const float2 d = mul2(w, silu_grad2(z, sg));  // dZ3 / dy = w4 silu'(z3)
-                    w4c[j] = d.x;
-                    w4c[j + 1] = d.y;
-                    v[j] = x.x;
-                    v[j + 1] = x.y;
-                }
-                ypart[cq][row] = y2.x + y2.y;
-                __syncthreads();
-                const float r = ((ypart[0][row] + ypart[1][row]) + (ypart[2][row] + ypart[3][row])) + b4 - target;
-                const float dy = 2.f * r / (float)a.n;
-                if (cq == 0) {
-                    lsum = fmaf(r, r, lsum);
-                    gb4 += dy;
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float2 g = mul2(make_float2(v[j], v[j + 1]), v2(dy));         // w4's gradient terms
-                    const float2 d = mul2(make_float2(w4c[j], w4c[j + 1]), v2(dy));     // dZ3
-                    v[j] = g.x;
-                    v[j + 1] = g.y;
-                    w4c[j] = d.x;
-                    w4c[j + 1] = d.y;
-                }
-#pragma unroll
-                for (int g = 0; g < 4; g++)
-                    *reinterpret_cast<uint4*>(sDZ + img_off(4 * cq + g, row)) = pack8(w4c + 8 * g);
-                gw4 += warp_column_sums(v, lane);
+            for (int j = 0; j < 32; j += 2) {
+                const float2 z = make_float2(v[j], v[j + 1]);
+                const float2 x = mul2(z, sigmoid2(z));
+                v[j] = x.x;
+                v[j + 1] = x.y;
             }
+#pragma unroll
+            for (int g = 0; g < 4; g++) *reinterpret_cast<uint4*>(dst + img_off(4 * cq + g, row)) = pack8(v + 8 * g);
+            uint8_t* tmp = src;
+            src = dst;
+            dst = tmp;
         }
-        // backward: after the forward X2 is in XA and X3 in XB
-#pragma unroll 1
-        for (int l = kLayers - 1; l >= 1 && ok; l--) {
-            to_tensor_core();
+        if (!ok) break;
+        // head: y from the BF16 activations, as in inference; the four column
+        // quarters' sums meet in shared memory
+        float w4g[32];  // w4's gradient terms of this row
+        {
+            if (!(ok = to_tensor_core(late))) break;
             if (threadIdx.x == 0) {
                 tc_fence_after();
-                if (l >= 2)
-                    weight_grads(l == 3 ? kTmDW3 : kTmDW2, kTmDB + (l == 3 ? 16u : 0u), l == 3 ? xb_addr : xa_addr,
-                                 kIdescDW, t > t0);
+                umma_chain<kHidden / 16>(tmem + kTmWork, umma_desc(xb_addr, kCoreCol, 128), 2 * kCoreCol,
+                                         umma_desc(w_addr + 2 * wb_off(kLayers - 1), kCoreCol, 128), 2 * kCoreCol,
+                                         kIdescFwd, false);
+                umma_commit(&bar);
+            }
+            float bv[32], w4c[32];
+            load32(a.params + b_off(kLayers - 1) + 32 * cq, bv);
+            load32(a.params + kHeadW + 32 * cq, w4c);
+            late |= !arrived(&bar, phase);
+            tmem_ld32(tmem + kTmWork + tl, w4g);
+            float2 y2 = v2(0.f);
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+                const float2 z = add2(make_float2(w4g[j], w4g[j + 1]), make_float2(bv[j], bv[j + 1]));
+                const float2 sg = sigmoid2(z);
+                const float2 x = __bfloat1622float2(__float22bfloat162_rn(mul2(z, sg)));  // X4
+                const float2 w = make_float2(w4c[j], w4c[j + 1]);
+                y2 = fma2(x, w, y2);
+                const float2 d = mul2(w, silu_grad2(z, sg));  // dZ3 / dy = w4 silu'(z3)
+                w4c[j] = d.x;
+                w4c[j + 1] = d.y;
+                w4g[j] = x.x;
+                w4g[j + 1] = x.y;
+            }
+            ypart[cq][row] = y2.x + y2.y;
+            __syncthreads();
+            const float r = ((ypart[0][row] + ypart[1][row]) + (ypart[2][row] + ypart[3][row])) + b4 - target;
+            const float dy = 2.f * r / (float)a.n;
+            if (cq == 0) {
+                lsum = fmaf(r, r, lsum);
+                gb4 += dy;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+                const float2 g = mul2(make_float2(w4g[j], w4g[j + 1]), v2(dy));
+                const float2 d = mul2(make_float2(w4c[j], w4c[j + 1]), v2(dy));  // dZ3
+                w4g[j] = g.x;
+                w4g[j + 1] = g.y;
+                w4c[j] = d.x;
+                w4c[j + 1] = d.y;
+            }
+#pragma unroll
+            for (int g = 0; g < 4; g++)
+                *reinterpret_cast<uint4*>(sDZ + img_off(4 * cq + g, row)) = pack8(w4c + 8 * g);
+        }
+        // backward: X2 is in XA and X3 in XB
+        uint4 feat[3];
+#pragma unroll
+        for (int l = kLayers - 1; l >= 1; l--) {
+            if (!(ok = to_tensor_core(late))) break;
+            if (threadIdx.x == 0) {
+                tc_fence_after();
                 // dX = dZ_l W_l: M = the tile's rows, N = 128 inputs, K = 128 outputs
                 umma_chain<kHidden / 16>(tmem + kTmWork, umma_desc(dz_addr, kCoreCol, 128), 2 * kCoreCol,
                                          umma_desc(w_addr + 2 * wb_off(l), 128, kCoreCol), 256, kIdescDX, false);
                 umma_commit(&bar);
+                if (l >= 2) {  // runs on under the epilogue's arithmetic
+                    weight_grads(l == 3 ? kTmDW3 : kTmDW2, dz_addr, l == 3 ? xb_addr : xa_addr, kIdescDW, t > t0);
+                    umma_commit(&bar_dw);
+                }
             }
-            // this thread's z_{l-1} (32 BF16 values) while the products run
+            if (l == 1 && copier) {
+                bulk_store(dz1img, dz_addr, kImgBytes);
+                bulk_wait_read();  // before the barrier below lets dZ0 over it
+            }
+            // this thread's z_{l-1} (32 BF16 values)
             uint4 zr[4];
 #pragma unroll
             for (int g = 0; g < 4; g++) zr[g] = *reinterpret_cast<const uint4*>(zimg(l - 1) + img_off(4 * cq + g, row));
-            // and the next tile's features into XA (X2's products are done)
-            if (l == 1 && t + 1 < t1) features(t + 1, target);
-            ok = cta_wait(&bar, phase);
-            if (!ok) break;
-            float v[32], z[32];
+            // w4's gradient and the next tile's features, in what the products leave free
+            if (l == 3) column_halvings<16, 16>(w4g, lane);
+            if (l == 2) {
+                column_halvings<8, 1>(w4g, lane);
+                gw4 += w4g[0];
+                if (more)
+#pragma unroll
+                    for (int ax = 0; ax < 3; ax++)
+                        feat[ax] = *reinterpret_cast<const uint4*>(x0next + img_off(4 * ax + cq, row));
+            }
+            if (l == 1 && more) {  // X2's products are done
+                target = p.w / a.out_scale;
+#pragma unroll
+                for (int ax = 0; ax < 3; ax++) *reinterpret_cast<uint4*>(sXA + img_off(4 * ax + cq, row)) = feat[ax];
+            }
+            late |= !arrived(&bar, phase);
+            if (l == 1) __syncthreads();
+            float v[32];
             tmem_ld32(tmem + kTmWork + tl, v);
 #pragma unroll
-            for (int g = 0; g < 4; g++) unpack8(zr[g], z + 8 * g);
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                const float2 zz = make_float2(z[j], z[j + 1]);
-                const float2 d = mul2(make_float2(v[j], v[j + 1]), silu_grad2(zz, sigmoid2(zz)));
-                v[j] = d.x;
-                v[j + 1] = d.y;
-            }
-#pragma unroll
             for (int g = 0; g < 4; g++) {
-                const uint4 u = pack8(v + 8 * g);
-                if (l > 1) *reinterpret_cast<uint4*>(sDZ + img_off(4 * cq + g, row)) = u;
-                if (l == 2) *reinterpret_cast<uint4*>(dz1img + img_off(4 * cq + g, row)) = u;
-                if (l == 1) *reinterpret_cast<uint4*>(dz0img + img_off(4 * cq + g, row)) = u;
+                float z[8];
+                unpack8(zr[g], z);
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    const float2 zz = make_float2(z[j], z[j + 1]);
+                    const float2 d = mul2(make_float2(v[8 * g + j], v[8 * g + j + 1]), silu_grad2(zz, sigmoid2(zz)));
+                    v[8 * g + j] = d.x;
+                    v[8 * g + j + 1] = d.y;
+                }
             }
+            if (l >= 2) late |= !arrived(&bar_dw, phase_dw);  // dZ_l's image, and X_l's, are free
+#pragma unroll
+            for (int g = 0; g < 4; g++) *reinterpret_cast<uint4*>(sDZ + img_off(4 * cq + g, row)) = pack8(v + 8 * g);
         }
     }
+    // the last tile's dZ0; then every image is in scratch for all threads
+    ok = to_tensor_core(late) && ok;
+    if (copier) {
+        if (ok && t1 > t0) bulk_store(slots + (size_t)(t1 - 1 - t0) * kSlotBytes + kX0Bytes + kImgBytes, dz_addr, kImgBytes);
+        bulk_wait();
+        asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    __syncthreads();
+    // [dW_1 db_1], then [dW_0 db_0] over the CTA's tiles from the slots' images, in
+    // three stages of shared memory (the weights are done with).  Each item is one
+    // tile's X and dZ; an empty group keeps the count.  The gradients already
+    // complete are written out while the first items' products run.
+    const int tiles = t1 - t0, items = 2 * tiles;
+    auto load_item = [&](int i) {
+        if (i < items) {
+            const bool first = i >= tiles;  // layer 0
+            const uint8_t* slot = slots + (size_t)(first ? i - tiles : i) * kSlotBytes;
+            uint8_t* st = smem + (i % 3) * kStageBytes;
+            const uint8_t* x = first ? slot : slot + kX0Bytes;
+            const uint8_t* dz = slot + kX0Bytes + (first ? 1 : 2) * kImgBytes;
+            for (int k = threadIdx.x; k < (first ? kX0Bytes : kImgBytes) / 16; k += kTrainThreads)
+                cp_async16(st + 16 * k, x + 16 * k);
+            for (int k = threadIdx.x; k < kImgBytes / 16; k += kTrainThreads)
+                cp_async16(st + kXBytes + 16 * k, dz + 16 * k);
+            ones(st + (first ? kX0Bytes : kImgBytes));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (ok)
+        for (int i = 0; i < 3; i++) load_item(i);
     float* part = a.partial + (size_t)blockIdx.x * kPartStride;
-    const bool any = t1 > t0;
     // this thread's lane is output row `row` of each dW, its chunk the
-    // columns 32 cq .. + 31 (layer 0 has three chunks); the bias sums are
-    // column 0 of their 16-column blocks
+    // columns 32 cq .. + 31 (layer 0 has three chunks); the bias sum is the
+    // first column behind the weights'
     auto flush = [&](int l, uint32_t col0) {
         const int in = in_dim(l);
-        if (32 * cq >= in) return;  // warp-uniform
         float v[32];
-        if (any) tmem_ld32(tmem + col0 + tl, v);
+        if (32 * cq < in) {  // warp-uniform
+            tmem_ld32(tmem + col0 + tl, v);
+            float4* d4 = reinterpret_cast<float4*>(part + w_off(l)) + 8 * cq * kHidden + row;
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = any ? v[j] : 0.f;
-        float4* d4 = reinterpret_cast<float4*>(part + w_off(l) + (size_t)row * in + 32 * cq);
-#pragma unroll
-        for (int j = 0; j < 8; j++) d4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    };
-    auto flush_bias = [&](int la, int lb) {  // db_la in column kTmDB, db_lb in kTmDB + 16
-        if (cq != 0) return;
-        float v[32];
-        tmem_ld32(tmem + kTmDB + ((uint32_t)(32 * q) << 16), v);
-        part[b_off(la) + row] = any ? v[0] : 0.f;
-        part[b_off(lb) + row] = any ? v[16] : 0.f;
-    };
-    if (ok) {
-        flush(2, kTmDW2);
-        flush(3, kTmDW3);
-        flush_bias(2, 3);
-    }
-    // dW_1, db_1, dW_0, db_0 over the CTA's tiles from the slots' images
-    // (written by other threads of the CTA: the barrier orders their stores
-    // before these reads, and the TMEM reads above before the MMAs below)
-    tc_fence_before();
-    __syncthreads();
-    for (int t = t0; t < t1 && ok; t++) {
-        const uint8_t* x0img = slots + (size_t)(t - t0) * kSlotBytes;
-        const uint8_t* x1img = x0img + kX0Bytes;
-        const uint8_t* dz0img = x1img + kImgBytes;
-        const uint8_t* dz1img = dz0img + kImgBytes;
-        for (int i = threadIdx.x; i < kImgBytes / 16; i += kTrainThreads) {
-            cp_async16(sXA + 16 * i, x1img + 16 * i);
-            cp_async16(sDZ + 16 * i, dz1img + 16 * i);
+            for (int j = 0; j < 8; j++) d4[j * kHidden] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
-        for (int i = threadIdx.x; i < kX0Bytes / 16; i += kTrainThreads) cp_async16(sXB + 16 * i, x0img + 16 * i);
-        cp_async_wait_all();
-        to_tensor_core();
+        if (cq == 0) {
+            tmem_ld32(tmem + col0 + in + ((uint32_t)(32 * q) << 16), v);
+            part[b_off(l) + row] = v[0];
+        }
+    };
+    for (int i = 0; i < items && ok; i++) {
+        asm volatile("cp.async.wait_group 2;" ::: "memory");  // item i
+        if (!(ok = to_tensor_core(late))) break;
         if (threadIdx.x == 0) {
             tc_fence_after();
-            weight_grads(kTmDW2, kTmDB, xa_addr, kIdescDW, t > t0);
+            const uint32_t st = w_addr + (uint32_t)(i % 3) * kStageBytes;
+            if (i < tiles) weight_grads(kTmDW1, st + kXBytes, st, kIdescDW, i > 0);
+            else weight_grads(kTmDW0, st + kXBytes, st, kIdescDW0, i > tiles);
             umma_commit(&bar);
         }
-        ok = cta_wait(&bar, phase);
-        if (!ok) break;
-        for (int i = threadIdx.x; i < kImgBytes / 16; i += kTrainThreads) cp_async16(sDZ + 16 * i, dz0img + 16 * i);
-        cp_async_wait_all();
-        to_tensor_core();
-        if (threadIdx.x == 0) {
-            tc_fence_after();
-            weight_grads(kTmDW3, kTmDB + 16, xb_addr, kIdescDW0, t > t0);
-            umma_commit(&bar);
-        }
-        ok = cta_wait(&bar, phase);
+        __syncwarp();
+        if (i == 0) flush(2, kTmDW2);
+        if (i == 1) flush(3, kTmDW3);
+        if (i == tiles) flush(1, kTmDW1);
+        late |= !arrived(&bar, phase);
+        load_item(i + 3);
     }
+    cp_async_wait_all();
+    ok = !__syncthreads_or(late) && ok;
     if (ok) {
-        flush(1, kTmDW2);
-        flush(0, kTmDW3);
-        flush_bias(1, 0);
+        flush(0, kTmDW0);
         // w4: column sums over the four lane quarters
         float* red = reinterpret_cast<float*>(sXA);  // [4][kHidden]
         red[q * kHidden + 32 * cq + lane] = gw4;
@@ -951,12 +1044,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(TrainArgs a) {
             part[kParams] = (((ypart[0][0] + ypart[0][1]) + ypart[0][2]) + ypart[0][3]) / (float)a.n;
         }
     } else {
-        // as in k_mlp_infer: a second bounded wait for the pending commit
+        // as in k_mlp_infer: a second bounded wait for the pending commits
         // before the columns are freed; the status flag makes the host
         // discard the step's results either way
         if (threadIdx.x == 0) atomicExch(a.status, 1);
         uint32_t polls = 0;
-        while (!mbar_try_wait(&bar, phase ^ 1u) && ++polls < 4 * kWaitLimit) {
+        while (!(mbar_try_wait(&bar, phase ^ 1u) && mbar_try_wait(&bar_dw, phase_dw ^ 1u)) &&
+               ++polls < 4 * kWaitLimit) {
         }
     }
     tc_fence_before();
@@ -967,30 +1061,53 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(TrainArgs a) {
 // The step's gradient: the sum of the CTAs' rows of `partial`, in CTA order.
 // With lr > 0, Adam (beta 0.9 / 0.999, eps 1e-8) on the FP32 master weights
 // and the BF16 copies refreshed; `grad` and `loss` receive the sums when not
-// null.
-__global__ void k_adam_partials(const float* partial, int parts, float* p, float* m, float* v, float lr, float c1,
-                                float c2, __nv_bfloat16* wb, LayerMap lm, float* grad, float* loss) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= kParams; i += gridDim.x * blockDim.x) {
-        float gi = 0.f;
-        for (int c = 0; c < parts; c++) gi += partial[(size_t)c * kPartStride + i];
-        if (i == kParams) {  // the loss
-            if (loss) *loss = gi;
-            continue;
-        }
-        if (grad) grad[i] = gi;
-        if (!(lr > 0.f)) continue;
-        const float mi = 0.9f * m[i] + 0.1f * gi;
-        const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + 1e-8f);
-        p[i] = pi;
+// null.  A thread takes one sum with 32 rows' loads in flight: 32 MB of rows in
+// L2, about 5 us a step (14 with four loads in flight;
+// four neighbouring sums a thread, in 16-byte loads, left three warps an SM and took 22).
+constexpr int kAdamThreads = 128;
+constexpr int kAdamBlocks = (kParams + kAdamThreads) / kAdamThreads;  // the parameters and the loss
+__global__ void __launch_bounds__(kAdamThreads) k_adam_partials(const float* __restrict__ partial, int parts, float* p,
+                                                                float* m, float* v, float lr, float c1, float c2,
+                                                                __nv_bfloat16* wb, float* grad, float* loss) {
+    const int place = blockIdx.x * kAdamThreads + threadIdx.x;
+    start_wait();
+    launch_next();  // the next step's k_mlp_train: its features need none of this
+    if (place > kParams) return;
+    // the parameter with this place in a row, and its place among the BF16 copies
+    int i = place, copy = -1;
 #pragma unroll
-        for (int l = 0; l < kLayers; l++) {
-            const int rel = i - lm.w[l];
-            if (rel >= 0 && rel < kHidden * lm.in[l]) wb[lm.wb[l] + rel] = __float2bfloat16_rn(pi);
-        }
+    for (int l = 0; l < kLayers; l++) {
+        const int rel = place - w_off(l), out = (rel >> 2) % kHidden, col = (rel >> 2) / kHidden * 4 + (rel & 3);
+        if (rel < 0 || rel >= kHidden * in_dim(l)) continue;
+        i = w_off(l) + out * in_dim(l) + col;
+        copy = wb_off(l) + (col >> 3) * (8 * kHidden) + 8 * out + (col & 7);
     }
+    const bool adam = lr > 0.f && i < kParams;
+    float pi = 0.f, mi = 0.f, vi = 0.f;
+    if (adam) pi = p[i], mi = m[i], vi = v[i];
+    float gi = 0.f;
+    int c = 0;
+    for (; c + 32 <= parts; c += 32) {
+        float r[32];
+#pragma unroll
+        for (int k = 0; k < 32; k++) r[k] = partial[(size_t)(c + k) * kPartStride + place];
+#pragma unroll
+        for (int k = 0; k < 32; k++) gi += r[k];
+    }
+    for (; c < parts; c++) gi += partial[(size_t)c * kPartStride + place];
+    if (i == kParams) {
+        if (loss) *loss = gi;
+        return;
+    }
+    if (grad) grad[i] = gi;
+    if (!adam) return;
+    mi = 0.9f * mi + 0.1f * gi;
+    vi = 0.999f * vi + 0.001f * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    pi = pi - lr * (mi * c1) / (sqrtf(vi * c2) + 1e-8f);
+    p[i] = pi;
+    if (copy >= 0) wb[copy] = __float2bfloat16_rn(pi);
 }
 
 // ---------------------------------------------------------------------------
@@ -1120,6 +1237,23 @@ LayerMap layer_map() {
     return lm;
 }
 
+// A launch that may begin before the kernel ahead of it in the stream has ended
+// (the kernel itself waits where it needs that one's results).
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 }  // namespace
 }  // namespace lvn
 
@@ -1198,8 +1332,7 @@ struct lvn_surrogate {
         a.scratch = train_scratch.as<uint8_t>();
         a.partial = partial.as<float>();
         a.status = status.as<int>();
-        k_mlp_train<<<grid, kTrainThreads, kTrainSmem, stream>>>(a);
-        SG_CK(cudaGetLastError());
+        SG_CK(launch_early(k_mlp_train, grid, kTrainThreads, kTrainSmem, stream, a));
         *parts = grid;
         return LVN_OK;
     }
@@ -1337,10 +1470,9 @@ int lvn_surrogate_grad(lvn_surrogate* s, const float* samples, int32_t n, float*
     if (rc) return rc;
     int parts = 0;
     if ((rc = s->train_launch(s->pts.as<float4>(), n, 0, n, &parts))) return rc;
-    k_adam_partials<<<(kParams + 256) / 256, 256, 0, s->stream>>>(s->partial.as<float>(), parts, nullptr, nullptr,
-                                                                   nullptr, 0.f, 0.f, 0.f, nullptr, layer_map(),
-                                                                   s->grads.as<float>(), s->loss.as<float>());
-    SG_CK(cudaGetLastError());
+    SG_CK(launch_early(k_adam_partials, kAdamBlocks, kAdamThreads, 0, s->stream, (const float*)s->partial.as<float>(),
+                       parts, (float*)nullptr, (float*)nullptr, (float*)nullptr, 0.f, 0.f, 0.f, (__nv_bfloat16*)nullptr,
+                       s->grads.as<float>(), s->loss.as<float>()));
     if ((rc = check_status(s))) return rc;
     if (grad_out) SG_CK(cudaMemcpy(grad_out, s->grads.p, 4ull * kParams, cudaMemcpyDeviceToHost));
     if (loss_out) SG_CK(cudaMemcpy(loss_out, s->loss.p, 4, cudaMemcpyDeviceToHost));
@@ -1351,7 +1483,6 @@ int lvn_surrogate_train(lvn_surrogate* s, int32_t steps, int32_t batch, float lr
     if (!s || steps < 0 || batch <= 0 || batch % kTile || !(lr > 0.f)) return LVN_ERR_INVALID;
     if (s->pool_n < batch) return LVN_ERR_INVALID;  // lvn_surrogate_sample first
     int rc;
-    const LayerMap lm = layer_map();
     // the losses stay on the device until the end, so the host never waits
     // on a step and the launches queue ahead of the GPU
     if (steps > 0 && (rc = s->loss_hist.ensure(sizeof(float) * (size_t)steps))) return rc;
@@ -1364,10 +1495,10 @@ int lvn_surrogate_train(lvn_surrogate* s, int32_t steps, int32_t batch, float lr
         s->step++;
         const float c1 = 1.f / (1.f - std::pow(0.9f, (float)s->step));
         const float c2 = 1.f / (1.f - std::pow(0.999f, (float)s->step));
-        k_adam_partials<<<(kParams + 256) / 256, 256, 0, s->stream>>>(
-            s->partial.as<float>(), parts, s->params.as<float>(), s->adam_m.as<float>(), s->adam_v.as<float>(), lr, c1,
-            c2, s->wb.as<__nv_bfloat16>(), lm, nullptr, s->loss_hist.as<float>() + it);
-        SG_CK(cudaGetLastError());
+        SG_CK(launch_early(k_adam_partials, kAdamBlocks, kAdamThreads, 0, s->stream,
+                           (const float*)s->partial.as<float>(), parts, s->params.as<float>(), s->adam_m.as<float>(),
+                           s->adam_v.as<float>(), lr, c1, c2, s->wb.as<__nv_bfloat16>(), (float*)nullptr,
+                           s->loss_hist.as<float>() + it));
     }
     if (losses && steps > 0)
         SG_CK(cudaMemcpyAsync(losses, s->loss_hist.p, sizeof(float) * (size_t)steps, cudaMemcpyDeviceToHost, s->stream));

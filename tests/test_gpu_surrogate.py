@@ -269,3 +269,26 @@ def test_trained_network_gain_over_the_method_without_it(lvn_gpu):
     assert rms_trained * 5.0 <= rms_untrained, (rms_trained, rms_untrained)
     assert rms_trained * 1.5 <= rms_linear, (rms_trained, rms_linear)
     assert used_untrained == 0 and used_trained > used_untrained
+
+
+@pytest.mark.parametrize("n", [128, 153 * 128, 700 * 128])
+def test_training_step_uneven_tiles(surrogate, n):
+    """One tile in all, and batches that leave the last CTA fewer tiles than the
+    others: the gradient against float64, and one Adam step from zero moments
+    against its formula on that gradient, every parameter in its place.  The
+    step's constants in FP32 (1 - 0.999f is off by 1.3e-5 of itself) bound the
+    update's relative error by 1e-5 of the rate 1e-3, and the weights are below
+    1, so 5e-8 holds both with rounding to spare."""
+    pts = surrogate.sample(n, seed=23, fetch=True)
+    p0 = surrogate.params().astype(np.float64)
+    g, loss = surrogate.grad(pts)
+    rg, rloss = reference(surrogate.params(), pts, pts[:, 3])
+    assert abs(loss - rloss) <= 0.02 * rloss
+    for a, b in blocks():
+        assert np.linalg.norm(g[a:b] - rg[a:b]) <= 0.05 * np.linalg.norm(rg[a:b]) + 1e-7
+    losses = surrogate.train(1, batch=n, lr=1e-3)
+    assert losses[0] == np.float32(loss)
+    g = g.astype(np.float64)
+    assert np.abs(surrogate.params() - (p0 - 1e-3 * g / (np.abs(g) + 1e-8))).max() <= 5e-8
+    got, want = surrogate.eval(pts), reference(surrogate.params(), pts)
+    assert np.linalg.norm(got - want) <= 0.05 * np.linalg.norm(want) + 1e-3
