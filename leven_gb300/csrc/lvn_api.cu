@@ -393,7 +393,8 @@ struct lvn_meshgen {
     // the fresh-batch DAG: hermite on `aux` beside the voxel, hash and quad
     // stages, with a grid of dag_hermite_per_sm CTAs per SM (0 = its tuned shape)
     cudaStream_t aux = nullptr, aux2 = nullptr;  // hermite; the quad chain
-    cudaEvent_t ev_fork = nullptr, ev_herm = nullptr, ev_hash = nullptr, ev_mesh = nullptr;
+    cudaEvent_t ev_field = nullptr, ev_plan = nullptr, ev_fork = nullptr, ev_vplan = nullptr, ev_vox = nullptr;
+    cudaEvent_t ev_etab = nullptr, ev_hash = nullptr, ev_mesh = nullptr;
     int dag_hermite_per_sm = 0;
 
     // the shapes an autotuning in progress on this context is trying (CTAs
@@ -708,60 +709,81 @@ int enqueue_exports(lvn_meshgen* m, const BatchPtrs& b, const DirectOut* direct,
 constexpr int kLeafSlices = 4;  // leaf / vertex-export pipeline depth for pinned host outputs
 
 // The fresh-batch DAG (one graph when captured):
-//   field, CSG, edges                                           (stream)
-//   -> hermite                                                   (aux)
-//   || voxels, primes, hash-table fill                           (stream)
-//      -> leaf-hash insert, quads, triangles                     (aux2)
-//         [pinned outputs: triangles exported on aux2]
-//      || edge-hash insert, join hermite, leaves                 (stream)
-//         [pinned outputs: the leaves write their vertices to the host
-//          array as they are made; an unaligned array instead gets the
-//          leaves in slices, each exported on the side stream while the
-//          next is computed]
+//   field, CSG, edges -> hermite                                 (stream)
+//   || voxels (their counts beside the edges') -> quads, triangles  (aux2)
+//      [pinned outputs: triangles exported on aux2]
+//   || edge table, then leaf table                                (aux)
+//   -> join voxels and edge table -> leaves                       (stream)
+//      [pinned outputs: the leaves write their vertices to the host
+//       array as they are made; an unaligned array instead gets the
+//       leaves in slices, each exported on the side stream while the
+//       next is computed]
 //   -> join -> seams, simplification, exports' join              (stream)
-// No branch reads what another writes before their join: the chain beside
-// hermite reads edge keys, not edge information; the quad chain reads leaf
-// codes and corners, not leaf vertices.  The FP32-bound hermite overlaps the
-// latency-bound hash stages (its grid is sized by the autotuner for this), the
-// leaves overlap the quad stages, and the exports over C2C (about 190 GB/s)
-// start as soon as their data exists.
+// A small batch is bound by its longest chain of dependent kernels, field to
+// seams: hermite and the leaves lie on it, the quads and both tables do not.
+// (With the tables' primes, fill and inserts and the voxels one after the other
+// before the leaves, and the quads behind the leaf table, a 64^3 chunk took 118 us
+// and a 16^3 chunk 73, where they take 98 and 62.)  No branch reads what another
+// writes before their join: the voxels' rows take the changed plane once the edges
+// are listed, the tables read edge keys and leaf codes, the quads leaf codes and
+// corners.  In a large batch the FP32-bound hermite overlaps the latency-bound
+// rest (its grid is sized by the autotuner for this), and the exports over C2C
+// (about 190 GB/s) start as soon as their data exists.
 int enqueue_fresh_dag(lvn_meshgen* m, const BatchPtrs& b, bool any_ops, const DirectOut* direct) {
     cudaStream_t s0 = m->stream;
     LVN_CK(launch_reset(b, s0));
     LVN_CK(launch_field(b, s0));
     if (any_ops) LVN_CK(launch_csg(b, s0));
+    const cudaStream_t quad = m->aux2, tab = m->aux;
+    LVN_CK(cudaEventRecord(m->ev_field, s0));
+    LVN_CK(cudaStreamWaitEvent(quad, m->ev_field, 0));
+    LVN_CK(launch_vox_count(b, quad));
     LVN_CK(launch_edge_count(b, s0));
     LVN_CK(launch_edge_plan(b, s0));
+    LVN_CK(cudaEventRecord(m->ev_plan, s0));
     LVN_CK(launch_edge_scatter(b, s0));
     LVN_CK(cudaEventRecord(m->ev_fork, s0));
-    LVN_CK(cudaStreamWaitEvent(m->aux, m->ev_fork, 0));
     BatchPtrs bh = b;
     if (m->dag_hermite_per_sm > 0) bh.grid_per_sm[ST_HERMITE] = m->dag_hermite_per_sm;
-    LVN_CK(launch_hermite(bh, m->aux));
-    LVN_CK(cudaEventRecord(m->ev_herm, m->aux));
-    LVN_CK(launch_vox_count(b, s0));
-    LVN_CK(launch_vox_plan(b, s0));
-    LVN_CK(launch_vox_scatter(b, s0));
-    LVN_CK(launch_primes(b, s0));
-    LVN_CK(launch_hash_fill(b, s0));
+    LVN_CK(launch_hermite(bh, s0));
+    // the voxels; their rows take the changed plane, which the edges are done with
+    LVN_CK(cudaStreamWaitEvent(quad, m->ev_plan, 0));
+    LVN_CK(launch_vox_plan(b, quad));
+    LVN_CK(cudaEventRecord(m->ev_vplan, quad));
+    LVN_CK(cudaStreamWaitEvent(quad, m->ev_fork, 0));
+    LVN_CK(launch_vox_scatter(b, quad));
+    LVN_CK(cudaEventRecord(m->ev_vox, quad));
+    // the tables: the leaves wait for the edges'
+    BatchPtrs bt = b;
+    bt.tables = 1;
+    LVN_CK(cudaStreamWaitEvent(tab, m->ev_plan, 0));
+    LVN_CK(launch_primes(bt, tab));
+    LVN_CK(launch_hash_fill(bt, tab));
+    LVN_CK(cudaStreamWaitEvent(tab, m->ev_fork, 0));
+    LVN_CK(launch_edge_insert(bt, tab));
+    LVN_CK(cudaEventRecord(m->ev_etab, tab));
+    bt.tables = 2;
+    LVN_CK(cudaStreamWaitEvent(tab, m->ev_vplan, 0));
+    LVN_CK(launch_primes(bt, tab));
+    LVN_CK(launch_hash_fill(bt, tab));
+    LVN_CK(cudaStreamWaitEvent(tab, m->ev_vox, 0));
+    LVN_CK(launch_node_insert(bt, tab));
+    LVN_CK(cudaEventRecord(m->ev_hash, tab));
     const bool simp = b.simp_on != 0;
     const bool pipelined = direct && !simp;
     // the quad chain
-    LVN_CK(cudaEventRecord(m->ev_hash, s0));
-    LVN_CK(cudaStreamWaitEvent(m->aux2, m->ev_hash, 0));
-    LVN_CK(launch_node_insert(b, m->aux2));
-    LVN_CK(launch_mesh_count(b, m->aux2));
-    LVN_CK(launch_mesh_plan(b, m->aux2));
+    LVN_CK(launch_mesh_count(b, quad));
+    LVN_CK(launch_mesh_plan(b, quad));
     if (!simp) {
-        BatchPtrs bt = b;
-        bt.scatter_what = 1;  // triangles now, seams once the leaves exist
-        LVN_CK(launch_mesh_scatter(bt, m->aux2));
-        if (pipelined) LVN_CK(launch_export(b, 1, direct->dst[1], direct->cap[1], m->aux2));
+        BatchPtrs bq = b;
+        bq.scatter_what = 1;  // triangles now, seams once the leaves exist
+        LVN_CK(launch_mesh_scatter(bq, quad));
+        if (pipelined) LVN_CK(launch_export(b, 1, direct->dst[1], direct->cap[1], quad));
     }
-    LVN_CK(cudaEventRecord(m->ev_mesh, m->aux2));
-    // the leaves
-    LVN_CK(launch_edge_insert(b, s0));
-    LVN_CK(cudaStreamWaitEvent(s0, m->ev_herm, 0));
+    LVN_CK(cudaEventRecord(m->ev_mesh, quad));
+    // the leaves, behind the hermite data
+    LVN_CK(cudaStreamWaitEvent(s0, m->ev_vox, 0));
+    LVN_CK(cudaStreamWaitEvent(s0, m->ev_etab, 0));
     // pinned host vertices: k_leaf writes them itself when the array is
     // 16-byte aligned; otherwise the leaves run in slices, each exported on
     // the side stream while the next is computed
@@ -793,6 +815,7 @@ int enqueue_fresh_dag(lvn_meshgen* m, const BatchPtrs& b, bool any_ops, const Di
     }
     LVN_CK(launch_mesh_scatter(bs, s0));
     if (simp) LVN_CK(launch_simplify(b, s0));
+    LVN_CK(cudaStreamWaitEvent(s0, m->ev_hash, 0));
     if (direct) {
         if (simp) {
             const int rc = enqueue_exports(m, b, direct, s0);
@@ -1051,10 +1074,9 @@ int run_fresh_batch(lvn_meshgen* m, std::vector<ChunkDesc>& descs, const std::ve
         if (!m->aux) {
             LVN_CK(cudaStreamCreateWithFlags(&m->aux, cudaStreamNonBlocking));
             LVN_CK(cudaStreamCreateWithFlags(&m->aux2, cudaStreamNonBlocking));
-            LVN_CK(cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming));
-            LVN_CK(cudaEventCreateWithFlags(&m->ev_herm, cudaEventDisableTiming));
-            LVN_CK(cudaEventCreateWithFlags(&m->ev_hash, cudaEventDisableTiming));
-            LVN_CK(cudaEventCreateWithFlags(&m->ev_mesh, cudaEventDisableTiming));
+            for (cudaEvent_t* e : {&m->ev_field, &m->ev_plan, &m->ev_fork, &m->ev_vplan, &m->ev_vox, &m->ev_etab,
+                                   &m->ev_hash, &m->ev_mesh})
+                LVN_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         }
         auto enqueue_all = [&]() -> int {
             int r = enqueue_inputs(m, n, brushes.size());
@@ -1650,14 +1672,12 @@ void lvn_meshgen_destroy(lvn_meshgen* m) {
     for (int i = 0; i <= ST_COUNT; i++)
         if (m->ev[i]) cudaEventDestroy(m->ev[i]);
     if (m->graph_exec) cudaGraphExecDestroy(m->graph_exec);
-    if (m->ev_fork) cudaEventDestroy(m->ev_fork);
-    if (m->ev_hash) cudaEventDestroy(m->ev_hash);
-    if (m->ev_mesh) cudaEventDestroy(m->ev_mesh);
+    for (cudaEvent_t e : {m->ev_field, m->ev_plan, m->ev_fork, m->ev_vplan, m->ev_vox, m->ev_etab, m->ev_hash, m->ev_mesh})
+        if (e) cudaEventDestroy(e);
     if (m->aux2) cudaStreamDestroy(m->aux2);
     if (m->ev_leaf) cudaEventDestroy(m->ev_leaf);
     if (m->ev_side) cudaEventDestroy(m->ev_side);
     if (m->side) cudaStreamDestroy(m->side);
-    if (m->ev_herm) cudaEventDestroy(m->ev_herm);
     if (m->aux) cudaStreamDestroy(m->aux);
     if (m->own_stream) cudaStreamDestroy(m->stream);
     delete m;

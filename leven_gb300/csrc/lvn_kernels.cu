@@ -607,7 +607,8 @@ __global__ void k_reset(BatchPtrs b) {
 // Field bit planes.  Row (y, z) of a chunk's field packs x = 0..65 into a
 // uint4 (bits 0-31, 32-63, 64-65).  Plane 0: plain solid (material != AIR
 // before CSG); plane 1: final air (material == AIR after CSG); plane 2:
-// changed by this CSG batch.  Row index r = y + FD * z, so the linear
+// changed by this CSG batch until the edges are listed, then the chunk's
+// active voxels by row (VoxelRows).  Row index r = y + FD * z, so the linear
 // successor of field point (FD-1, y, z) is bit 0 of row r + 1, as in the
 // reference's linear field index.
 // ---------------------------------------------------------------------------
@@ -1257,20 +1258,28 @@ __device__ __forceinline__ int table_slot_bound(int k) {
     return k > 0 ? max((int)CUCKOO_MIN_TABLE_SIZE, 2 * k) + 512 + CUCKOO_STASH_SIZE : 0;
 }
 
-// The two cuckoo primes of every chunk, one warp per chunk.
+// The two cuckoo primes of every chunk, one warp per chunk (b.tables: 1 the edge
+// table's, 2 the leaf table's, 0 both).
 __global__ void __launch_bounds__(256) k_primes(BatchPtrs b) {
     if (b.bs->overflow) return;
     const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (c >= b.n) return;
     ChunkState& st = b.cs[c];
     const int e = st.num_edges, v = st.nodes;
-    const int pe = e > 0 ? warp_find_next_prime(max((int)CUCKOO_MIN_TABLE_SIZE, 2 * e)) : 0;
-    const int pv = v > 0 ? warp_find_next_prime(max((int)CUCKOO_MIN_TABLE_SIZE, 2 * v)) : 0;
-    if ((threadIdx.x & 31) == 0) {
-        st.edge_prime = (uint32_t)pe;
-        st.node_prime = (uint32_t)pv;
-        st.edge_magic = pe ? 0xffffffffu / (uint32_t)pe : 0u;
-        st.node_magic = pv ? 0xffffffffu / (uint32_t)pv : 0u;
+    const bool lane0 = (threadIdx.x & 31) == 0;
+    if (b.tables != 2) {
+        const int pe = e > 0 ? warp_find_next_prime(max((int)CUCKOO_MIN_TABLE_SIZE, 2 * e)) : 0;
+        if (lane0) {
+            st.edge_prime = (uint32_t)pe;
+            st.edge_magic = pe ? 0xffffffffu / (uint32_t)pe : 0u;
+        }
+    }
+    if (b.tables != 1) {
+        const int pv = v > 0 ? warp_find_next_prime(max((int)CUCKOO_MIN_TABLE_SIZE, 2 * v)) : 0;
+        if (lane0) {
+            st.node_prime = (uint32_t)pv;
+            st.node_magic = pv ? 0xffffffffu / (uint32_t)pv : 0u;
+        }
     }
 }
 
@@ -2061,6 +2070,26 @@ __device__ __forceinline__ VoxRow vox_row(const BatchPtrs& b, int c, int vrow) {
     return v;
 }
 
+// The leaf at a voxel, by rank: a chunk's leaves are listed in row order, then x
+// order, so a leaf's index is its row's first plus the active voxels before it.
+// Row (y, z)'s record {active bits 0-31, 32-63, first leaf} lies in plane 2, which
+// nothing reads once the edges are listed: one 16-byte load answers for a whole
+// row, where the leaf hash table costs a probe or more, with its modulo, for each
+// voxel.
+static_assert(sizeof(uint4) == 16 && Geo<64>::FD <= 96, "64 voxels in two words");
+struct VoxelRow {
+    uint4 r;
+    __device__ __forceinline__ int leaf(int x) const {  // chunk-local index, -1 = not active
+        const unsigned w = x < 32 ? r.x : r.y, m = (1u << (x & 31)) - 1u;
+        if (!((w >> (x & 31)) & 1u)) return -1;
+        return (int)r.z + __popc(w & m) + (x < 32 ? 0 : __popc(r.x));
+    }
+};
+template <int VPC>
+__device__ __forceinline__ VoxelRow voxel_row(const BatchPtrs& b, int c, int y, int z) {
+    return VoxelRow{plane_ptr<VPC>(b, c, 2)[y + Geo<VPC>::FD * z]};
+}
+
 template <int VPC>
 __global__ void __launch_bounds__(kThreads) k_vox_count(BatchPtrs b) {
     using G = Geo<VPC>;
@@ -2122,6 +2151,10 @@ __global__ void __launch_bounds__(kThreads) k_vox_scatter(BatchPtrs b) {
     const int cnt = popc4(act);
     int total;
     const int ex = block_exclusive<kThreads>(cnt, total, sm);
+    // the row's record for VoxelRow; a fresh field without operations left zeros
+    if (valid && (cnt > 0 || b.derive_mats == 0 || b.desc[c].op_count > 0))
+        plane_ptr<VPC>(b, c, 2)[vrow % VPC + G::FD * (vrow / VPC)] =
+            make_uint4(act.x, act.y, (unsigned)(b.vox_tiles[(size_t)c * G::NBV + tile] + ex), 0u);
     // the warp's active voxels, in row order then x order, are spread over
     // its lanes: voxel j of the warp goes to lane j % 32
     const int lane = threadIdx.x & 31;
@@ -2206,7 +2239,7 @@ __global__ void __launch_bounds__(kThreads) k_vox_scatter(BatchPtrs b) {
 
 __global__ void k_hash_fill(BatchPtrs b) {
     if (b.bs->overflow) return;
-    const long long ne = b.bs->total_edge_slots, nn = b.bs->total_node_slots;
+    const long long ne = b.tables != 2 ? b.bs->total_edge_slots : 0, nn = b.tables != 1 ? b.bs->total_node_slots : 0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ne + nn; i += stride) {
         if (i < ne) b.edge_slots[i] = CUCKOO_EMPTY;
@@ -2711,16 +2744,13 @@ __global__ void __launch_bounds__(kNodeTile) k_mesh_count(BatchPtrs b) {
         int packed = 0;
         if (local < st.nodes) {
             const int i = st.node_off + local;
-            HashView hv;
-            hv.prime = st.node_prime;
-            hv.magic = st.node_magic;
-            hv.table = b.node_slots + st.node_table_off;
-            hv.stash = hv.table + hv.prime;
-            hv.stash_used = st.node_stash_used;
-#pragma unroll
-            for (int k = 0; k < 10; k++) hv.p[k] = b.desc[c].node_params[k];
             int pos[3];
             position_for_code<VPC>(b.node_codes[i], pos[0], pos[1], pos[2]);
+            // the rows of the neighbours at (y, z) + (0, 0), (0, 1), (1, 0), (1, 1);
+            // on the chunk's faces the next row is not asked for
+            const int y1 = min(pos[1] + 1, VPC - 1), z1 = min(pos[2] + 1, VPC - 1);
+            const VoxelRow rows[4] = {voxel_row<VPC>(b, c, pos[1], pos[2]), voxel_row<VPC>(b, c, pos[1], z1),
+                                      voxel_row<VPC>(b, c, y1, pos[2]), voxel_row<VPC>(b, c, y1, z1)};
             const int corners = b.node_info[i] & 0xff;
             int quads = 0;
 #pragma unroll
@@ -2728,8 +2758,7 @@ __global__ void __launch_bounds__(kNodeTile) k_mesh_count(BatchPtrs b) {
                 int4 q = make_int4(-1, -1, -1, 0);
                 const int aa = pos[(axis + 1) % 3], bb = pos[(axis + 2) % 3];
                 // ProcessEdge (octree.cl:335-372): a quad needs the edge's sign
-                // change and all three neighbours; the sign is tested first, so
-                // that the neighbour lookups run only for the edges it passes
+                // change and all three neighbours
                 const int edge = axis * 4 + 3;
                 const int m1 = (corners >> edge_c0(edge)) & 1, m2 = (corners >> edge_c1(edge)) & 1;
                 if (aa != VPC - 1 && bb != VPC - 1 && m1 != m2) {
@@ -2741,7 +2770,7 @@ __global__ void __launch_bounds__(kNodeTile) k_mesh_count(BatchPtrs b) {
                         if (axis == 0) { oy = (k >> 1) & 1; oz = k & 1; }
                         else if (axis == 1) { ox = k & 1; oz = (k >> 1) & 1; }
                         else { oy = k & 1; ox = (k >> 1) & 1; }
-                        nb[k - 1] = (int)hv.find(code_for_position<VPC>(pos[0] + ox, pos[1] + oy, pos[2] + oz));
+                        nb[k - 1] = rows[2 * oy + oz].leaf(pos[0] + ox);
                     }
                     if (nb[0] != -1 && nb[1] != -1 && nb[2] != -1) {
                         q = make_int4(nb[0], nb[1], nb[2], 1 | (m1 != 0 ? 2 : 0));
@@ -2915,12 +2944,25 @@ __device__ __forceinline__ int* simp_cell(const BatchPtrs& b, int c, int k, int 
            n * (y + n * z);
 }
 
-// create the level-k entry of cell (x, y, z) of chunk c if it has none
+// create the level-k entry of cell (x, y, z) of chunk c if it has none; the whole
+// warp calls, lanes without a cell with `valid` false.  The lanes that won a cell
+// take their entries with one addition to the level's count (one a cell made the
+// count's atomics the kernel's time).
 template <int VPC>
-__device__ __forceinline__ void simp_claim(const BatchPtrs& b, int c, int k, int x, int y, int z) {
-    int* cell = simp_cell<VPC>(b, c, k, x, y, z);
-    if (atomicCAS(cell, -1, -2) != -1) return;
-    const int e = atomicAdd(b.simp_count + k, 1);
+__device__ __forceinline__ void simp_claim(const BatchPtrs& b, bool valid, int c, int k, int x, int y, int z) {
+    int* cell = nullptr;
+    bool won = false;
+    if (valid) {
+        cell = simp_cell<VPC>(b, c, k, x, y, z);
+        won = atomicCAS(cell, -1, -2) == -1;
+    }
+    const unsigned winners = __ballot_sync(FULL, won);
+    if (!winners) return;
+    const int lane = threadIdx.x & 31, first = __ffs(winners) - 1;
+    int e = 0;
+    if (lane == first) e = atomicAdd(b.simp_count + k, __popc(winners));
+    e = __shfl_sync(FULL, e, first) + __popc(winners & ((1u << lane) - 1u));
+    if (!won) return;
     SimpNode& n = b.simp_nodes[b.simp_level_off[k] + e];
     n.chunk = c;
     n.pos = x | (y << 8) | (z << 16);
@@ -2933,10 +2975,11 @@ template <int VPC>
 __global__ void __launch_bounds__(kThreads) k_simp_seed(BatchPtrs b) {
     if (b.bs->overflow) return;
     const int total = b.bs->total_nodes;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        int x, y, z;
-        position_for_code<VPC>(b.node_codes[i], x, y, z);
-        simp_claim<VPC>(b, b.node_chunk[i], 1, x >> 1, y >> 1, z >> 1);
+    for (int i0 = blockIdx.x * blockDim.x; i0 < total; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        int x = 0, y = 0, z = 0;
+        if (i < total) position_for_code<VPC>(b.node_codes[i], x, y, z);
+        simp_claim<VPC>(b, i < total, i < total ? b.node_chunk[i] : 0, 1, x >> 1, y >> 1, z >> 1);
     }
 }
 
@@ -2947,73 +2990,67 @@ __global__ void __launch_bounds__(kThreads) k_simp_level(BatchPtrs b, int k) {
     SimpNode* nodes = b.simp_nodes + b.simp_level_off[k];
     const SimpNode* below = b.simp_nodes + b.simp_level_off[k > 1 ? k - 1 : 1];
     const int h = 1 << (k - 1);
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
-        SimpNode& nd = nodes[e];
-        const int c = nd.chunk;
-        const int px = nd.pos & 255, py = (nd.pos >> 8) & 255, pz = nd.pos >> 16;
-        const ChunkState& st = b.cs[c];
-        HashView hv;
-        if (k == 1) {
-            hv.prime = st.node_prime;
-            hv.magic = st.node_magic;
-            hv.table = b.node_slots + st.node_table_off;
-            hv.stash = hv.table + hv.prime;
-            hv.stash_used = st.node_stash_used;
-#pragma unroll
-            for (int j = 0; j < 10; j++) hv.p[j] = b.desc[c].node_params[j];
-        }
-        bool blocked = false;
-        SimpQef q;
-        simp_zero(q);
-        int mats[8];
-        int anchor = 0x7fffffff;
-        for (int i = 0; i < 8; i++) {
-            const int ox = (i >> 2) & 1, oy = (i >> 1) & 1, oz = i & 1;  // CHILD_MIN_OFFSETS
-            const int cx = 2 * px + ox, cy = 2 * py + oy, cz = 2 * pz + oz;
-            mats[i] = MATERIAL_NONE;
-            if (blocked) continue;
-            if (k == 1) {
-                const uint32_t local = hv.find(code_for_position<VPC>(cx, cy, cz));
-                if (local == ~0u) continue;
-                if (cx == 0 || cx == VPC - 1 || cy == 0 || cy == VPC - 1 || cz == 0 || cz == VPC - 1) {
-                    blocked = true;  // seam voxels stay leaves
-                    continue;
+    for (int e0 = blockIdx.x * blockDim.x; e0 < count; e0 += gridDim.x * blockDim.x) {
+        const int e = e0 + threadIdx.x;
+        int c = 0, px = 0, py = 0, pz = 0;
+        if (e < count) {
+            SimpNode& nd = nodes[e];
+            c = nd.chunk;
+            px = nd.pos & 255, py = (nd.pos >> 8) & 255, pz = nd.pos >> 16;
+            const ChunkState& st = b.cs[c];
+            bool blocked = false;
+            SimpQef q;
+            simp_zero(q);
+            int mats[8];
+            int anchor = 0x7fffffff;
+            for (int i = 0; i < 8; i++) {
+                const int ox = (i >> 2) & 1, oy = (i >> 1) & 1, oz = i & 1;  // CHILD_MIN_OFFSETS
+                const int cx = 2 * px + ox, cy = 2 * py + oy, cz = 2 * pz + oz;
+                mats[i] = MATERIAL_NONE;
+                if (blocked) continue;
+                if (k == 1) {
+                    const int local = voxel_row<VPC>(b, c, cy, cz).leaf(cx);
+                    if (local < 0) continue;
+                    if (cx == 0 || cx == VPC - 1 || cy == 0 || cy == VPC - 1 || cz == 0 || cz == VPC - 1) {
+                        blocked = true;  // seam voxels stay leaves
+                        continue;
+                    }
+                    const int vi = st.node_off + local;
+                    simp_merge(q, b.leaf_qef[vi], (float)(ox * h), (float)(oy * h), (float)(oz * h));
+                    mats[i] = (b.node_info[vi] >> 8) & 0xff;
+                    anchor = min(anchor, local);
+                } else {
+                    const int ce = *simp_cell<VPC>(b, c, k - 1, cx, cy, cz);
+                    if (ce < 0) continue;
+                    const SimpNode& ch = below[ce];
+                    if (!ch.collapsed) {
+                        blocked = true;
+                        continue;
+                    }
+                    simp_merge(q, ch.q, (float)(ox * h), (float)(oy * h), (float)(oz * h));
+                    mats[i] = ch.material;
+                    anchor = min(anchor, ch.anchor);
                 }
-                const int vi = st.node_off + (int)local;
-                simp_merge(q, b.leaf_qef[vi], (float)(ox * h), (float)(oy * h), (float)(oz * h));
-                mats[i] = (b.node_info[vi] >> 8) & 0xff;
-                anchor = min(anchor, (int)local);
-            } else {
-                const int ce = *simp_cell<VPC>(b, c, k - 1, cx, cy, cz);
-                if (ce < 0) continue;
-                const SimpNode& ch = below[ce];
-                if (!ch.collapsed) {
-                    blocked = true;
-                    continue;
+            }
+            int collapsed = 0;
+            if (!blocked) {
+                float x, y, z;
+                const float err = simp_solve(q, (float)(2 * h), x, y, z);
+                if (err <= b.simp_threshold) {
+                    collapsed = 1;
+                    const ChunkDesc& d = b.desc[c];
+                    const float fs = (float)d.scale;
+                    nd.wpos[0] = fmaf(fs * ((float)(px << k) + x), (float)LEAF_SIZE_SCALE, (float)d.min[0]);
+                    nd.wpos[1] = fmaf(fs * ((float)(py << k) + y), (float)LEAF_SIZE_SCALE, (float)d.min[1]);
+                    nd.wpos[2] = fmaf(fs * ((float)(pz << k) + z), (float)LEAF_SIZE_SCALE, (float)d.min[2]);
+                    nd.material = dominant_material(mats);
+                    nd.anchor = anchor;
+                    nd.q = q;
                 }
-                simp_merge(q, ch.q, (float)(ox * h), (float)(oy * h), (float)(oz * h));
-                mats[i] = ch.material;
-                anchor = min(anchor, ch.anchor);
             }
+            nd.collapsed = collapsed;
         }
-        int collapsed = 0;
-        if (!blocked) {
-            float x, y, z;
-            const float err = simp_solve(q, (float)(2 * h), x, y, z);
-            if (err <= b.simp_threshold) {
-                collapsed = 1;
-                const ChunkDesc& d = b.desc[c];
-                const float fs = (float)d.scale;
-                nd.wpos[0] = fmaf(fs * ((float)(px << k) + x), (float)LEAF_SIZE_SCALE, (float)d.min[0]);
-                nd.wpos[1] = fmaf(fs * ((float)(py << k) + y), (float)LEAF_SIZE_SCALE, (float)d.min[1]);
-                nd.wpos[2] = fmaf(fs * ((float)(pz << k) + z), (float)LEAF_SIZE_SCALE, (float)d.min[2]);
-                nd.material = dominant_material(mats);
-                nd.anchor = anchor;
-                nd.q = q;
-            }
-        }
-        nd.collapsed = collapsed;
-        if (k < Geo<VPC>::DEPTH) simp_claim<VPC>(b, c, k + 1, px >> 1, py >> 1, pz >> 1);
+        if (k < Geo<VPC>::DEPTH) simp_claim<VPC>(b, e < count, c, k + 1, px >> 1, py >> 1, pz >> 1);
     }
 }
 

@@ -111,6 +111,7 @@ struct BatchPtrs {
     // see search_bounds
     float4* search;              // [n][kSearchEntries]
 
+    int tables;  // k_primes and k_hash_fill: 1 the edge table, 2 the leaf table, 0 both
     // k_mesh_scatter writes triangles (scatter_what 1), seams (2) or both (0);
     // k_leaf and the vertex export take slice `slice` of `nslices` equal leaf
     // ranges (nslices <= 1: all of them)
