@@ -604,11 +604,17 @@ __global__ void k_reset(BatchPtrs b) {
 }
 
 // ---------------------------------------------------------------------------
+// The overflow flags as one answer for the CTA: another stream's plan may set them
+// while a kernel starts, and threads that read them apart would part at a barrier.
+// A batch that overflowed is run again whatever its kernels still wrote.
+__device__ __forceinline__ bool any_overflow(const BatchPtrs& b) { return __syncthreads_or(b.bs->overflow); }
+
+// ---------------------------------------------------------------------------
 // Field bit planes.  Row (y, z) of a chunk's field packs x = 0..65 into a
 // uint4 (bits 0-31, 32-63, 64-65).  Plane 0: plain solid (material != AIR
 // before CSG); plane 1: final air (material == AIR after CSG); plane 2:
 // changed by this CSG batch until the edges are listed, then the chunk's
-// active voxels by row (VoxelRows).  Row index r = y + FD * z, so the linear
+// active voxels by row (VoxelRow).   Row index r = y + FD * z, so the linear
 // successor of field point (FD-1, y, z) is bit 0 of row r + 1, as in the
 // reference's linear field index.
 // ---------------------------------------------------------------------------
@@ -1396,7 +1402,7 @@ template <int VPC>
 __global__ void __launch_bounds__(kThreads) k_edge_scatter(BatchPtrs b) {
     using G = Geo<VPC>;
     __shared__ int sm[kThreads / 32 + 1];
-    if (b.bs->overflow) return;
+    if (any_overflow(b)) return;
     const int c = blockIdx.y, tile = blockIdx.x;
     const int row = tile * kThreads + threadIdx.x;
     const bool valid = row < G::FD * G::FD;
@@ -1941,7 +1947,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kHermiteSmemThreads, 1) k_hermite_smem(BatchPtrs b) {
     extern __shared__ __align__(16) uint8_t stab[];  // the lookup tables, the searches' densities and lists
     __shared__ __align__(16) float sg[64];
-    if (b.bs->overflow) return;  // the same for every thread
+    if (any_overflow(b)) return;
     stage_gradients(sg, b.grad);
     const uint4* src = reinterpret_cast<const uint4*>(b.perm_t3);
     for (int i = threadIdx.x; i < kT3Bytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(stab)[i] = __ldg(src + i);
@@ -2309,7 +2315,7 @@ template <bool NODES>
 __global__ void __launch_bounds__(kRepairThreads) k_hash_repair(BatchPtrs b) {
     __shared__ int list[kRepairThreads];
     __shared__ int nl, failed, stashed;
-    if (b.bs->overflow) return;  // the same for every thread
+    if (any_overflow(b)) return;
     if (threadIdx.x == 0) nl = 0;
     __syncthreads();
     const int c = blockIdx.x * kRepairThreads + threadIdx.x;
