@@ -2977,15 +2977,43 @@ __device__ __forceinline__ void simp_claim(const BatchPtrs& b, bool valid, int c
     atomicExch(cell, e);
 }
 
+// Level 1's entries: the cells of 2^3 voxels with a leaf, from the voxel rows.  A
+// thread takes a row of cells (four voxel rows), so no two claim a cell: 14 us
+// for 256 terrain chunks' 0.77 M leaves (41 with a compare-and-swap a leaf).
 template <int VPC>
 __global__ void __launch_bounds__(kThreads) k_simp_seed(BatchPtrs b) {
     if (b.bs->overflow) return;
-    const int total = b.bs->total_nodes;
-    for (int i0 = blockIdx.x * blockDim.x; i0 < total; i0 += gridDim.x * blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        int x = 0, y = 0, z = 0;
-        if (i < total) position_for_code<VPC>(b.node_codes[i], x, y, z);
-        simp_claim<VPC>(b, i < total, i < total ? b.node_chunk[i] : 0, 1, x >> 1, y >> 1, z >> 1);
+    constexpr int H = VPC / 2;
+    const int lane = threadIdx.x & 31;
+    const int total = b.n * (H * H);  // a multiple of 16; whole warps enter the loop
+    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < total; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + lane;
+        const int c = min(i, total - 1) / (H * H), y = i % H, z = i / H % H;
+        unsigned long long cells = 0;  // bit 2 x of cell x
+        if (i < total && b.cs[c].nodes > 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint4 r = voxel_row<VPC>(b, c, 2 * y + (k & 1), 2 * z + (k >> 1)).r;
+                cells |= (unsigned long long)r.y << 32 | r.x;
+            }
+            cells = (cells | cells >> 1) & 0x5555555555555555ull;
+        }
+        const int count = __popcll(cells), inc = warp_inclusive(count);
+        const int all = __shfl_sync(FULL, inc, 31);
+        if (!all) continue;
+        int e = 0;
+        if (lane == 0) e = atomicAdd(b.simp_count + 1, all);
+        e = __shfl_sync(FULL, e, 0) + inc - count;
+        int* row = simp_cell<VPC>(b, c, 1, 0, min(y, H - 1), min(z, H - 1));
+        for (; cells; cells &= cells - 1, e++) {
+            const int x = (__ffsll((long long)cells) - 1) >> 1;
+            SimpNode& n = b.simp_nodes[b.simp_level_off[1] + e];
+            n.chunk = c;
+            n.pos = x | (y << 8) | (z << 16);
+            n.collapsed = 0;
+            n.anchor = 0;
+            row[x] = e;
+        }
     }
 }
 
