@@ -12,7 +12,9 @@
 // the children still to visit, so only the nodes the reference's recursion
 // reaches are examined.  The listed nodes are then sorted in shared memory
 // into the recursion's order (pre-order for the selection, post-order for the
-// touch set) by a key built from their leaf-grid position.
+// touch set) by a key built from their leaf-grid position.  A selection of
+// ordinary size is made by one warp per camera instead, which keeps each level
+// in the recursion's order and counts places: it sorts nothing.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,9 +47,13 @@ constexpr int kWalkThreads = 256;
 constexpr int kSlotNodes = 2 * kMaxOpen + kMaxNodes;  // scratch per CTA: two open lists + the listed nodes
 constexpr int kHostStride = 1024;                     // first-pass list length per camera, host-buffer form
 constexpr int kMaxBoxes = 4096;                       // operations per touch-set call
-constexpr int kWarpList = 1024;  // selection by one warp per camera: listed nodes
-constexpr int kWarpOpen = 512;   // and open nodes per level; beyond either the CTA walk redoes the camera
-constexpr int kWarpsPerCta = 8;
+// selection by one warp per camera: the nodes it visits (listed ones, open ones
+// and the top level's), beyond which the CTA walk redoes the camera, its top
+// level's limit, and the warps of a CTA.  55 KB a CTA, four CTAs an SM: 28 warps,
+// so that 4096 cameras run at once on 152 SMs.
+constexpr int kWarpItems = 1264;
+constexpr int kWarpTop = 512;
+constexpr int kWarpsPerCta = 7;
 constexpr int kRedo = -2;        // count of a camera the warp walk left to the CTA walk
 
 struct Node {
@@ -226,112 +232,152 @@ __global__ void __launch_bounds__(kWalkThreads) k_clipmap_walk(Tree t, const flo
 }
 
 // Selection with one warp per camera (warp-synchronous: ballots, shuffles and
-// __syncwarp, no CTA barriers).  Open nodes are packed leaf-grid positions
-// (10 bits an axis) and LOD; a listed node is kept only as its sort key, which
-// identifies it (first leaf and LOD).  A camera that lists more than
-// kWarpList nodes or opens more than kWarpOpen in a level gets kRedo.
-__device__ __forceinline__ uint64_t pack_open(const int32_t p[3], int lod) {
-    return ((uint64_t)p[0] << 23) | ((uint64_t)p[1] << 13) | ((uint64_t)p[2] << 3) | (uint64_t)lod;
-}
+// __syncwarp, no CTA barriers).  The levels' nodes lie one level behind the other,
+// each level in the recursion's order: the top level in Morton order, then every
+// open node's eight children in their parents' order (so a level starts at a
+// multiple of 8, an open node's children are an aligned group, and the r-th open
+// node of a level owns the next level's group r).  Going down, the nodes are
+// tested; going up, an open node's listed descendants are summed from its group;
+// going down again, a node's place is its parent's plus the listed ones before it
+// in the group, and the listed nodes go straight to their places.  A camera that
+// visits more than kWarpItems nodes gets kRedo.
+//
+// Bound by the latency of about 45 dependent steps of 32 nodes.  4096 cameras
+// (420 listed nodes each on average) take 29 us with the walk of what is left over;
+// sorting the listed nodes' keys, a bitonic network of 45 passes, it was 145.
+struct alignas(16) WarpSelection {
+    uint32_t pos[kWarpItems];        // leaf-grid position, 10 bits an axis; the LOD is the level's
+    uint16_t count[kWarpItems];      // listed nodes at and below; kOpenNode = has children here
+    uint16_t first[kWarpItems / 8];  // a group's first place
+    int32_t start[8], size[8];       // by level
+};
+constexpr unsigned kOpenNode = 0x8000u;
+static_assert(kNumLods <= 8 && kWarpItems % 16 == 0 && kWarpItems < (int)kOpenNode, "levels, groups, counts");
+static_assert(kWarpTop <= kWarpItems && 4 * (sizeof(WarpSelection) * kWarpsPerCta + 1024) <= 228 * 1024, "four CTAs an SM");
 
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_clipmap_select_warp(Tree t, const float* __restrict__ cams,
-                                                                          int num_queries, uint64_t* scratch,
-                                                                          lvn_chunk_desc* out, int stride,
-                                                                          int32_t* counts) {
-    extern __shared__ unsigned long long wkeys[];  // [kWarpsPerCta][kWarpList]
+                                                                          int num_queries, lvn_chunk_desc* out,
+                                                                          int stride, int32_t* counts) {
+    extern __shared__ __align__(16) uint8_t selections[];  // [kWarpsPerCta]
+    constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1;
-    unsigned long long* keys = wkeys + wib * kWarpList;
-    const int wslot = blockIdx.x * kWarpsPerCta + wib;
-    uint64_t* open = scratch + (size_t)wslot * 2 * kWarpOpen;  // list c at open + c * kWarpOpen
+    WarpSelection& w = reinterpret_cast<WarpSelection*>(selections)[wib];
     const int leaf = CLIPMAP_LEAF_SIZE;
-    for (int q = wslot; q < num_queries; q += gridDim.x * kWarpsPerCta) {
+    for (int q = blockIdx.x * kWarpsPerCta + wib; q < num_queries; q += gridDim.x * kWarpsPerCta) {
         const float cam[3] = {cams[3 * q], cams[3 * q + 1], cams[3 * q + 2]};
-        const int per = t.per, ntop = per * per * per, top_units = t.top_size / leaf;
-        for (int i = lane; i < ntop; i += 32) {  // the host keeps ntop <= kWarpOpen for this walk
-            const int32_t p[3] = {(i / (per * per)) * top_units, ((i / per) % per) * top_units, (i % per) * top_units};
-            open[i] = pack_open(p, t.top_lod);
+        // the top level (the host keeps it within kWarpTop): i's bits are triples
+        // of one bit an axis, as in the recursion
+        const int ntop = t.per * t.per * t.per, top_units = t.top_size / leaf;
+        for (int i = lane; i < ntop; i += 32) {
+            int p[3] = {0, 0, 0};
+            for (int bit = 0; (1 << bit) < t.per; bit++)
+                for (int a = 0; a < 3; a++) p[a] |= ((i >> (3 * bit + 2 - a)) & 1) << bit;
+            w.pos[i] = (uint32_t)(p[0] * top_units) << 20 | (uint32_t)(p[1] * top_units) << 10 | (uint32_t)(p[2] * top_units);
         }
         __syncwarp();
-        int cur = 0, n = ntop, listed = 0;
+        int s = 0, n = ntop, levels = 0;
         bool over = false;
-        for (int lod = t.top_lod; lod >= 0; lod--) {
-            int next = 0;
+        for (int lod = t.top_lod; lod >= 0 && n > 0; lod--) {
+            const int child = (s + n + 7) & ~7;  // the next level's start
+            int opened = 0;
             for (int base = 0; base < n; base += 32) {
-                const int i = base + lane;
-                Node nd;
+                const int i = s + base + lane;
                 bool list = false, expand = false;
-                if (i < n) {
-                    const uint64_t o = open[cur * kWarpOpen + i];
-                    const int32_t p[3] = {(int32_t)((o >> 23) & 1023), (int32_t)((o >> 13) & 1023),
-                                          (int32_t)((o >> 3) & 1023)};
-                    for (int a = 0; a < 3; a++) nd.min[a] = t.root_min[a] + p[a] * leaf;
+                uint32_t p = 0;
+                if (base + lane < n) {
+                    p = w.pos[i];
+                    Node nd;
+                    nd.min[0] = t.root_min[0] + (int)(p >> 20) * leaf;
+                    nd.min[1] = t.root_min[1] + (int)((p >> 10) & 1023u) * leaf;
+                    nd.min[2] = t.root_min[2] + (int)(p & 1023u) * leaf;
                     nd.size = leaf << lod;
                     list = distance_to_node(nd, cam) >= kLodActiveDistances[lod];
                     expand = !list && lod > 0;
+                    w.count[i] = (uint16_t)(list ? 1u : expand ? kOpenNode : 0u);
                 }
-                const unsigned bl = __ballot_sync(0xffffffffu, list);
-                if (list) {
-                    const int pos = listed + __popc(bl & below);
-                    if (pos < kWarpList) keys[pos] = order_key(nd, t, lod, false);
+                const unsigned be = __ballot_sync(FULL, expand);
+                const int at = child + 8 * (opened + __popc(be & below));
+                if (expand && at + 8 <= kWarpItems) {
+                    const uint32_t h = 1u << (lod - 1);
+                    uint4* const c = reinterpret_cast<uint4*>(w.pos + at);
+                    c[0] = make_uint4(p, p + h, p + (h << 10), p + (h << 10) + h);
+                    p += h << 20;
+                    c[1] = make_uint4(p, p + h, p + (h << 10), p + (h << 10) + h);
                 }
-                listed += __popc(bl);
-                const unsigned be = __ballot_sync(0xffffffffu, expand);
-                if (expand) {
-                    const int pos = next + 8 * __popc(be & below);
-                    const int32_t h = (nd.size >> 1) / leaf;
-                    int32_t p[3];
-                    for (int a = 0; a < 3; a++) p[a] = (nd.min[a] - t.root_min[a]) / leaf;
-                    for (int c = 0; c < 8; c++) {
-                        const int32_t cp[3] = {p[0] + ((c >> 2) & 1) * h, p[1] + ((c >> 1) & 1) * h, p[2] + (c & 1) * h};
-                        if (pos + c < kWarpOpen) open[(cur ^ 1) * kWarpOpen + pos + c] = pack_open(cp, lod - 1);
-                    }
-                }
-                next += 8 * __popc(be);
+                opened += __popc(be);
+            }
+            if (lane == 0) w.start[levels] = s, w.size[levels] = n;
+            levels++;
+            s = child;
+            n = 8 * opened;
+            if (s + n > kWarpItems) {
+                over = true;
+                break;
             }
             __syncwarp();
-            over |= next > kWarpOpen;
-            n = min(next, kWarpOpen);
-            cur ^= 1;
         }
-        over |= listed > kWarpList;
-        if (!over) {
-            // bitonic network over any n (mirrored first step), warp-synchronous
-            for (int k = 2; k < 2 * listed; k <<= 1) {
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const int mask = j == (k >> 1) ? k - 1 : j;
-                    for (int i = lane; i < listed; i += 32) {
-                        const int l = i ^ mask;
-                        if (l > i && l < listed) {
-                            const unsigned long long a = keys[i], b = keys[l];
-                            if (a > b) {
-                                keys[i] = b;
-                                keys[l] = a;
-                            }
-                        }
-                    }
-                    __syncwarp();
+        __syncwarp();
+        if (over) {
+            if (lane == 0) counts[q] = kRedo;
+            continue;
+        }
+        for (int l = levels - 2; l >= 0; l--) {
+            const int from = w.start[l], len = w.size[l], child = w.start[l + 1];
+            int opened = 0;
+            for (int base = 0; base < len; base += 32) {
+                const int i = from + base + lane;
+                const bool open = base + lane < len && (w.count[i] & kOpenNode);
+                const unsigned bo = __ballot_sync(FULL, open);
+                if (open) {  // at most kWarpItems below: the halves do not meet
+                    const uint4 k = *reinterpret_cast<const uint4*>(w.count + child + 8 * (opened + __popc(bo & below)));
+                    const unsigned m = 0x7fff7fffu, sum = (k.x & m) + (k.y & m) + (k.z & m) + (k.w & m);
+                    w.count[i] = (uint16_t)(kOpenNode | ((sum & 0xffffu) + (sum >> 16)));
+                }
+                opened += __popc(bo);
+            }
+            __syncwarp();
+        }
+        int listed = 0;
+        for (int l = 0; l < levels; l++) {
+            const int from = w.start[l], len = w.size[l], child = l + 1 < levels ? w.start[l + 1] : 0;
+            const int lod = t.top_lod - l;
+            int opened = 0;
+            for (int base = 0; base < len; base += 32) {
+                const int i = from + base + lane;
+                const unsigned c = base + lane < len ? w.count[i] : 0u;
+                const int below_here = (int)(c & (kOpenNode - 1u));
+                int place = below_here;  // inclusive, then exclusive, over the warp or the group
+                const int width = l == 0 ? 32 : 8;
+                for (int d = 1; d < width; d <<= 1) {
+                    const int v = __shfl_up_sync(FULL, place, d);
+                    if ((lane & (width - 1)) >= d) place += v;
+                }
+                const int upto = place;
+                place -= below_here;
+                if (l == 0) {
+                    place += listed;
+                    listed += __shfl_sync(FULL, upto, 31);
+                } else if (base + lane < len) {
+                    place += w.first[i >> 3];
+                }
+                const bool open = (c & kOpenNode) != 0;
+                const unsigned bo = __ballot_sync(FULL, open);
+                if (open) w.first[(child >> 3) + opened + __popc(bo & below)] = (uint16_t)place;
+                opened += __popc(bo);
+                if (c == 1u && place < stride) {
+                    const uint32_t p = w.pos[i];
+                    lvn_chunk_desc d;
+                    d.min[0] = t.root_min[0] + (int)(p >> 20) * leaf;
+                    d.min[1] = t.root_min[1] + (int)((p >> 10) & 1023u) * leaf;
+                    d.min[2] = t.root_min[2] + (int)(p & 1023u) * leaf;
+                    d.size = leaf << lod;
+                    out[(size_t)q * stride + place] = d;
                 }
             }
-            const int nout = min(listed, stride);
-            for (int i = lane; i < nout; i += 32) {
-                const unsigned long long key = keys[i];
-                const int lod = (int)(key & 7);
-                const unsigned long long code = key >> 3;
-                int32_t p[3] = {0, 0, 0};
-                for (int bit = t.depth - 1; bit >= 0; bit--) {
-                    const int tr = (int)((code >> (3 * bit)) & 7);
-                    p[0] = (p[0] << 1) | ((tr >> 2) & 1);
-                    p[1] = (p[1] << 1) | ((tr >> 1) & 1);
-                    p[2] = (p[2] << 1) | (tr & 1);
-                }
-                lvn_chunk_desc d;
-                for (int a = 0; a < 3; a++) d.min[a] = t.root_min[a] + p[a] * leaf;
-                d.size = leaf << lod;
-                out[(size_t)q * stride + i] = d;
-            }
+            __syncwarp();
         }
-        if (lane == 0) counts[q] = over ? kRedo : listed;
+        if (lane == 0) counts[q] = listed;
         __syncwarp();
     }
 }
@@ -382,7 +428,6 @@ struct Work {
     Grow<lvn_chunk_desc> wide, wide_big, packed;   // pass outputs (stride kHostStride / kMaxNodes), packed lists
     Grow<int32_t, true> hcounts, hplace;           // pinned
     int32_t* dboxes = nullptr;                     // kMaxBoxes x 6
-    Grow<uint64_t> wscratch;                       // the warp walk's open lists
 };
 Work& work() {
     static Work w;
@@ -432,7 +477,7 @@ int ensure_work(Work& w, int num_queries) {
         CM_TRY(cudaFuncSetAttribute(k_clipmap_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(sizeof(unsigned long long) * kMaxNodes)));
         CM_TRY(cudaFuncSetAttribute(k_clipmap_select_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(unsigned long long) * kWarpList * kWarpsPerCta)));
+                                    (int)sizeof(WarpSelection) * kWarpsPerCta));
         CM_TRY(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
         CM_TRY(cudaMalloc(&w.dboxes, sizeof(int32_t) * 6 * kMaxBoxes));
         w.device = dev;
@@ -462,14 +507,13 @@ void launch_walk(const Work& w, const Tree& t, const float* dcams, int num_queri
 // CTA walk for the cameras it left (on the same stream).
 int launch_select(Work& w, const Tree& t, const float* dcams, int num_queries, lvn_chunk_desc* out, int stride,
                   int32_t* counts, cudaStream_t s) {
-    if (t.per * t.per * t.per > kWarpOpen) {
+    if (t.per * t.per * t.per > kWarpTop) {
         launch_walk(w, t, dcams, num_queries, nullptr, 0, out, stride, counts, s);
         return cuda_rc(cudaGetLastError());
     }
-    const int ctas = std::max(1, std::min((num_queries + kWarpsPerCta - 1) / kWarpsPerCta, 3 * w.num_sms));
-    CM_TRY(w.wscratch.fit((size_t)ctas * kWarpsPerCta * 2 * kWarpOpen));
-    k_clipmap_select_warp<<<ctas, kWarpsPerCta * 32, sizeof(unsigned long long) * kWarpList * kWarpsPerCta, s>>>(
-        t, dcams, num_queries, w.wscratch.p, out, stride, counts);
+    const int ctas = std::max(1, std::min((num_queries + kWarpsPerCta - 1) / kWarpsPerCta, 4 * w.num_sms));
+    k_clipmap_select_warp<<<ctas, kWarpsPerCta * 32, sizeof(WarpSelection) * kWarpsPerCta, s>>>(t, dcams, num_queries,
+                                                                                               out, stride, counts);
     CM_TRY(cudaGetLastError());
     launch_walk(w, t, dcams, num_queries, nullptr, 0, out, stride, counts, s, 1);
     return cuda_rc(cudaGetLastError());

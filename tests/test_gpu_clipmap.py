@@ -33,6 +33,23 @@ def test_select_batch(lvn_gpu, root_min, root_size):
         assert np.array_equal(got[q], ref), (q, cam)
 
 
+@pytest.mark.parametrize("log2root", [9, 13, 14, 15, 16])
+def test_select_levels(lvn_gpu, log2root):
+    """One to 512 nodes at the top level and two to six levels below them, with
+    cameras among the leaves (the most nodes visited), far outside, and not
+    finite."""
+    lvn = lvn_gpu
+    size = 1 << log2root
+    lo = (-size // 2, -256, 1024 - size)
+    rng = np.random.default_rng(log2root)
+    cams = np.concatenate([rng.uniform(lo, np.array(lo) + size, (60, 3)), rng.uniform(-4 * size, 4 * size, (20, 3)),
+                           np.array(lo) + size / 2 + rng.uniform(-256, 256, (20, 3)),
+                           [[np.inf, 0, 0], [0, -np.inf, 0], [3e38, 3e38, -3e38]]]).astype(np.float32)
+    got = lvn.clipmap_select(cams, lo, size)
+    for q, cam in enumerate(cams):
+        assert np.array_equal(got[q], O.clipmap_select(cam, lo, size)), (q, cam)
+
+
 def test_select_device_form(lvn_gpu):
     """The device form on torch buffers: lists truncated at the stride, full
     counts reported, nothing synchronised by the call."""
