@@ -706,6 +706,17 @@ int enqueue_exports(lvn_meshgen* m, const BatchPtrs& b, const DirectOut* direct,
     return LVN_OK;
 }
 
+// The streams and events of the batch DAG.
+int ensure_aux(lvn_meshgen* m) {
+    if (m->aux) return LVN_OK;
+    LVN_CK(cudaStreamCreateWithFlags(&m->aux, cudaStreamNonBlocking));
+    LVN_CK(cudaStreamCreateWithFlags(&m->aux2, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&m->ev_field, &m->ev_plan, &m->ev_fork, &m->ev_vplan, &m->ev_vox, &m->ev_etab, &m->ev_hash,
+                           &m->ev_mesh})
+        LVN_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    return LVN_OK;
+}
+
 constexpr int kLeafSlices = 4;  // leaf / vertex-export pipeline depth for pinned host outputs
 
 // The fresh-batch DAG (one graph when captured):
@@ -729,23 +740,10 @@ constexpr int kLeafSlices = 4;  // leaf / vertex-export pipeline depth for pinne
 // corners.  In a large batch the FP32-bound hermite overlaps the latency-bound
 // rest (its grid is sized by the autotuner for this), and the exports over C2C
 // (about 190 GB/s) start as soon as their data exists.
-int enqueue_fresh_dag(lvn_meshgen* m, const BatchPtrs& b, bool any_ops, const DirectOut* direct) {
-    cudaStream_t s0 = m->stream;
-    LVN_CK(launch_reset(b, s0));
-    LVN_CK(launch_field(b, s0));
-    if (any_ops) LVN_CK(launch_csg(b, s0));
-    const cudaStream_t quad = m->aux2, tab = m->aux;
-    LVN_CK(cudaEventRecord(m->ev_field, s0));
-    LVN_CK(cudaStreamWaitEvent(quad, m->ev_field, 0));
-    LVN_CK(launch_vox_count(b, quad));
-    LVN_CK(launch_edge_count(b, s0));
-    LVN_CK(launch_edge_plan(b, s0));
-    LVN_CK(cudaEventRecord(m->ev_plan, s0));
-    LVN_CK(launch_edge_scatter(b, s0));
-    LVN_CK(cudaEventRecord(m->ev_fork, s0));
-    BatchPtrs bh = b;
-    if (m->dag_hermite_per_sm > 0) bh.grid_per_sm[ST_HERMITE] = m->dag_hermite_per_sm;
-    LVN_CK(launch_hermite(bh, s0));
+// The part behind the edges: voxels, tables, quads, leaves, seams.  ev_plan (the
+// edge plan) and ev_fork (the edges) are recorded, the voxel counts enqueued on aux2.
+int enqueue_mesh_dag(lvn_meshgen* m, const BatchPtrs& b, const DirectOut* direct) {
+    const cudaStream_t s0 = m->stream, quad = m->aux2, tab = m->aux;
     // the voxels; their rows take the changed plane, which the edges are done with
     LVN_CK(cudaStreamWaitEvent(quad, m->ev_plan, 0));
     LVN_CK(launch_vox_plan(b, quad));
@@ -829,6 +827,25 @@ int enqueue_fresh_dag(lvn_meshgen* m, const BatchPtrs& b, bool any_ops, const Di
         }
     }
     return LVN_OK;
+}
+
+int enqueue_fresh_dag(lvn_meshgen* m, const BatchPtrs& b, bool any_ops, const DirectOut* direct) {
+    cudaStream_t s0 = m->stream;
+    LVN_CK(launch_reset(b, s0));
+    LVN_CK(launch_field(b, s0));
+    if (any_ops) LVN_CK(launch_csg(b, s0));
+    LVN_CK(cudaEventRecord(m->ev_field, s0));
+    LVN_CK(cudaStreamWaitEvent(m->aux2, m->ev_field, 0));
+    LVN_CK(launch_vox_count(b, m->aux2));
+    LVN_CK(launch_edge_count(b, s0));
+    LVN_CK(launch_edge_plan(b, s0));
+    LVN_CK(cudaEventRecord(m->ev_plan, s0));
+    LVN_CK(launch_edge_scatter(b, s0));
+    LVN_CK(cudaEventRecord(m->ev_fork, s0));
+    BatchPtrs bh = b;
+    if (m->dag_hermite_per_sm > 0) bh.grid_per_sm[ST_HERMITE] = m->dag_hermite_per_sm;
+    LVN_CK(launch_hermite(bh, s0));
+    return enqueue_mesh_dag(m, b, direct);
 }
 
 // Device addresses of caller arrays that are pinned (or registered) host
@@ -1071,13 +1088,7 @@ int run_fresh_batch(lvn_meshgen* m, std::vector<ChunkDesc>& descs, const std::ve
             rc = surrogate_prologue(m, descs, brushes.size(), b);
             if (rc) return rc;
         }
-        if (!m->aux) {
-            LVN_CK(cudaStreamCreateWithFlags(&m->aux, cudaStreamNonBlocking));
-            LVN_CK(cudaStreamCreateWithFlags(&m->aux2, cudaStreamNonBlocking));
-            for (cudaEvent_t* e : {&m->ev_field, &m->ev_plan, &m->ev_fork, &m->ev_vplan, &m->ev_vox, &m->ev_etab,
-                                   &m->ev_hash, &m->ev_mesh})
-                LVN_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-        }
+        if ((rc = ensure_aux(m))) return rc;
         auto enqueue_all = [&]() -> int {
             int r = enqueue_inputs(m, n, brushes.size());
             if (m->profile) {  // one stage at a time, each timed
@@ -1315,15 +1326,17 @@ int one_desc(lvn_meshgen* m, const int32_t min[3], int32_t size, std::vector<Chu
     return build_descs(m, &cd, 1, descs, none, false);
 }
 
-// Copy the pool state of chunk 0 (corners + edge list) into a field entry.
-int save_field(lvn_meshgen* m, FieldEntry& f) {
+// Copy chunk 0's edge list, and its corners if they are in the pools, into a field entry.
+int save_field(lvn_meshgen* m, FieldEntry& f, bool corners) {
     const ChunkState& cs = m->last_cs[0];
-    const size_t F = (size_t)field_size(m->vpc);
-    const size_t PB = sizeof(uint4) * 3 * (size_t)field_rows(m->vpc);
-    LVN_CK(f.mats.ensure(F));
-    LVN_CK(f.planes.ensure(PB));
-    LVN_CK(cudaMemcpyAsync(f.mats.p, m->mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
-    LVN_CK(cudaMemcpyAsync(f.planes.p, m->planes.p, PB, cudaMemcpyDeviceToDevice, m->stream));
+    if (corners) {
+        const size_t F = (size_t)field_size(m->vpc);
+        const size_t PB = sizeof(uint4) * 3 * (size_t)field_rows(m->vpc);
+        LVN_CK(f.mats.ensure(F));
+        LVN_CK(f.planes.ensure(PB));
+        LVN_CK(cudaMemcpyAsync(f.mats.p, m->mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
+        LVN_CK(cudaMemcpyAsync(f.planes.p, m->planes.p, PB, cudaMemcpyDeviceToDevice, m->stream));
+    }
     f.num_edges = cs.num_edges;
     LVN_CK(f.keys.ensure(sizeof(int32_t) * std::max(1, cs.num_edges)));
     LVN_CK(f.info.ensure(sizeof(float4) * std::max(1, cs.num_edges)));
@@ -1354,7 +1367,7 @@ int generate_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntr
     m->last_fresh = false;
     if (m->h_bs.as<BatchState>()->overflow) return LVN_ERR_DEVICE_STATUS;
     f.last_op = 0;
-    return save_field(m, f);
+    return save_field(m, f, true);
 }
 
 // ApplyCSGOperations on a cached field (compute_csg.cpp:11-219)
@@ -1375,13 +1388,15 @@ int apply_csg_to_field(lvn_meshgen* m, const int32_t min[3], int32_t size, Field
     cap.vcap = std::max(cap.vcap, m->vcap);
     if ((rc = ensure_pools(m, 1, cap))) return rc;
     if ((rc = upload(m, descs, brushes))) return rc;
-    const size_t F = (size_t)field_size(m->vpc);
+    // the corners are changed in place; the pools are sized for every edge the new
+    // list can have, so nothing after the first kernel gives the change up
     const size_t R = (size_t)field_rows(m->vpc);
-    LVN_CK(cudaMemcpyAsync(m->mats.p, f.mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
-    LVN_CK(cudaMemcpyAsync(m->planes.p, f.planes.p, sizeof(uint4) * 2 * R, cudaMemcpyDeviceToDevice, m->stream));
-    // no corner is changed by this batch until the CSG kernel says so
-    LVN_CK(cudaMemsetAsync(m->planes.as<uint4>() + 2 * R, 0, sizeof(uint4) * R, m->stream));
     BatchPtrs b = make_ptrs(m, 1);
+    b.mats = f.mats.as<uint8_t>();
+    b.planes = f.planes.as<uint4>();
+    m->dbg_mats = b.mats;
+    // no corner is changed by this batch until the CSG kernel says so
+    LVN_CK(cudaMemsetAsync(b.planes + 2 * R, 0, sizeof(uint4) * R, m->stream));
     b.plain_class = 0;
     b.need_mats = 1;
     b.derive_mats = 0;
@@ -1399,7 +1414,7 @@ int apply_csg_to_field(lvn_meshgen* m, const int32_t min[3], int32_t size, Field
     if ((rc = read_states(m, 1))) return rc;
     m->last_fresh = false;
     if (m->h_bs.as<BatchState>()->overflow) return LVN_ERR_DEVICE_STATUS;
-    return save_field(m, f);
+    return save_field(m, f, false);
 }
 
 // LoadDensityField (compute_density_field.cpp:235-274)
@@ -1476,8 +1491,19 @@ int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEnt
         m->dbg_mats = b.mats;
         m->dbg_keys = b.edge_keys;
         m->dbg_info = b.edge_info;
-        if ((rc = enqueue_octree_stages(m, b))) return rc;
-        if (staged && (rc = enqueue_exports(m, b, staged, m->stream))) return rc;
+        if (m->profile) {  // one stage at a time, each timed
+            if ((rc = enqueue_octree_stages(m, b))) return rc;
+            if (staged && (rc = enqueue_exports(m, b, staged, m->stream))) return rc;
+        } else {  // the fresh batch's DAG from the edges on (one stage after
+            // another: 334 us for an edit and a remesh of a 64^3 chunk, 265 so, the copies of the corners
+            // into the pools and back included)
+            if ((rc = ensure_aux(m))) return rc;
+            LVN_CK(cudaEventRecord(m->ev_plan, m->stream));
+            LVN_CK(cudaEventRecord(m->ev_fork, m->stream));
+            LVN_CK(cudaStreamWaitEvent(m->aux2, m->ev_fork, 0));
+            LVN_CK(launch_vox_count(b, m->aux2));
+            if ((rc = enqueue_mesh_dag(m, b, staged))) return rc;
+        }
         if ((rc = read_states(m, 1))) return rc;
         m->last_fresh = false;
         const BatchState& hb = *m->h_bs.as<BatchState>();
