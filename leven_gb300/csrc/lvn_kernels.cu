@@ -661,81 +661,90 @@ __device__ __forceinline__ float dens_h(const N& nz, const DensityParams& dp, fl
 
 // ---------------------------------------------------------------------------
 // stage 1: density field (GenerateDefaultField, density_field.cl:11-37)
-// One CTA per (z slice, chunk), one thread per x; heightfield modes evaluate
-// the height term once per (x, z) column.  Writes the byte materials and the
-// three bit planes (warp ballots along x).
-// ---------------------------------------------------------------------------
-
-template <int VPC, int MODE>
+// Heightfield modes evaluate the height term once per (x, z) column.  Writes the
+// byte materials and the three bit planes (warp ballots along x).
+//
+// A CTA takes ZB rows of z: their heights one after the other over its threads
+// (66 columns leave two lanes in a row's third warp, a third of the noise's
+// instructions; 264 leave eight idle threads in three passes), then a warp a row
+// for the bits.  ZB = 4 from kFieldRowsChunks chunks on (442 terrain chunks 110 ->
+// 86 us, 128 of the 2D fBm 26.5 -> 24.0); 1 below, where a CTA a row is what fills
+// the chip.
+constexpr int kFieldRowsChunks = 32;
+template <int VPC, int MODE, int ZB>
 __global__ void __launch_bounds__(96) k_field(BatchPtrs b) {
     using G = Geo<VPC>;
+    static_assert(MODE != LVN_DENSITY_CAVES, "a density with a 3D term uses k_field_caves");
     __shared__ __align__(16) float sg[64];
-    __shared__ uint32_t words[3][G::FD];  // solid-bit word of each warp, per row y
+    __shared__ uint8_t cross[ZB * G::FD];  // a column's first air row
+    __shared__ uint4 rows[3][G::FD];       // a warp's solid rows
     stage_gradients(sg, b.grad);
     __syncthreads();
-    const int c = blockIdx.y, z = blockIdx.x;
+    const int c = blockIdx.y, z0 = blockIdx.x * ZB, nz_rows = min(ZB, G::FD - z0);
     if (b.s_on && b.sslot[c] >= 0) return;  // the surrogate's field (k_field_sdens)
-    const int x = threadIdx.x;
-    const bool valid = x < G::FD;
     // descriptor fields in registers: the byte stores below may alias them
     const int scale = b.desc[c].scale;
     const int ox = b.desc[c].off[0], oy = b.desc[c].off[1], oz = b.desc[c].off[2];
     const Noise nz{b.perm_t3, sg};
     const DensityParams& dp = b.density;
-    const float wx = (float)(x * scale + ox);
-    const float wz = (float)(z * scale + oz);
-    const float h = valid ? height_m<MODE>(nz, dp, wx, wz) : 0.f;
-    if (valid && b.hmap) b.hmap[(size_t)c * G::FD * G::FD + x + G::FD * z] = h;
     const int dm = b.default_material;
     const bool write_mats = b.need_mats != 0;
-    uint8_t* mats = b.mats + (size_t)c * G::F + x + G::FD * G::FD * z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    static_assert(MODE != LVN_DENSITY_CAVES, "a density with a 3D term uses k_field_caves");
-    // y - amp * h rounds monotonically in y, so the column is solid below
-    // the first y whose density is >= 0 and air from there up
-    int ycross = 0;
-    if (valid && dm != MATERIAL_AIR) {
-        int lo = 0, hi = G::FD;  // first y in [lo, hi) with density >= 0, hi if none
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (dens_h<MODE>(nz, dp, h, wx, (float)(mid * scale + oy), wz) < 0.f) lo = mid + 1;
-            else hi = mid;
+    for (int k = threadIdx.x; k < nz_rows * G::FD; k += 96) {
+        const int x = k % G::FD, z = z0 + k / G::FD;
+        const float wx = (float)(x * scale + ox), wz = (float)(z * scale + oz);
+        const float h = height_m<MODE>(nz, dp, wx, wz);
+        if (b.hmap) b.hmap[(size_t)c * G::FD * G::FD + x + G::FD * z] = h;
+        // y - amp * h rounds monotonically in y, so the column is solid below
+        // the first y whose density is >= 0 and air from there up
+        int ycross = 0;
+        if (dm != MATERIAL_AIR) {
+            int lo = 0, hi = G::FD;  // first y in [lo, hi) with density >= 0, hi if none
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (dens_h<MODE>(nz, dp, h, wx, (float)(mid * scale + oy), wz) < 0.f) lo = mid + 1;
+                else hi = mid;
+            }
+            ycross = lo;
         }
-        ycross = lo;
-    }
-    if (valid && write_mats)
-        for (int y = 0; y < G::FD; y++) mats[G::FD * y] = (uint8_t)(y < ycross ? dm : MATERIAL_AIR);
-    // the warp's row words: every valid column is solid below the warp's
-    // lowest crossing and air from its highest up, so only the rows between
-    // need a ballot.  Lane l keeps rows l, l + 32 and l + 64.
-    const unsigned vmask = __ballot_sync(FULL, valid);
-    const int ymin = __reduce_min_sync(FULL, valid ? ycross : G::FD);
-    const int ymax = __reduce_max_sync(FULL, valid ? ycross : 0);
-    uint32_t w0 = 0, w1 = 0, w2 = 0;
-    for (int y = ymin; y < ymax; y++) {
-        const unsigned sb = __ballot_sync(FULL, y < ycross);
-        if ((y & 31) == lane) {
-            w0 = y < 32 ? sb : w0;
-            w1 = y >= 32 && y < 64 ? sb : w1;
-            w2 = y >= 64 ? sb : w2;
+        cross[k] = (uint8_t)ycross;
+        if (write_mats) {
+            uint8_t* mats = b.mats + (size_t)c * G::F + x + G::FD * G::FD * z;
+            for (int y = 0; y < G::FD; y++) mats[G::FD * y] = (uint8_t)(y < ycross ? dm : MATERIAL_AIR);
         }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int y = lane + 32 * k;
-        if (y < G::FD) words[warp][y] = y < ymin ? vmask : y >= ymax ? 0u : k == 0 ? w0 : k == 1 ? w1 : w2;
     }
     __syncthreads();
-    // one thread per row writes the three 16-byte plane rows
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint4 V = low_bits(G::FD);
-    uint4* P = plane_ptr<VPC>(b, c, 0) + G::FD * z;
-    uint4* A = plane_ptr<VPC>(b, c, 1) + G::FD * z;
-    uint4* X = plane_ptr<VPC>(b, c, 2) + G::FD * z;
-    for (int y = threadIdx.x; y < G::FD; y += blockDim.x) {
-        const uint4 p = make_uint4(words[0][y], words[1][y], words[2][y], 0u);
-        P[y] = p;
-        A[y] = and4(not4(p), V);
-        X[y] = make_uint4(0u, 0u, 0u, 0u);
+    for (int r = warp; r < nz_rows; r += 3) {
+        // every column is solid below the row's lowest crossing and air from its
+        // highest up, so only the rows between need their bits gathered
+        int yc[3];
+#pragma unroll
+        for (int w = 0; w < 3; w++) yc[w] = 32 * w + lane < G::FD ? (int)cross[r * G::FD + 32 * w + lane] : -1;
+        int lo = G::FD, hi = 0;
+#pragma unroll
+        for (int w = 0; w < 3; w++) {
+            if (yc[w] >= 0) lo = min(lo, yc[w]);
+            hi = max(hi, yc[w]);
+        }
+        const int ymin = __reduce_min_sync(FULL, lo), ymax = __reduce_max_sync(FULL, hi);
+        for (int y = ymin; y < ymax; y++) {
+            const unsigned s0 = __ballot_sync(FULL, y < yc[0]);
+            const unsigned s1 = G::FD > 32 ? __ballot_sync(FULL, y < yc[1]) : 0u;
+            const unsigned s2 = G::FD > 64 ? __ballot_sync(FULL, y < yc[2]) : 0u;
+            if (lane == 0) rows[warp][y] = make_uint4(s0, s1, s2, 0u);
+        }
+        __syncwarp();
+        uint4* P = plane_ptr<VPC>(b, c, 0) + G::FD * (z0 + r);
+        uint4* A = plane_ptr<VPC>(b, c, 1) + G::FD * (z0 + r);
+        uint4* X = plane_ptr<VPC>(b, c, 2) + G::FD * (z0 + r);
+        for (int y = lane; y < G::FD; y += 32) {
+            const uint4 p = y < ymin ? V : y >= ymax ? make_uint4(0u, 0u, 0u, 0u) : rows[warp][y];
+            P[y] = p;
+            A[y] = and4(not4(p), V);
+            X[y] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncwarp();  // the next row's bits go where these were read
     }
 }
 
@@ -1134,9 +1143,7 @@ __global__ void __launch_bounds__(kCsgThreads) k_csg(BatchPtrs b) {
 // ---------------------------------------------------------------------------
 // Cached-field CSG (compute_csg.cpp:140-175): the field's existing edges that
 // no changed corner touches are kept, in order, ahead of the created edges.
-// One CTA, chunk 0 of a one-chunk batch.
-// ---------------------------------------------------------------------------
-
+// Chunk 0 of a one-chunk batch.
 //
 // A CTA a block of 1024 old edges: it first counts the kept ones of the blocks
 // before its own (loads that wait for nothing), then places its own.  One CTA
@@ -3390,12 +3397,27 @@ cudaError_t launch_reset(const BatchPtrs& b, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <int MODE, int ZB>
+static void launch_field_rows(const BatchPtrs& b, cudaStream_t s) {
+    const dim3 grid((b.vpc + 2 + ZB - 1) / ZB, b.n);
+    switch (b.vpc) {
+        case 8: k_field<8, MODE, ZB><<<grid, 96, 0, s>>>(b); break;
+        case 16: k_field<16, MODE, ZB><<<grid, 96, 0, s>>>(b); break;
+        case 32: k_field<32, MODE, ZB><<<grid, 96, 0, s>>>(b); break;
+        case 64: k_field<64, MODE, ZB><<<grid, 96, 0, s>>>(b); break;
+    }
+}
 cudaError_t launch_field(const BatchPtrs& b, cudaStream_t s) {
-    dim3 grid(b.vpc + 2, b.n);
+    const bool many = b.n >= kFieldRowsChunks;
+    const dim3 grid(b.vpc + 2, b.n);
     switch (b.density.mode) {
-        case LVN_DENSITY_REFERENCE: LVN_VPC_DISPATCH(b.vpc, (k_field<V, LVN_DENSITY_REFERENCE><<<grid, 96, 0, s>>>(b))); break;
-        case LVN_DENSITY_FBM2D: LVN_VPC_DISPATCH(b.vpc, (k_field<V, LVN_DENSITY_FBM2D><<<grid, 96, 0, s>>>(b))); break;
-        default: LVN_VPC_DISPATCH(b.vpc, (k_field_caves<V><<<grid, 96, 0, s>>>(b))); break;
+        case LVN_DENSITY_REFERENCE:
+            many ? launch_field_rows<LVN_DENSITY_REFERENCE, 4>(b, s) : launch_field_rows<LVN_DENSITY_REFERENCE, 1>(b, s);
+            break;
+        case LVN_DENSITY_FBM2D:
+            many ? launch_field_rows<LVN_DENSITY_FBM2D, 4>(b, s) : launch_field_rows<LVN_DENSITY_FBM2D, 1>(b, s);
+            break;
+        default: LVN_VPC_DISPATCH(b.vpc, (k_field_caves<V><<<grid, 96, 0, s>>>(b)));
     }
     if (b.s_on) LVN_VPC_DISPATCH(b.vpc, (k_field_sdens<V><<<grid, 128, 0, s>>>(b)));
     return cudaGetLastError();
