@@ -582,6 +582,8 @@ def run_lvn(args):
                 "traffic_from_profile": traffic_note,
                 "kernel": dominant, "ms_per_launch": round(dom_ms, 4), "peak_source": f"SMs x 128 x 2 x {clk} MHz",
                 "flop_per_launch": int(flops)}
+        if dominant == "hermite":
+            roof["flop_note"] = "counted at the reference's 23 samples an edge; the bounded search evaluates fewer"
     else:
         b = stage_work(dominant, res_np, n)
         ach = b / (dom_ms / 1e3) / 1e9 if b else None
@@ -721,9 +723,10 @@ def density_flops(wl):
 
 
 def hermite_edge_flops(h, p):
-    """The operations k_hermite performs for a plain edge: 23 density samples
-    (the rest p each) and the edge arithmetic, plus the height terms it
-    evaluates: an x or z edge 15 (its end points' heights come from the
+    """The operations of the reference's crossing search and normal for a plain
+    edge (the kernels' bounded search leaves out samples that cannot be the
+    least): 23 density samples (the rest p each) and the edge arithmetic, plus
+    the height terms: an x or z edge 15 (its end points' heights come from the
     field's height map) and 4 for the x and z normal samples; a y edge the 4
     normal heights only (its own height is the map's, and the y normal pair
     shares it)."""

@@ -1241,14 +1241,13 @@ bool mesh_stage(lvn_meshgen* m, DirectOut* d) {
     const int64_t face = (int64_t)m->vpc * m->vpc;
     const int64_t nv = 4 * face, nt = 8 * face, ns = 2 * face;
     const size_t bytes = sizeof(lvn_mesh_vertex) * (nv + ns) + sizeof(lvn_mesh_triangle) * nt;
-    if (!m->h_mesh.p) {
-        if (m->h_mesh.ensure(bytes) != cudaSuccess || ensure_side(m) != LVN_OK) {
-            cudaGetLastError();
-            m->h_mesh.release();
-            return false;
-        }
+    if (!m->h_mesh.p && m->h_mesh.ensure(bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    char* p = m->h_mesh.as<char>();  // vertices, seam nodes, triangles: each 16-byte aligned
+    // vertices, seam nodes, triangles: each 16-byte aligned, so that the leaves and
+    // seams are written by their own kernels and the side stream is not needed
+    char* p = m->h_mesh.as<char>();
     d->dst[0] = p;
     d->dst[2] = p + sizeof(lvn_mesh_vertex) * nv;
     d->dst[1] = p + sizeof(lvn_mesh_vertex) * (nv + ns);

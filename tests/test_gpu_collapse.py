@@ -75,3 +75,15 @@ def test_simplify_errors(lvn_gpu):
     with pytest.raises(lvn.LvnError):
         lvn.mesh_simplify(np.zeros((1, 12), np.float32), np.zeros((1, 3), np.int32), [[0, 1, 0, 1]],
                           [[0, 0, 0, 0]], [bad])
+
+
+@pytest.mark.parametrize("vpc,n", [(8, 40), (16, 24), (32, 1), (32, 30), (64, 1), (64, 20)])
+def test_simplify_cluster_sizes(lvn_gpu, vpc, n):
+    """Lone meshes and batches of several sizes: every number of CTAs a mesh may
+    be given, with prefix sums over one and over several of them."""
+    lvn = lvn_gpu
+    size = 4 * vpc
+    chunks = [((x % 8 * size, (x % 3 - 1) * size, x // 8 * size), size) for x in range(n)]
+    v, t, res = batch(lvn, chunks, lvn.LVN_DENSITY_CAVES, vpc=vpc)
+    simplified = check(lvn, chunks, v, t, res, device=n > 1)
+    assert simplified > 0 or vpc < 32
