@@ -1209,6 +1209,20 @@ __device__ __forceinline__ RowEdges row_edges(const BatchPtrs& b, int c, int row
     const uint4* X = plane_ptr<VPC>(b, c, 2);
     const uint4 V = low_bits(G::FD);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    // without operations nothing is changed and plain solid is what is not final
+    // air: three loads instead of nine (442 terrain nodes: counts 27 -> 23 us, lists
+    // 40 -> 36)
+    if (b.plain_class && b.desc[c].op_count == 0) {
+        RowEdges e;
+        e.kept[0] = e.kept[1] = e.kept[2] = e.created[0] = e.created[1] = e.created[2] = zero;
+        if (y < G::HD && z < G::HD) {
+            const uint4 H = low_bits(G::HD), a0 = A[row];
+            e.kept[0] = and4(H, xor4(a0, shr1(a0)));
+            e.kept[1] = and4(H, xor4(a0, A[row + 1]));
+            e.kept[2] = and4(H, xor4(a0, A[row + G::FD]));
+        }
+        return e;
+    }
     const uint4 a0 = A[row], x0 = X[row];
     const bool has_y = row + 1 < R, has_z = row + G::FD < R;
     const uint4 a_next = has_y ? A[row + 1] : V;
