@@ -40,3 +40,32 @@ def test_single_chunk_matches_batch(lvn_gpu, vpc, density, cache, simplify):
         mg.close()
         ref.close()
         lvn.set_density(mode=0)
+
+
+@pytest.mark.parametrize("n", [4, 9])
+@pytest.mark.parametrize("simplify", [-1.0, 0.05])
+def test_overflowing_batch_matches_single(lvn_gpu, n, simplify):
+    """Batches of chunks so dense that the first run overflows the edge or the
+    leaf pools part of the way: the rerun's meshes are the single chunks'."""
+    lvn = lvn_gpu
+    lvn.clear_csg_operations()
+    lvn.set_density(**DENSE)
+    chunks = [((256 * i, -128, 0), 256) for i in range(n)]
+    mg, one = lvn.MeshGen(64), lvn.MeshGen(64)
+    try:
+        one.set_option(lvn.LVN_OPT_CACHE, 0)
+        mg.set_simplify(simplify)
+        one.set_simplify(simplify)
+        for rep in range(2):
+            v, t, s, res = mg.generate_chunks(chunks)
+            for c, (mn, sz) in enumerate(chunks):
+                m = one.generate_chunk_mesh(mn, sz, 1 << 18)
+                vo, nv, to, nt, so, ns = res[c, :6]
+                assert res[c, 6] > 48 * 1024  # edges, past a chunk's share of the first pools
+                assert np.array_equal(v[vo:vo + nv].view(np.int32), m.vertices.view(np.int32))
+                assert np.array_equal(t[to:to + nt], m.triangles)
+                assert np.array_equal(s[so:so + ns], m.seams)
+    finally:
+        mg.close()
+        one.close()
+        lvn.set_density(mode=0)
