@@ -129,6 +129,12 @@ __global__ void __launch_bounds__(kWalkThreads) k_clipmap_walk(Tree t, const flo
     Node* const open = scratch + (size_t)blockIdx.x * kSlotNodes;  // open list c at open + c * kMaxOpen
     Node* const listed = open + 2 * kMaxOpen;
     const int tid = threadIdx.x, nth = blockDim.x;
+    if (redo_only) {  // mostly none of this CTA's cameras is left: one look at them all, not one a turn
+        bool left = false;
+        for (int64_t q = blockIdx.x + (int64_t)gridDim.x * tid; q < num_queries; q += (int64_t)gridDim.x * nth)
+            left |= counts[q] == kRedo;
+        if (!__syncthreads_or(left)) return;
+    }
     for (int q = blockIdx.x; q < num_queries; q += gridDim.x) {
         if (redo_only && counts[q] != kRedo) continue;  // the warp walk answered this camera
         float cam[3] = {0.f, 0.f, 0.f};
@@ -243,8 +249,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_clipmap_walk(Tree t, const flo
 // visits more than kWarpItems nodes gets kRedo.
 //
 // Bound by the latency of about 45 dependent steps of 32 nodes.  4096 cameras
-// (420 listed nodes each on average) take 29 us with the walk of what is left over;
-// sorting the listed nodes' keys, a bitonic network of 45 passes, it was 145.
+// (420 listed nodes each on average) take 26 us with the walk of what is left over
+// (29 while that walk read one camera's count a turn); sorting the listed nodes'
+// keys, a bitonic network of 45 passes, it was 145.
 struct alignas(16) WarpSelection {
     uint32_t pos[kWarpItems];        // leaf-grid position, 10 bits an axis; the LOD is the level's
     uint16_t count[kWarpItems];      // listed nodes at and below; kOpenNode = has children here
