@@ -1325,26 +1325,54 @@ int one_desc(lvn_meshgen* m, const int32_t min[3], int32_t size, std::vector<Chu
     return build_descs(m, &cd, 1, descs, none, false);
 }
 
-// Copy chunk 0's edge list, and its corners if they are in the pools, into a field entry.
-int save_field(lvn_meshgen* m, FieldEntry& f, bool corners) {
-    const ChunkState& cs = m->last_cs[0];
-    if (corners) {
-        const size_t F = (size_t)field_size(m->vpc);
-        const size_t PB = sizeof(uint4) * 3 * (size_t)field_rows(m->vpc);
-        LVN_CK(f.mats.ensure(F));
-        LVN_CK(f.planes.ensure(PB));
-        LVN_CK(cudaMemcpyAsync(f.mats.p, m->mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
-        LVN_CK(cudaMemcpyAsync(f.planes.p, m->planes.p, PB, cudaMemcpyDeviceToDevice, m->stream));
+// Chunk 0's edge list from the pools into a field entry.  No failure: where there is
+// no memory for a list of the new size the entry takes the pools' own buffers, which
+// the next call allocates again, so that an entry whose corners an edit has changed
+// always gets the edges that go with them.
+int save_edges(lvn_meshgen* m, FieldEntry& f) {
+    const int32_t n = m->last_cs[0].num_edges;
+    const size_t kb = sizeof(int32_t) * std::max(1, n), ib = sizeof(float4) * std::max(1, n);
+    DevBuf keys = f.keys, info = f.info;
+    if (keys.bytes < kb || info.bytes < ib) {
+        keys = DevBuf(), info = DevBuf();
+        if (keys.ensure(kb) != cudaSuccess || info.ensure(ib) != cudaSuccess) {
+            cudaGetLastError();
+            keys.release();
+            std::swap(keys, m->edge_keys);
+            std::swap(info, m->edge_info);
+            m->ecap = 0;
+        }
+        f.keys.release();
+        f.info.release();
+        f.keys = keys, f.info = info;
     }
-    f.num_edges = cs.num_edges;
-    LVN_CK(f.keys.ensure(sizeof(int32_t) * std::max(1, cs.num_edges)));
-    LVN_CK(f.info.ensure(sizeof(float4) * std::max(1, cs.num_edges)));
-    LVN_CK(cudaMemcpyAsync(f.keys.p, m->edge_keys.p, sizeof(int32_t) * cs.num_edges, cudaMemcpyDeviceToDevice,
-                           m->stream));
-    LVN_CK(cudaMemcpyAsync(f.info.p, m->edge_info.p, sizeof(float4) * cs.num_edges, cudaMemcpyDeviceToDevice,
-                           m->stream));
+    if (m->edge_keys.p) {
+        LVN_CK(cudaMemcpyAsync(f.keys.p, m->edge_keys.p, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, m->stream));
+        LVN_CK(cudaMemcpyAsync(f.info.p, m->edge_info.p, sizeof(float4) * n, cudaMemcpyDeviceToDevice, m->stream));
+    }
     LVN_CK(cudaStreamSynchronize(m->stream));
+    f.num_edges = n;
+    m->dbg_keys = f.keys.as<int32_t>();
+    m->dbg_info = f.info.as<float4>();
     return LVN_OK;
+}
+
+// Copy chunk 0's corners and edge list from the pools into a field entry.
+int save_field(lvn_meshgen* m, FieldEntry& f) {
+    const size_t F = (size_t)field_size(m->vpc);
+    const size_t PB = sizeof(uint4) * 3 * (size_t)field_rows(m->vpc);
+    LVN_CK(f.mats.ensure(F));
+    LVN_CK(f.planes.ensure(PB));
+    LVN_CK(cudaMemcpyAsync(f.mats.p, m->mats.p, F, cudaMemcpyDeviceToDevice, m->stream));
+    LVN_CK(cudaMemcpyAsync(f.planes.p, m->planes.p, PB, cudaMemcpyDeviceToDevice, m->stream));
+    return save_edges(m, f);
+}
+
+void release_field(FieldEntry& f) {
+    f.mats.release();
+    f.planes.release();
+    f.keys.release();
+    f.info.release();
 }
 
 // GenerateDefaultDensityField + FindDefaultEdges (compute_density_field.cpp:138-231)
@@ -1366,10 +1394,11 @@ int generate_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntr
     m->last_fresh = false;
     if (m->h_bs.as<BatchState>()->overflow) return LVN_ERR_DEVICE_STATUS;
     f.last_op = 0;
-    return save_field(m, f, true);
+    return save_field(m, f);
 }
 
-// ApplyCSGOperations on a cached field (compute_csg.cpp:11-219)
+// ApplyCSGOperations on the cached field of a chunk (compute_csg.cpp:11-219).  After an
+// error the entry is as it was, or gone (f dangles).
 int apply_csg_to_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry& f,
                        const std::vector<lvn_csg_op>& ops) {
     if (ops.empty()) return LVN_OK;
@@ -1387,15 +1416,15 @@ int apply_csg_to_field(lvn_meshgen* m, const int32_t min[3], int32_t size, Field
     cap.vcap = std::max(cap.vcap, m->vcap);
     if ((rc = ensure_pools(m, 1, cap))) return rc;
     if ((rc = upload(m, descs, brushes))) return rc;
-    // the corners are changed in place; the pools are sized for every edge the new
-    // list can have, so nothing after the first kernel gives the change up
+    // The corners are changed in place.  What can fail for want of memory is behind
+    // this line or cannot fail (the pools are sized for every edge the new list can
+    // have; save_edges); an error of the device below drops the entry, whose corners
+    // and edges may no longer agree, and the chunk's next use makes it afresh from the
+    // stored operations.
     const size_t R = (size_t)field_rows(m->vpc);
     BatchPtrs b = make_ptrs(m, 1);
     b.mats = f.mats.as<uint8_t>();
     b.planes = f.planes.as<uint4>();
-    m->dbg_mats = b.mats;
-    // no corner is changed by this batch until the CSG kernel says so
-    LVN_CK(cudaMemsetAsync(b.planes + 2 * R, 0, sizeof(uint4) * R, m->stream));
     b.plain_class = 0;
     b.need_mats = 1;
     b.derive_mats = 0;
@@ -1403,17 +1432,30 @@ int apply_csg_to_field(lvn_meshgen* m, const int32_t min[3], int32_t size, Field
     b.prev_keys = f.keys.as<int32_t>();
     b.prev_info = f.info.as<float4>();
     b.prev_count = f.num_edges;
-    LVN_CK(launch_reset(b, m->stream));
-    if ((rc = stage(m, ST_CSG, launch_csg, b))) return rc;
-    LVN_CK(launch_prune_edges(b, m->stream));
-    if ((rc = stage(m, ST_EDGE_COUNT, launch_edge_count, b))) return rc;
-    if ((rc = stage(m, ST_EDGE_PLAN, launch_edge_plan, b))) return rc;
-    if ((rc = stage(m, ST_EDGE_SCATTER, launch_edge_scatter, b))) return rc;
-    if ((rc = stage(m, ST_HERMITE, launch_hermite, b))) return rc;
-    if ((rc = read_states(m, 1))) return rc;
-    m->last_fresh = false;
-    if (m->h_bs.as<BatchState>()->overflow) return LVN_ERR_DEVICE_STATUS;
-    return save_field(m, f, false);
+    auto edit = [&]() -> int {
+        // no corner is changed by this batch until the CSG kernel says so
+        LVN_CK(cudaMemsetAsync(b.planes + 2 * R, 0, sizeof(uint4) * R, m->stream));
+        LVN_CK(launch_reset(b, m->stream));
+        int r = stage(m, ST_CSG, launch_csg, b);
+        if (r) return r;
+        LVN_CK(launch_prune_edges(b, m->stream));
+        if ((r = stage(m, ST_EDGE_COUNT, launch_edge_count, b))) return r;
+        if ((r = stage(m, ST_EDGE_PLAN, launch_edge_plan, b))) return r;
+        if ((r = stage(m, ST_EDGE_SCATTER, launch_edge_scatter, b))) return r;
+        if ((r = stage(m, ST_HERMITE, launch_hermite, b))) return r;
+        if ((r = read_states(m, 1))) return r;
+        m->last_fresh = false;
+        if (m->h_bs.as<BatchState>()->overflow) return LVN_ERR_DEVICE_STATUS;
+        return save_edges(m, f);
+    };
+    if ((rc = edit())) {
+        m->dbg_keys = nullptr, m->dbg_info = nullptr;
+        release_field(f);
+        m->fields.erase(key_of(min, size));
+        return rc;
+    }
+    m->dbg_mats = b.mats;
+    return LVN_OK;
 }
 
 // LoadDensityField (compute_density_field.cpp:235-274)
@@ -1427,10 +1469,7 @@ int load_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry** 
         FieldEntry fresh;
         int rc = generate_field(m, min, size, fresh);
         if (rc) {
-            fresh.mats.release();
-            fresh.planes.release();
-            fresh.keys.release();
-            fresh.info.release();
+            release_field(fresh);
             return rc;
         }
         f = &m->fields.emplace(k, std::move(fresh)).first->second;
@@ -1440,9 +1479,12 @@ int load_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEntry** 
     std::vector<lvn_csg_op> replay;
     for (size_t i = (size_t)std::max(0, f->last_op); i < g.ops.size(); i++)
         if (overlaps(lo, hi, g.ops[i].lo, g.ops[i].hi)) replay.push_back(g.ops[i].op);
+    if (!replay.empty()) {
+        const int rc = apply_csg_to_field(m, min, size, *f, replay);
+        if (rc) return rc;  // not counted as replayed
+    }
     f->last_op = (int32_t)g.ops.size();
     *out = f;
-    if (!replay.empty()) return apply_csg_to_field(m, min, size, *f, replay);
     return LVN_OK;
 }
 
@@ -1482,14 +1524,12 @@ int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEnt
         LVN_CK(cudaMemcpyAsync(m->bs.p, m->h_bs.p, sizeof(bs), cudaMemcpyHostToDevice, m->stream));
         BatchPtrs b = make_ptrs(m, 1);
         b.derive_mats = 0;  // the cached field may hold CSG materials
-        // the octree stages only read the field and its edges: no copy to the pools
+        // the octree stages read the field and its edges where they lie (and leave the
+        // voxels' rows in plane 2): no copy to the pools
         b.mats = f.mats.as<uint8_t>();
         b.planes = f.planes.as<uint4>();
         b.edge_keys = f.keys.as<int32_t>();
         b.edge_info = f.info.as<float4>();
-        m->dbg_mats = b.mats;
-        m->dbg_keys = b.edge_keys;
-        m->dbg_info = b.edge_info;
         if (m->profile) {  // one stage at a time, each timed
             if ((rc = enqueue_octree_stages(m, b))) return rc;
             if (staged && (rc = enqueue_exports(m, b, staged, m->stream))) return rc;
@@ -1505,6 +1545,9 @@ int mesh_from_field(lvn_meshgen* m, const int32_t min[3], int32_t size, FieldEnt
         }
         if ((rc = read_states(m, 1))) return rc;
         m->last_fresh = false;
+        m->dbg_mats = b.mats;
+        m->dbg_keys = b.edge_keys;
+        m->dbg_info = b.edge_info;
         const BatchState& hb = *m->h_bs.as<BatchState>();
         if (hb.overflow) {
             cap.vcap = std::max<int64_t>(cap.vcap * 2, (int64_t)hb.total_nodes + 1024);
@@ -1688,12 +1731,7 @@ void lvn_meshgen_destroy(lvn_meshgen* m) {
     m->h_sslot.release();
     m->h_lattices.release();
     m->h_mesh.release();
-    for (auto& kv : m->fields) {
-        kv.second.mats.release();
-        kv.second.planes.release();
-        kv.second.keys.release();
-        kv.second.info.release();
-    }
+    for (auto& kv : m->fields) release_field(kv.second);
     for (int i = 0; i <= ST_COUNT; i++)
         if (m->ev[i]) cudaEventDestroy(m->ev[i]);
     if (m->graph_exec) cudaGraphExecDestroy(m->graph_exec);
@@ -2026,7 +2064,10 @@ int lvn_meshgen_is_chunk_empty(lvn_meshgen* m, const int32_t min[3], int32_t siz
     if (it == m->fields.end()) {
         FieldEntry fresh;
         const int rc = generate_field(m, min, size, fresh);
-        if (rc) return rc;
+        if (rc) {
+            release_field(fresh);
+            return rc;
+        }
         it = m->fields.emplace(k, std::move(fresh)).first;
     }
     *is_empty = it->second.num_edges == 0 ? 1 : 0;
