@@ -434,7 +434,7 @@ int64_t simp_node_capacity(int vpc, int n, int64_t vcap, int64_t* off) {
 }
 
 // Size every pool for `n` chunks with at least the given edge / node capacity.
-int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
+int grow_pools(lvn_meshgen* m, int n, Capacity want) {
     const int F = field_size(m->vpc);
     const int C = m->vpc * m->vpc * m->vpc;
     const int64_t ecap = std::max<int64_t>(want.ecap, 1024);
@@ -452,7 +452,10 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
     LVN_CK(m->h_desc.ensure(sizeof(ChunkDesc) * n));
     LVN_CK(m->h_cs.ensure(sizeof(ChunkState) * n));
     LVN_CK(m->h_bs.ensure(sizeof(BatchState)));
+    // each capacity is 0 while its pools grow: ensure frees the old buffer first, and a
+    // growth that fails must not leave a capacity without the memory behind it
     if (ecap > m->ecap) {
+        m->ecap = 0;
         LVN_CK(m->edge_keys.ensure(sizeof(int32_t) * ecap));
         LVN_CK(m->edge_chunk.ensure(sizeof(int32_t) * ecap));
         LVN_CK(m->edge_info.ensure(sizeof(float4) * ecap));
@@ -461,10 +464,12 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
     }
     const int64_t eslots = 2 * m->ecap + (int64_t)n * (CUCKOO_MIN_TABLE_SIZE + CUCKOO_STASH_SIZE + 512);
     if (eslots > m->eslot_cap) {
+        m->eslot_cap = 0;
         LVN_CK(m->edge_slots.ensure(sizeof(unsigned long long) * eslots));
         m->eslot_cap = eslots;
     }
     if (vcap > m->vcap) {
+        m->vcap = m->vert_cap = m->tri_cap = m->seam_cap = 0;
         LVN_CK(m->node_codes.ensure(sizeof(uint32_t) * vcap));
         LVN_CK(m->node_info.ensure(sizeof(int32_t) * vcap));
         LVN_CK(m->node_chunk.ensure(sizeof(int32_t) * vcap));
@@ -479,17 +484,20 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
     }
     const int64_t nslots = 2 * m->vcap + (int64_t)n * (CUCKOO_MIN_TABLE_SIZE + CUCKOO_STASH_SIZE + 512);
     if (nslots > m->nslot_cap) {
+        m->nslot_cap = 0;
         LVN_CK(m->node_slots.ensure(sizeof(unsigned long long) * nslots));
         m->nslot_cap = nslots;
     }
     const int64_t ntiles = m->vcap / kNodeTile + n + 1;
     if (ntiles > m->ntile_cap) {
+        m->ntile_cap = 0;
         LVN_CK(m->node_tile_counts.ensure(sizeof(int2) * ntiles));
         m->ntile_cap = ntiles;
     }
     (void)C;
     if (m->simp_threshold >= 0.f) {
         if (m->vcap > m->simp_vcap) {
+            m->simp_vcap = 0;
             LVN_CK(m->leaf_vertices.ensure(sizeof(lvn_mesh_vertex) * m->vcap));
             LVN_CK(m->leaf_qef.ensure(sizeof(SimpQef) * m->vcap));
             LVN_CK(m->simp_rep.ensure(sizeof(int) * m->vcap));
@@ -499,22 +507,30 @@ int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
             m->simp_vcap = m->vcap;
         }
         if (n > m->simp_grid_chunks) {
+            m->simp_grid_chunks = 0;
             LVN_CK(m->simp_grid.ensure(sizeof(int) * (size_t)n * (size_t)simp_grid_cells(m->vpc)));
             m->simp_grid_chunks = n;
         }
         const int64_t nodes = simp_node_capacity(m->vpc, n, m->vcap, nullptr);
         if (nodes > m->simp_node_cap) {
+            m->simp_node_cap = 0;
             LVN_CK(m->simp_nodes.ensure(sizeof(SimpNode) * nodes));
             m->simp_node_cap = nodes;
         }
         LVN_CK(m->simp_count.ensure(sizeof(int) * 8));
         if (m->ntile_cap > m->simp_tile_cap) {
+            m->simp_tile_cap = 0;
             LVN_CK(m->simp_tile_counts.ensure(sizeof(int2) * m->ntile_cap));
             m->simp_tile_cap = m->ntile_cap;
         }
     }
     m->chunk_cap = std::max(m->chunk_cap, n);
     return LVN_OK;
+}
+int ensure_pools(lvn_meshgen* m, int n, Capacity want) {
+    const int rc = grow_pools(m, n, want);
+    if (rc) m->last_n = 0;  // the last batch is no longer there to be fetched
+    return rc;
 }
 
 Capacity default_capacity(const lvn_meshgen* m, int n) {
