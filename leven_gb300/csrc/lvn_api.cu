@@ -1292,12 +1292,14 @@ MeshView pool_mesh(const lvn_meshgen* m) {
     return w;
 }
 
-// Host memory to a caller's host array: a plain copy (cudaMemcpy takes 7 us a
-// call before it moves a byte).  A null or device pointer is left to cudaMemcpy.
+// Host memory to a caller's host array: a plain copy for pageable memory (cudaMemcpy
+// takes 7 us a call before it moves a byte).  Pinned and managed arrays are left to
+// cudaMemcpy, which comes after what the default stream still has to do with them, and
+// so are null and device pointers, which it refuses.
 int host_store(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return LVN_OK;
     cudaPointerAttributes at;
-    if (!dst || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeDevice) {
+    if (!dst || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
         LVN_CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToHost));
         return LVN_OK;
     }
@@ -1321,11 +1323,13 @@ int deliver_mesh(lvn_meshgen* m, const DirectOut* staged, lvn_mesh_out* out) {
         if (!rc) rc = host_store(out->seams, staged->dst[2], bs);
         return rc;
     }
-    int rc = copy_out(m, out->vertices, w.v, bv, out->memory);
-    if (!rc) rc = copy_out(m, out->triangles, w.t, bt, out->memory);
-    if (!rc) rc = copy_out(m, out->seams, w.s, bs, out->memory);
-    if (rc) return rc;
-    LVN_CK(cudaStreamSynchronize(m->stream));
+    // the batch is complete; the copies run on the default stream, behind the caller's
+    // pending work on the arrays, as the other single-chunk routes' do
+    const cudaMemcpyKind kind = out->memory == LVN_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    if (bv) LVN_CK(cudaMemcpyAsync(out->vertices, w.v, bv, kind, cudaStreamLegacy));
+    if (bt) LVN_CK(cudaMemcpyAsync(out->triangles, w.t, bt, kind, cudaStreamLegacy));
+    if (bs) LVN_CK(cudaMemcpyAsync(out->seams, w.s, bs, kind, cudaStreamLegacy));
+    LVN_CK(cudaStreamSynchronize(cudaStreamLegacy));
     return LVN_OK;
 }
 
