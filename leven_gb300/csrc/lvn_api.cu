@@ -2258,15 +2258,12 @@ namespace lvn {
 
 // A bound on |amp3 * fbm3| as the kernels compute it, for the cave density
 // (0 for the heightfield densities, which have no 3D term), from a bound on
-// |snoise3|.  kNoise3Bound: a point's four simplex corners are among the
-// lattice points within sqrt(0.6) of it; the sum over those of the largest
-// 32 (0.6 - r^2)^4 |g . p| any gradient of the table gives is at most 0.9825 in
-// a cell (tests/test_search_bounds.py).  kSampleBound takes |g| r for |g . p|,
-// which no gradient reaches at every corner at once: 1.2972
-// (tests/test_cave_bound.py); the surrogate's samples are drawn by it.  fbm3
-// sums the octaves scaled by amplitudes 1, gain3, gain3^2, ...; the 0.1% on top
-// covers single-precision rounding of those sums and products.
-constexpr double kNoise3Bound = 1.0, kSampleBound = 1.2972;
+// |snoise3|: kNoise3Bound (lvn_types.h), or kSampleBound, which takes |g| r for
+// |g . p|, though no gradient reaches it at every corner at once (1.2972); the
+// surrogate's samples are drawn by that one.  fbm3 sums the octaves scaled by
+// amplitudes 1, gain3, gain3^2, ...; the 0.1% on top covers single-precision
+// rounding of those sums and products.
+constexpr double kSampleBound = 1.2972;
 
 static float cave_band(const DensityParams& d, double bound) {
     if (d.mode != LVN_DENSITY_CAVES) return 0.f;

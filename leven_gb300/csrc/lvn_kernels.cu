@@ -500,6 +500,7 @@ constexpr float kNoise3Max = 1.0f, kNoise2Max = 1.02f;      // A
 constexpr float kNoise3Slope = 14.f, kNoise2Slope = 11.5f;  // the gradient's 1-norm
 constexpr float kNoise3Jump = 0.0054f;                      // B
 constexpr int kJumpOctaves = 3;
+static_assert(kNoise3Max == (float)kNoise3Bound, "one bound on |snoise3|");
 
 __device__ __forceinline__ void search_bounds(const DensityParams& dp, const ChunkDesc& d, int vpc, float cave_rem1,
                                               float4* out) {

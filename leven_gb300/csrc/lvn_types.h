@@ -62,6 +62,13 @@ constexpr uint32_t CUCKOO_MIN_TABLE_SIZE = 2048u;  // compute_cuckoo.cpp:15
 // 2 kCaveSteps octaves)
 constexpr int kCaveSteps = 16;
 
+// The bound on |snoise3| that decides points by their sign: the cave band and the
+// octave remainders (lvn_api.cu), the crossing search's kNoise3Max (lvn_kernels.cu).
+// A point's four simplex corners are among the lattice points within sqrt(0.6) of it;
+// the sum over those of the largest 32 (0.6 - r^2)^4 |g . p| any gradient of the table
+// gives is at most 0.983 in a cell.
+constexpr double kNoise3Bound = 1.0;
+
 
 typedef lvn_density_params DensityParams;
 
