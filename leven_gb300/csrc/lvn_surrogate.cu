@@ -666,12 +666,14 @@ __device__ __forceinline__ bool to_tensor_core(bool late) {
     return !__syncthreads_or(late);
 }
 
-// 32 consecutive floats (16-byte aligned, the same for every lane) into registers
+// 32 consecutive floats (16-byte aligned, the same for every lane) into registers;
+// plain loads, since the kernel before may still write them when this one starts
+// (read-only ones are not ordered by start_wait)
 __device__ __forceinline__ void load32(const float* p, float (&v)[32]) {
     const float4* p4 = reinterpret_cast<const float4*>(p);
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const float4 t = __ldg(p4 + i);
+        const float4 t = p4[i];
         v[4 * i] = t.x;
         v[4 * i + 1] = t.y;
         v[4 * i + 2] = t.z;
@@ -1066,7 +1068,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const __grid_con
 // four neighbouring sums a thread, in 16-byte loads, left three warps an SM and took 22).
 constexpr int kAdamThreads = 128;
 constexpr int kAdamBlocks = (kParams + kAdamThreads) / kAdamThreads;  // the parameters and the loss
-__global__ void __launch_bounds__(kAdamThreads) k_adam_partials(const float* __restrict__ partial, int parts, float* p,
+__global__ void __launch_bounds__(kAdamThreads) k_adam_partials(const float* partial, int parts, float* p,
                                                                 float* m, float* v, float lr, float c1, float c2,
                                                                 __nv_bfloat16* wb, float* grad, float* loss) {
     const int place = blockIdx.x * kAdamThreads + threadIdx.x;
