@@ -567,7 +567,8 @@ constexpr uint32_t kCoreCol = (kTile / 8) * 128;  // bytes between core-matrix c
 constexpr int kTrainThreads = 512;  // 16 warps: lane quarter warp & 3, column quarter warp >> 2
 constexpr int kX0Bytes = kTile * kIn * 2;       // 24 KB feature image
 constexpr int kImgBytes = kTile * kHidden * 2;  // 32 KB activation image
-constexpr int kOnesBytes = kTile * 16 * 2;      // 4 KB: 128 rows x 16 columns of 1.0
+constexpr int kOnesCols = 16;
+constexpr int kOnesBytes = kTile * kOnesCols * 2;  // 4 KB: 128 rows x 16 columns of 1.0
 constexpr int kXBytes = kImgBytes + kOnesBytes;  // an activation image and the ones behind it
 constexpr int kTrainSmem = kWbBytes + 2 * kXBytes + kImgBytes;
 static_assert(kTrainSmem + 4 * kTile * 4 + 64 <= 227 * 1024, "one CTA per SM");
@@ -588,6 +589,10 @@ constexpr uint32_t kTmDW2 = 144;   // dW_2 and db_2 (16 columns) over the CTA's 
 constexpr uint32_t kTmDW3 = 288;   // dW_3 and db_3
 constexpr uint32_t kTmDW1 = 0;     // after the last tile: dW_1 and db_1
 constexpr uint32_t kTmDW0 = 144;   // and, once dW_2 is out, dW_0 (96 columns) and db_0
+static_assert(kTmDW1 + kHidden + kOnesCols <= kTmDW0, "dW_1 is read while dW_0 is written");
+static_assert(kTmDW1 + kHidden + kOnesCols <= kTmDW2 && kTmDW2 + kHidden + kOnesCols <= kTmDW3,
+              "dW_2 and dW_3 are read while dW_1 is written");
+static_assert(kTmDW0 + kIn + kOnesCols <= kTmDW3, "dW_3 is read while dW_0 is written");
 constexpr uint32_t kIdescFwd = umma_idesc(kTile, kHidden);
 constexpr uint32_t kIdescDX = umma_idesc(kTile, kHidden) | (1u << 16);                 // B MN-major
 // A and B MN-major; the ones behind the X image make 16 more columns
@@ -996,9 +1001,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const __grid_con
 #pragma unroll
             for (int j = 0; j < 8; j++) d4[j * kHidden] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
-        if (cq == 0) {
-            tmem_ld32(tmem + col0 + in + ((uint32_t)(32 * q) << 16), v);
-            part[b_off(l) + row] = v[0];
+        if (cq == 0) {  // the 16 columns of the ones and no further: a product may be writing there
+            uint32_t r[kOnesCols];
+            tmem_issue16(tmem + col0 + in + ((uint32_t)(32 * q) << 16), r);
+            tmem_wait16(r);
+            part[b_off(l) + row] = __uint_as_float(r[0]);
         }
     };
     for (int i = 0; i < items && ok; i++) {
