@@ -606,7 +606,8 @@ __global__ void k_reset(BatchPtrs b) {
 
 // ---------------------------------------------------------------------------
 // The overflow flags as one answer for the CTA: another stream's plan may set them
-// while a kernel starts, and threads that read them apart would part at a barrier.
+// while a kernel starts, and threads that read them apart would part at a barrier, a
+// vote or a shuffle.
 // A batch that overflowed is run again whatever its kernels still wrote.
 __device__ __forceinline__ bool any_overflow(const BatchPtrs& b) { return __syncthreads_or(b.bs->overflow); }
 
@@ -1295,7 +1296,7 @@ __device__ __forceinline__ int table_slot_bound(int k) {
 // The two cuckoo primes of every chunk, one warp per chunk (b.tables: 1 the edge
 // table's, 2 the leaf table's, 0 both).
 __global__ void __launch_bounds__(256) k_primes(BatchPtrs b) {
-    if (b.bs->overflow) return;
+    if (any_overflow(b)) return;
     const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (c >= b.n) return;
     ChunkState& st = b.cs[c];
@@ -1956,8 +1957,7 @@ __global__ void __launch_bounds__(kThreads, kHermiteCtas) k_hermite(BatchPtrs b)
     __shared__ float sval[kSearch ? 15 * kThreads : 1];
     __shared__ WarpTasks wt[kSearch ? kThreads / 32 : 1];
     stage_gradients(sg, b.grad);
-    __syncthreads();
-    if (b.bs->overflow) return;
+    if (any_overflow(b)) return;  // and the gradients are staged
     hermite_list<MODE, kThreads>(b, Noise{b.perm_t3, sg}, sval + threadIdx.x, wt + (threadIdx.x >> 5));
 }
 
@@ -1994,8 +1994,7 @@ __global__ void __launch_bounds__(kThreads) k_hermite_wide(BatchPtrs b) {
     const int FD2 = (b.vpc + 2) * (b.vpc + 2);
     __shared__ __align__(16) float sg[64];
     stage_gradients(sg, b.grad);
-    __syncthreads();
-    if (b.bs->overflow) return;
+    if (any_overflow(b)) return;  // and the gradients are staged
     const Noise nz{b.perm_t3, sg};
     const DensityParams& dp = b.density;
     const int nplain = b.bs->total_xz + b.bs->total_y;
@@ -2607,7 +2606,7 @@ __global__ void __launch_bounds__(256) k_leaf_qef_check(BatchPtrs b, unsigned lo
 // CreateLeafNodes + SolveQEFs + GenerateMeshVertexBuffer (octree.cl:236-331, 475-487)
 template <int VPC, bool HOST>
 __global__ void __launch_bounds__(kThreads, 4) k_leaf(BatchPtrs b) {
-    if (b.bs->overflow) return;
+    if (any_overflow(b)) return;
     const int total = b.bs->total_nodes;
     int lo = 0, hi = total;
     if (b.nslices > 1) {  // this launch's share of the leaves
