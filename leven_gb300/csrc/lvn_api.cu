@@ -1118,34 +1118,14 @@ int run_fresh_batch(lvn_meshgen* m, std::vector<ChunkDesc>& descs, const std::ve
             return r;
         };
         if (m->use_graphs && !m->profile && !m->surrogate) {
-            // N3: the batch is one graph launch; re-captured only when a
-            // buffer, a capacity or the shape of the batch changes
-            std::vector<uintptr_t> key = {(uintptr_t)n, (uintptr_t)brushes.size(), (uintptr_t)m->crossing_mode,
-                                          (uintptr_t)g.density.mode, (uintptr_t)b.vertices, (uintptr_t)b.vertex_cap,
-                                          (uintptr_t)b.triangles, (uintptr_t)b.triangle_cap, (uintptr_t)b.seams,
-                                          (uintptr_t)b.seam_cap, (uintptr_t)b.ecap, (uintptr_t)b.vcap,
-                                          (uintptr_t)b.edge_slot_cap, (uintptr_t)b.node_slot_cap,
-                                          (uintptr_t)b.node_tile_cap, (uintptr_t)m->desc.p, (uintptr_t)m->brushes.p,
-                                          (uintptr_t)m->mats.p, (uintptr_t)m->edge_keys.p, (uintptr_t)m->node_codes.p,
-                                          (uintptr_t)m->edge_slots.p, (uintptr_t)m->node_slots.p,
-                                          (uintptr_t)m->h_desc.p, (uintptr_t)m->h_brushes.p, (uintptr_t)m->h_cs.p,
-                                          (uintptr_t)g.perm.p, (uintptr_t)(direct ? direct->dst[0] : nullptr),
-                                          (uintptr_t)(direct ? direct->dst[1] : nullptr),
-                                          (uintptr_t)(direct ? direct->dst[2] : nullptr),
-                                          (uintptr_t)(direct ? direct->cap[0] : 0), (uintptr_t)(direct ? direct->cap[1] : 0),
-                                          (uintptr_t)(direct ? direct->cap[2] : 0), (uintptr_t)g.default_material,
-                                          (uintptr_t)b.simp_on, (uintptr_t)m->leaf_vertices.p, (uintptr_t)m->simp_nodes.p,
-                                          (uintptr_t)m->simp_grid.p, (uintptr_t)m->simp_rep.p,
-                                          (uintptr_t)m->simp_tile_counts.p};
-            uint32_t thr_bits;
-            std::memcpy(&thr_bits, &m->simp_threshold, 4);
-            key.push_back(thr_bits);
-            for (int st = 0; st < ST_COUNT; st++) key.push_back((uintptr_t)b.grid_per_sm[st]);
-            key.push_back((uintptr_t)m->dag_hermite_per_sm);
-            key.push_back((uintptr_t)b.hash_fault);
-            key.push_back((uintptr_t)b.hermite_form);
-            const uint32_t* dk = reinterpret_cast<const uint32_t*>(&g.density);
-            for (size_t i = 0; i < sizeof(g.density) / 4; i++) key.push_back(dk[i]);
+            // N3: the batch is one graph launch; re-captured only when something
+            // its kernels or copies are given changes
+            std::vector<uintptr_t> key((sizeof(b) + sizeof(uintptr_t) - 1) / sizeof(uintptr_t), 0);
+            std::memcpy(key.data(), &b, sizeof(b));
+            key.insert(key.end(), {(uintptr_t)brushes.size(), (uintptr_t)m->h_desc.p, (uintptr_t)m->h_brushes.p,
+                                   (uintptr_t)m->h_cs.p, (uintptr_t)m->h_bs.p, (uintptr_t)m->dag_hermite_per_sm});
+            for (int i = 0; direct && i < 3; i++)
+                key.insert(key.end(), {(uintptr_t)direct->dst[i], (uintptr_t)direct->cap[i]});
             if (!m->graph_exec || key != m->graph_key) {
                 if (m->graph_exec) {
                     cudaGraphExecDestroy(m->graph_exec);
