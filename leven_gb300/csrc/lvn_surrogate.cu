@@ -817,9 +817,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const __grid_con
                 if (l == 0 && t > t0) bulk_store(dz1img - kImgBytes - kSlotBytes, dz_addr, kImgBytes);
                 if (l == 1) bulk_store(x1img, xb_addr, kImgBytes);
             }
+            if (more) *reinterpret_cast<uint4*>(x0next + img_off(4 * l + cq, row)) = feature8(p, l);
             float bv[32];
             load32(a.params + b_off(l) + 32 * cq, bv);
-            if (more) *reinterpret_cast<uint4*>(x0next + img_off(4 * l + cq, row)) = feature8(p, l);
             late |= !arrived(&bar, phase);
             float v[32];
             tmem_ld32(tmem + kTmWork + tl, v);
