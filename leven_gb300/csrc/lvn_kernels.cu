@@ -492,7 +492,7 @@ __device__ __forceinline__ float simp_solve(const SimpQef& q, float s, float& ox
 //     octaves' share is added per edge, where they do change simplex
 //     (edge_jump); without that test an LOD0 edge takes 10.2 samples, with it
 //     for two octaves 7.6, for three 7.2, for four 7.1.
-// Entry 4 * class + log2(length) - 1 holds (Q, C, 1 / (8 Q), 0); class 0 is an
+// Entry kSearchLengths * class + log2(length) - 1 holds (Q, C, 1 / (8 Q), 0); class 0 is an
 // edge along y (3D term only), class 1 along x or z.  Non-finite parameters
 // give an infinite C, with which no sample is ever skipped.
 constexpr float kNoise3Curve = 41.f, kNoise2Curve = 46.f;   // H
@@ -535,7 +535,7 @@ __device__ __forceinline__ void search_bounds(const DensityParams& dp, const Chu
     const float round = far * 2.f * eps * reach + 1e-4f;
     for (int e = 0; e < 2 * kSearchLengths; e++) {
         const bool xz = e >= kSearchLengths;
-        const float len = (float)d.scale * (float)(2 << (e & (kSearchLengths - 1))) * 0.0625f;
+        const float len = (float)d.scale * (float)(2 << e % kSearchLengths) * 0.0625f;
         // along y the height is one float for every sample
         float Q = 0.f, C = 2.f * (err3 + round + (xz ? err2 : 0.f)) + jump;
         auto octaves = [&](int n, float f, float lac, float a, float gain, float H, float A) {

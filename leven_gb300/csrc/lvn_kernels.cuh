@@ -128,7 +128,7 @@ struct BatchPtrs {
     int prev_count;
 };
 
-constexpr int kSearchLengths = 4;   // interval lengths 2, 4, 8, 16 of the 17-sample search
+constexpr int kSearchLengths = 3;   // interval lengths 2, 4, 8 of the 17-sample search (16 is always halved)
 constexpr int kSearchEntries = 2 * kSearchLengths + 1;  // the search's two edge classes, the cave field's grid
 
 constexpr int kRowTile = 256;       // field / voxel rows per CTA in the dense stages
