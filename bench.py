@@ -339,20 +339,23 @@ def run_reference(args):
 
 # algorithmic work per stage, used for the roofline of the dominant kernel
 def stage_work(stage, res, n_chunks, vpc=64):
-    F = (vpc + 2) ** 3
-    C3 = vpc ** 3
+    """Bytes a stage cannot do without: a chunk's field is bit planes of 16 bytes a
+    row, of which the edge and voxel passes need one (a few chunks with operations
+    need more)."""
+    rows = (vpc + 2) ** 2
+    plane = 16 * rows * n_chunks
     E = int(res[:, 6].sum())
     V = int(res[:, 7].sum())
     T = int(res[:, 3].sum()) // 2
     S = int(res[:, 5].sum())
     nbytes = {
-        "field": 2 * F * n_chunks,                              # corner words written
-        "edge_count": 2 * F * n_chunks,                         # corner words read
-        "edge_scatter": 2 * F * n_chunks + 8 * E,               # corners read, keys + chunk ids written
-        "vox_count": 2 * F * n_chunks,
-        "vox_scatter": 2 * F * n_chunks + 12 * V,
+        "field": 3 * plane + 4 * rows * n_chunks,               # three planes and the height map written
+        "edge_count": plane,
+        "edge_scatter": plane + 12 * E,                         # keys, chunk ids, work list written
+        "vox_count": plane,
+        "vox_scatter": plane + 12 * V,
         "leaf": 12 * V + 16 * E + 48 * V,                       # codes/info/chunk, hermite, vertices
-        "mesh_count": 12 * V + 48 * V,                          # codes/info/chunk in, quad scratch out
+        "mesh_count": plane + 8 * V + 48 * V,                   # voxel rows, codes/info in, quad scratch out
         "mesh_scatter": 48 * V + 12 * V + 24 * T + 48 * S,
         "hash_fill": 8 * (2 * E + 2 * V),
         "edge_insert": 8 * E + 16 * E,
@@ -576,14 +579,8 @@ def run_lvn(args):
         else:  # every field point of every chunk: the height per column, the cave term per point
             fd = wl.voxels_per_chunk + 2
             flops = n * (fd * fd * df[0] + fd ** 3 * df[1])
-        ach = flops / (dom_ms / 1e3) / 1e12
-        roof = {"bound": "fp32", "achieved": round(ach, 3), "peak": round(fp32_peak, 2),
-                "unit": "TFLOP/s", "frac": round(ach / fp32_peak, 4), "traffic": traffic,
-                "traffic_from_profile": traffic_note,
-                "kernel": dominant, "ms_per_launch": round(dom_ms, 4), "peak_source": f"SMs x 128 x 2 x {clk} MHz",
-                "flop_per_launch": int(flops)}
-        if dominant == "hermite":
-            roof["flop_note"] = "counted at the reference's 23 samples an edge; the bounded search evaluates fewer"
+        roof = dict(fp32_equivalent(flops, dom_ms, fp32_peak), kernel=dominant, traffic=traffic,
+                    traffic_from_profile=traffic_note, peak_source=f"SMs x 128 x 2 x {clk} MHz")
     else:
         b = stage_work(dominant, res_np, n)
         ach = b / (dom_ms / 1e3) / 1e9 if b else None
@@ -640,11 +637,14 @@ def run_lvn(args):
     line["stage_gbs"] = stage_gbs
     line["stage_gbs_peak"] = {"hbm_gbs": hbm_peak, "source": peak_src}
     # density samples a step determines: every field point of every chunk, and
-    # the 23 evaluations (17 search + 6 normal) of each plain edge's hermite data
+    # the 23 evaluations (17 search + 6 normal) of each plain edge's hermite data;
+    # the kernels evaluate those that can matter
     nxz, ny = edge_axis_counts(mg, lvn, n) if n <= 8192 else (0, 0)
     samples = n * (wl.voxels_per_chunk + 2) ** 3 + 23 * (nxz + ny)
     line["density_samples_per_s"] = round(samples / (ms / 1e3), 1)
     line["density_samples_per_step"] = int(samples)
+    line["density_samples_note"] = ("the reference's samples whose outcome a step determines; fewer are evaluated "
+                                    "(bounded search, cave grid, columns)")
     # the FP32 leaf solve against an FP64 solve of the same crossings, over
     # every leaf of the last (device-output) step: a GPU measurement pass
     step(True)
@@ -720,6 +720,17 @@ def density_flops(wl):
     if d["mode"] == 2 and d["octaves2"] == 8 and d["octaves3"] == 6:
         return FLOP_HEIGHT8, 2 + FLOP_CAVES6
     return None
+
+
+def fp32_equivalent(flops, ms, peak):
+    """The roofline entry of a density kernel from the operations the reference's
+    samples would take.  The kernels leave out samples that cannot matter, so the
+    rate is no share of the issue peak: `achieved` and `frac` stay empty."""
+    return {"bound": "fp32", "achieved": None, "frac": None, "peak": round(peak, 2), "unit": "TFLOP/s",
+            "ms_per_launch": round(ms, 4), "reference_flop_per_launch": int(flops),
+            "reference_equivalent_tflops": round(flops / (ms / 1e3) / 1e12, 3),
+            "note": "operations of the reference's samples (hermite: 23 an edge; field: every point), of which "
+                    "the kernel evaluates a part: an equivalent rate, not a roofline fraction"}
 
 
 def hermite_edge_flops(h, p):
