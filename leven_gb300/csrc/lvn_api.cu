@@ -2,9 +2,9 @@
 //
 // Replaces the reference's OpenCL host layer (leven/src/compute.cpp,
 // compute_density_field.cpp, compute_octree.cpp, compute_csg.cpp,
-// compute_cuckoo.cpp).  One CUDA stream per mesh-generation context; a batch
-// of chunks is enqueued as a fixed sequence of kernels with no host round
-// trip, then one small device-to-host read returns the per-chunk counts.
+// compute_cuckoo.cpp).  A mesh-generation context has a CUDA stream of its own and
+// two beside it; a batch of chunks is enqueued as a fixed graph of kernels with no
+// host round trip, then one small device-to-host read returns the per-chunk counts.
 // Device pools grow on demand and are reused across calls.
 #include <cuda_runtime.h>
 
@@ -390,9 +390,9 @@ struct lvn_meshgen {
     // export of pinned host outputs: a side stream and its events
     cudaStream_t side = nullptr;
     cudaEvent_t ev_leaf = nullptr, ev_side = nullptr;
-    // the fresh-batch DAG: hermite on `aux` beside the voxel, hash and quad
-    // stages, with a grid of dag_hermite_per_sm CTAs per SM (0 = its tuned shape)
-    cudaStream_t aux = nullptr, aux2 = nullptr;  // hermite; the quad chain
+    // the batch DAG: the hash tables on `aux` and the voxels and quads on `aux2`
+    // beside hermite, which has dag_hermite_per_sm CTAs per SM (0 = its tuned shape)
+    cudaStream_t aux = nullptr, aux2 = nullptr;
     cudaEvent_t ev_field = nullptr, ev_plan = nullptr, ev_fork = nullptr, ev_vplan = nullptr, ev_vox = nullptr;
     cudaEvent_t ev_etab = nullptr, ev_hash = nullptr, ev_mesh = nullptr;
     int dag_hermite_per_sm = 0;
@@ -739,7 +739,7 @@ constexpr int kLeafSlices = 4;  // leaf / vertex-export pipeline depth for pinne
 //   field, CSG, edges -> hermite                                 (stream)
 //   || voxels (their counts beside the edges') -> quads, triangles  (aux2)
 //      [pinned outputs: triangles exported on aux2]
-//   || edge table, then leaf table                                (aux)
+//   || edge table, then leaf table (for debug fetches)            (aux)
 //   -> join voxels and edge table -> leaves                       (stream)
 //      [pinned outputs: the leaves write their vertices to the host
 //       array as they are made; an unaligned array instead gets the

@@ -49,8 +49,9 @@ constexpr int kHostStride = 1024;                     // first-pass list length 
 constexpr int kMaxBoxes = 4096;                       // operations per touch-set call
 // selection by one warp per camera: the nodes it visits (listed ones, open ones
 // and the top level's), beyond which the CTA walk redoes the camera, its top
-// level's limit, and the warps of a CTA.  55 KB a CTA, four CTAs an SM: 28 warps,
-// so that 4096 cameras run at once on 152 SMs.
+// level's limit, and the warps of a CTA.  An SM's shared memory holds 28 such warps,
+// 55 KB for seven, in four CTAs that start and end apart; more nodes a warp would
+// leave fewer cameras at once, whatever their number.
 constexpr int kWarpItems = 1264;
 constexpr int kWarpTop = 512;
 constexpr int kWarpsPerCta = 7;

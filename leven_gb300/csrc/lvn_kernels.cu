@@ -1,7 +1,7 @@
 // lvn_kernels.cu -- the sm_103a kernels of the chunk-meshing pipeline.
 //
-// A batch of chunks flows through these stages (one launch each, all on one
-// stream, no host round trip):
+// A batch of chunks flows through these stages with no host round trip; behind the
+// edges they run on three streams (enqueue_mesh_dag in lvn_api.cu):
 //
 //   field      density per corner of each 66^3 field (heightfield modes reuse
 //              the height term down each y column)      density_field.cl:11-37
@@ -11,16 +11,18 @@
 //              (hermite index, axis) order; plain edges touched by CSG are
 //              dropped and CSG-created edges appended     density_field.cl:41-92,
 //                                                       apply_csg_operation.cl:253-437
-//   hermite    17-sample zero crossing + central-difference normal per edge
+//   hermite    the least of 17 samples (those that can be it) + central-difference
+//              normal per edge
 //                                                       density_field.cl:96-151,
 //                                                       apply_csg_operation.cl:443-477
 //   vox_*      count / plan / scatter of active voxels (leaf codes, edge
 //              masks, dominant material)                octree.cl:142-223
 //   hash_fill, edge_insert, node_insert
-//              cuckoo tables, one per chunk and key set   cuckoo.cl:26-71
+//              cuckoo tables, one per chunk and key set (the leaves' for debug
+//              fetches only)                              cuckoo.cl:26-71
 //   leaf       12 edge lookups, QEF accumulate + 10-sweep Jacobi solve,
 //              MeshVertex written in place              octree.cl:236-331,475-487
-//   mesh_*     quad emission with 3 node lookups per axis, seam nodes
+//   mesh_*     quad emission, the neighbours found by leaf rank, seam nodes
 //                                                       octree.cl:385-464,506-551
 //
 // Compactions are tile based: a CTA owns a tile of a chunk's dense domain,
@@ -51,7 +53,12 @@ constexpr int kHermiteCtas = 3;             // k_hermite: CTAs of kThreads per S
 // takes 12.9 us instead of 47, of the 2D fBm 13.6 instead of 21.8, of the
 // caves 29.5 instead of 42.  Two chunks still gain (17.3 against 22.9 us, 37
 // against 47); four lose with the fBm densities (25.4 against 23.1, 70 against
-// 54), whose searches skip samples, while the terrain takes all of them.
+// 54), whose searches skip samples, while the terrain takes all of them.  The
+// faces count, as a chunk's edges grow with them: at the limit 128 chunks of 8^3
+// take 15 us against 23-25 (caves 37-41 against 46-52), 32 of 16^3 14-15 against
+// 21-25 (33-37 against 43-52), 8 of 32^3 14 against 22-25 (33 against 45-49), of the
+// terrain 256, 64 and 16 chunks 29, 26-31 and 27-29 against 38-41.  Two 64^3 chunks
+// with an unusual 24 k edges of caves are level (49 against 47).
 constexpr int kHermiteWideFaces = 2 * 64 * 64;
 constexpr int kHermiteWideFacesTerrain = 4 * 64 * 64;
 

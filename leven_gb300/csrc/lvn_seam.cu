@@ -8,8 +8,8 @@
 // ContourProcessEdge, octree.cpp:236-474) on the CPU.
 //
 // Here the neighbour search, which walks the clipmap's node tree, stays on the
-// host; everything that touches seam nodes runs on the device, one CTA per
-// host, without building the tree:
+// host; everything that touches seam nodes runs on the device, without building
+// the tree:
 //   * the depth-first leaf order is the Morton order of the leaves' minimum
 //     corners (children are visited x << 2 | y << 1 | z), so the leaves are
 //     sorted by Morton key (in parts that fit shared memory) and numbered by rank;
