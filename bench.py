@@ -683,12 +683,15 @@ def committed_traffic(kernel):
     """DRAM bytes per launch of `kernel` on this workload as a committed ncu
     summary states them (profiles/<kernel>_<workload>.md, the table row
     `dram_bytes_per_launch`), with the file: a figure from an earlier capture,
-    not a measurement of this run."""
+    not a measurement of this run; None where the summary is of an earlier form."""
     if CHUNKS:
         return None
     path = ROOT / "profiles" / f"{kernel}_{PROFILE_TAG.get(WORKLOAD, WORKLOAD)}.md"
     try:
-        for line in path.read_text().splitlines():
+        text = path.read_text()
+        if "(An earlier form of the code" in text:
+            return None
+        for line in text.splitlines():
             if "dram_bytes_per_launch" in line:
                 return {"dram_bytes_per_launch": int(line.split("|")[2].strip()),
                         "file": str(path.relative_to(ROOT))}

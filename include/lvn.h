@@ -197,7 +197,10 @@ lvn_meshgen* lvn_meshgen_create(int32_t voxels_per_chunk);
 void         lvn_meshgen_destroy(lvn_meshgen* ctx);
 /* Compute_MeshGenContext::voxelsPerChunk (compute.h:52; compute.cpp:612-615) */
 int lvn_meshgen_voxels_per_chunk(const lvn_meshgen* ctx);
-/* Compute_MeshGenContext::applyCSGOperations (compute.h:54-57; compute_csg.cpp:224-242) */
+/* Compute_MeshGenContext::applyCSGOperations (compute.h:54-57; compute_csg.cpp:224-242).
+ * After an error the chunk's field is as it was; after an error of the device
+ * (LVN_ERR_CUDA, LVN_ERR_DEVICE_STATUS) it may be gone, and its next use makes it
+ * from the density and the stored operations. */
 int lvn_meshgen_apply_csg_operations(lvn_meshgen* ctx, const lvn_csg_op* ops, int32_t num_ops,
                                      const int32_t min[3], int32_t size);
 /* Compute_MeshGenContext::freeChunkOctree (compute.h:59-61; compute_octree.cpp:379-387) */
