@@ -1894,7 +1894,10 @@ int lvn_meshgen_set_surrogate(lvn_meshgen* m, lvn_surrogate* s, float gate) {
     m->surrogate = s;
     m->surrogate_gate = gate;
     m->octrees.clear();
+    for (auto& kv : m->fields) release_field(kv.second);
     m->fields.clear();
+    m->last_n = 0;  // a debug fetch may have pointed into a field
+    m->dbg_mats = nullptr, m->dbg_keys = nullptr, m->dbg_info = nullptr;
     return LVN_OK;
 }
 

@@ -1,4 +1,4 @@
-"""A batch whose pools cannot grow (a device allocation fails after the first run
+"""Pools and caches that fail or are dropped.  A batch whose pools cannot grow (a device allocation fails after the first run
 has found them too small) returns an error and leaves the context usable: the next
 batch, one that the pools had already held, meshes as before."""
 import numpy as np
@@ -40,5 +40,32 @@ def test_context_survives_a_failed_growth(lvn_gpu, n, simplify):
                 assert np.array_equal(x.view(np.int32), y.view(np.int32))
     finally:
         lvn.inject_fault(lvn.LVN_FAULT_NONE, 0)
+        mg.close()
+        lvn.set_density(mode=0)
+
+
+def test_dropped_caches_give_their_memory_back(lvn_gpu):
+    """Setting a context's surrogate drops its cached fields: 200 rounds of two cached
+    64^3 chunks (1.5 MB each) leave the device's free memory where it was."""
+    import torch
+
+    lvn = lvn_gpu
+    lvn.clear_csg_operations()
+    lvn.set_density(**W.FBM2D)
+    chunks = [((0, 0, 0), 256), ((256, 0, 0), 256)]
+    mg = lvn.MeshGen(64)
+
+    def rounds(n):
+        for _ in range(n):
+            meshes = [mg.generate_chunk_mesh(*c) for c in chunks]
+            assert all(m.triangles.shape[0] > 0 for m in meshes)
+            mg.set_surrogate(None)
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    try:
+        before = rounds(5)
+        assert rounds(200) >= before - (64 << 20)
+    finally:
         mg.close()
         lvn.set_density(mode=0)
