@@ -1,6 +1,7 @@
-"""Pools and caches that fail or are dropped.  A batch whose pools cannot grow (a device allocation fails after the first run
-has found them too small) returns an error and leaves the context usable: the next
-batch, one that the pools had already held, meshes as before."""
+"""Pools that cannot grow and caches that are dropped.  A batch whose pools cannot
+grow (a device allocation fails after the first run has found them too small) returns
+an error and leaves the context usable: the next batch, one that the pools had already
+held, meshes as before."""
 import numpy as np
 import pytest
 
